@@ -656,7 +656,7 @@ int tn_eigensolve_dense(tn_ctx c, int N, const double* A, int lda, int k, double
     // max_i sum_j |A_ij|; its SVD is then its eigen-decomposition, with the
     // eigenvalues s_i - sigma (descending) -- all on the device.
     const size_t n2 = (size_t)N * N;
-    DevBuf work;
+    DevBuf& work = cx.apiw[0];
     TN_CHECK(work.ensure(sizeof(double) * (4 * n2 + (size_t)N + 8)));
     double* W = work.as<double>();
     double* V = W + n2;
@@ -686,9 +686,7 @@ static int svd_common(tn_ctx c, int m, int n, const double* A, int lda, double* 
     const bool tall = m >= n;
     const int tm = tall ? m : n, tn = tall ? n : m;
     size_t need = (size_t)tm * tn + (size_t)tn * tn + (tall ? 0 : (size_t)tm * tn + (size_t)tn * tn);
-    TN_CHECK(cx.svdw.ensure(sizeof(double) * need + sizeof(SvdJob) * 2));
-    // svd_batched uploads its job array into cx.svdw: keep the matrices elsewhere
-    DevBuf work;
+    DevBuf& work = cx.apiw[0];
     TN_CHECK(work.ensure(sizeof(double) * need));
     double* Wm = work.as<double>();
     double* V = Wm + (size_t)tm * tn;
@@ -732,7 +730,7 @@ int tn_svd_solve(tn_ctx c, int m, int n, const double* A, int lda, double eps, i
         return TN_BAD_ARG;
     TN_ON_DEVICE(c->c.device);
     Ctx& cx = c->c;
-    DevBuf full;
+    DevBuf& full = cx.apiw[1];
     TN_CHECK(full.ensure(sizeof(double) * ((size_t)m * mn + (size_t)mn * n + mn)));
     double* Uf = full.as<double>();
     double* Vf = Uf + (size_t)m * mn;

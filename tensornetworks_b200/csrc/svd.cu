@@ -1,4 +1,5 @@
-// svd.cu -- one-sided (Hestenes) Jacobi SVD in FP64, one CTA per matrix.
+// svd.cu -- one-sided (Hestenes) Jacobi SVD in FP64: a thread-block cluster per
+// matrix with the columns in registers, or one CTA per matrix past its limits.
 //
 // Replaces LapackSVDSolver<T>::Solve (zgesvd, LapackSVDSolver.C:42-90).  The
 // columns of the tall working matrix are orthogonalised pairwise; pairs follow
@@ -8,9 +9,13 @@
 // Singular values come out descending; zero singular values get orthonormal
 // completion columns in U (as zgesvd provides), which the zero-padded bond
 // growth of the sweep relies on.  A batch of matrices runs as one launch.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "qr.h"
+
+namespace cg = cooperative_groups;
 
 namespace tnb {
 
@@ -29,6 +34,101 @@ __device__ __forceinline__ int rr_pos(int q, int r, int ne) {
     return q == 0 ? 0 : ((q - 1 + r) % (ne - 1)) + 1;
 }
 
+// Orthonormal completion of the U columns whose singular value is at most the
+// cut, by one whole block: unit vectors e_0, e_1, ... projected off every
+// accepted column (classical Gram-Schmidt applied twice: all dots of a pass are
+// independent, a warp each, and one barrier separates them from the update; the
+// column-after-column form takes three barriers per column), kept when more
+// than half of the unit vector is left.  Once the unit vectors are used up (the
+// rest of the space may be spread evenly over them), the one with the largest
+// remainder 1 - sum_p U(e, p)^2 is taken, which is never zero while columns are
+// missing.  U is read by L2 loads: other CTAs may have written it in this
+// launch.  dots: n doubles of shared memory, red and at: 32 each.
+__device__ void complete_u(const SvdJob& jb, double cut, double* red, double* dots, int* at) {
+    const int m = jb.m, n = jb.n;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+    int next_e = 0;
+    for (int c = 0; c < n; ++c) {
+        const double sc = __ldcg(jb.s + c);
+        if (sc > cut && sc > 0.0) continue;
+        double* uc = jb.U + (size_t)c * jb.ldu;
+        auto accepted = [&](int p) {
+            const double sp = __ldcg(jb.s + p);
+            return p != c && ((sp > cut && sp > 0.0) || p < c);
+        };
+        for (bool placed = false; !placed;) {
+            int e = next_e++;
+            const bool last = e >= m;
+            if (last) {
+                double best = -1.0;
+                int bi = 0;
+                for (int i = tid; i < m; i += blockDim.x) {
+                    double r = 1.0;
+                    for (int p = 0; p < n; ++p)
+                        if (accepted(p)) {
+                            const double u = __ldcg(jb.U + (size_t)p * jb.ldu + i);
+                            r = fma(-u, u, r);
+                        }
+                    if (r > best) { best = r; bi = i; }
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                    if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+                }
+                if (lane == 0) {
+                    red[wid] = best;
+                    at[wid] = bi;
+                }
+                __syncthreads();
+                if (tid == 0) {
+                    int w0 = 0;
+                    for (int w = 1; w < nw; ++w)
+                        if (red[w] > red[w0]) w0 = w;
+                    at[0] = at[w0];
+                }
+                __syncthreads();
+                e = at[0];
+            }
+            for (int i = tid; i < m; i += blockDim.x) uc[i] = (i == e) ? 1.0 : 0.0;
+            __syncthreads();
+            for (int pass = 0; pass < 2; ++pass) {
+                for (int p = wid; p < n; p += nw) {
+                    double part = 0;
+                    if (accepted(p)) {
+                        const double* up = jb.U + (size_t)p * jb.ldu;
+                        for (int i = lane; i < m; i += 32) part = fma(__ldcg(up + i), __ldcg(uc + i), part);
+                    }
+                    part = wsum(part);
+                    if (lane == 0) dots[p] = part;
+                }
+                __syncthreads();
+                for (int i = tid; i < m; i += blockDim.x) {
+                    double v = __ldcg(uc + i);
+                    for (int p = 0; p < n; ++p)
+                        if (dots[p] != 0.0) v = fma(-dots[p], __ldcg(jb.U + (size_t)p * jb.ldu + i), v);
+                    uc[i] = v;
+                }
+                __syncthreads();
+            }
+            double part = 0;
+            for (int i = tid; i < m; i += blockDim.x) part = fma(__ldcg(uc + i), __ldcg(uc + i), part);
+            part = wsum(part);
+            if (lane == 0) red[wid] = part;
+            __syncthreads();
+            double nr2 = 0;
+            for (int w = 0; w < nw; ++w) nr2 += red[w];
+            __syncthreads();
+            const double nr = sqrt(nr2);
+            if (nr > 0.5 || last) {
+                for (int i = tid; i < m; i += blockDim.x) uc[i] = nr > 0.0 ? __ldcg(uc + i) / nr : 0.0;
+                placed = true;
+            }
+            __syncthreads();
+        }
+    }
+}
+
 __global__ void __launch_bounds__(SVD_THREADS) jacobi_svd_kernel(const SvdJob* __restrict__ jobs, int vectors,
                                                                    size_t smem_cap) {
     extern __shared__ double smem[];
@@ -38,6 +138,7 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_svd_kernel(const SvdJob* _
     __shared__ int s_rot;
     __shared__ int s_sweeps;
     __shared__ double red[32];
+    __shared__ int at[32];
 
     // shared memory: norms (n), ranks (n ints), then A (m x n) and V (n x n) when they fit
     double* norms = smem;
@@ -140,54 +241,342 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_svd_kernel(const SvdJob* _
             for (int i = lane; i < n; i += 32) jb.Vt[(size_t)i * jb.ldvt + rk] = vj[i];
         }
         __syncthreads();
-        // orthonormal completion of U columns whose singular value is below the cut:
-        // unit vectors, Gram-Schmidt (twice) against every accepted column
-        int next_e = 0;
-        for (int c = 0; c < n; ++c) {
-            double sc = __ldcg(jb.s + c);
-            if (sc > cut && sc > 0.0) continue;
-            double* uc = jb.U + (size_t)c * jb.ldu;
-            bool placed = false;
-            while (!placed && next_e < m) {
-                const int e = next_e++;
-                for (int i = tid; i < m; i += blockDim.x) uc[i] = (i == e) ? 1.0 : 0.0;
-                __syncthreads();
-                for (int pass = 0; pass < 2; ++pass) {
-                    for (int p = 0; p < n; ++p) {
-                        if (p == c) continue;
-                        double sp = __ldcg(jb.s + p);
-                        if (!((sp > cut && sp > 0.0) || p < c)) continue;
-                        const double* up = jb.U + (size_t)p * jb.ldu;
-                        double part = 0;
-                        for (int i = tid; i < m; i += blockDim.x) part = fma(up[i], uc[i], part);
-                        part = wsum(part);
-                        if (lane == 0) red[wid] = part;
-                        __syncthreads();
-                        double dotv = 0;
-                        for (int w = 0; w < nw; ++w) dotv += red[w];
-                        __syncthreads();
-                        for (int i = tid; i < m; i += blockDim.x) uc[i] = fma(-dotv, up[i], uc[i]);
-                        __syncthreads();
-                    }
-                }
-                double part = 0;
-                for (int i = tid; i < m; i += blockDim.x) part = fma(uc[i], uc[i], part);
-                part = wsum(part);
-                if (lane == 0) red[wid] = part;
-                __syncthreads();
-                double nr2 = 0;
-                for (int w = 0; w < nw; ++w) nr2 += red[w];
-                __syncthreads();
-                double nr = sqrt(nr2);
-                if (nr > 0.5) {
-                    for (int i = tid; i < m; i += blockDim.x) uc[i] /= nr;
-                    placed = true;
-                }
-                __syncthreads();
-            }
-        }
+        complete_u(jb, cut, red, norms, at);
     }
     if (tid == 0 && jb.sweeps) *jb.sweeps = s_sweeps;
+}
+
+// ---------------------------------------------------------------------------
+// Cluster kernel: one matrix per thread-block cluster, its columns in registers.
+//
+// Warp w of the cluster holds four columns, two blocks of two ("top" and
+// "bottom"); lane l holds rows l + 32 q of each, the matrix's rows in the first
+// ET slots and, with vectors, the accumulated rotations' rows after them, so a
+// rotation is one pass over the registers.  A round rotates the four
+// top x bottom pairs as two steps of two independent pairs: the two dots of a
+// step share one butterfly (pair 0 ends in lanes 0-15, pair 1 in 16-31), each
+// half warp computes its own pair's angle at the same time, and one exchange
+// hands it to the other half.  The columns' squared norms travel with them and
+// follow the rotations, (al, be) -> (al - t ga, be + t ga); they are summed
+// afresh at the start of every sweep, whose last one (no rotation left) is the
+// convergence test.  Between rounds the blocks move one warp on (circle
+// method, block 0 fixed): written straight into the receiving warp's inbox,
+// in this CTA or by distributed shared memory in the neighbouring one, one
+// cluster barrier per round (inboxes alternate by round parity; with one
+// parity only, when two do not fit, a second barrier frees them).
+//
+// What bounds it: the serial chain of a round -- inbox read, two times (dot,
+// butterfly, angle, update), remote write, barrier -- about 1 us, times
+// n / 2 - 1 rounds, times 9-19 sweeps.  One CTA per matrix spends that latency
+// per pair of each warp's share and reads every column from shared memory (or
+// L2) three times per round.
+constexpr int JC_SLOTS_MAX = 16;  // row slots per column: four columns x 16 doubles = 128 registers
+
+__device__ __forceinline__ double jc_pick(bool hi, double a, double b) { return hi ? b : a; }
+
+// pow2 scale bringing x (>= 0) near 1 (1 for x = 0 or not finite)
+__device__ __forceinline__ double jc_scale(double x) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    return (e == 0 || e >= 0x7fe) ? 1.0 : __hiloint2double((0x7fe - e) << 20, 0);
+}
+
+// The rotations of the pairs (x0, y0) and (x1, y1); norms updated in place.
+template <int E>
+__device__ __forceinline__ bool jc_rotate2(double (&x0)[E], double (&y0)[E], double (&x1)[E], double (&y1)[E],
+                                           double& nx0, double& ny0, double& nx1, double& ny1, int ET, double tol) {
+    const bool hi = threadIdx.x & 16;
+    const double al = jc_pick(hi, nx0, nx1), be = jc_pick(hi, ny0, ny1);
+    const double thr = tol * sqrt(al * be);      // NaN for a padding column (norm -1): never rotated
+    const double sc = jc_scale(fmax(al, be));
+    const double d = (be - al) * sc;
+    double a0 = 0, b0 = 0, a1 = 0, b1 = 0;
+#pragma unroll
+    for (int q = 0; q < E; q += 2) {
+        if (q < ET) {
+            a0 = fma(x0[q], y0[q], a0);
+            a1 = fma(x1[q], y1[q], a1);
+        }
+        if (q + 1 < E && q + 1 < ET) {
+            b0 = fma(x0[q + 1], y0[q + 1], b0);
+            b1 = fma(x1[q + 1], y1[q + 1], b1);
+        }
+    }
+    a0 += b0;
+    a1 += b1;
+    double g = jc_pick(hi, a0, a1) + __shfl_xor_sync(0xffffffffu, jc_pick(hi, a1, a0), 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+    const bool rot = g != 0.0 && fabs(g) > thr;
+    if (!__any_sync(0xffffffffu, rot)) return false;
+    // tan of the angle that orthogonalises the pair, |t| <= 1: t = 2g / (d + sign(d) sqrt(d^2 + 4 g^2))
+    const double g2 = 2.0 * g * sc;
+    const double h = sqrt(fma(d, d, g2 * g2));
+    double t = g2 / (d >= 0 ? d + h : d - h);
+    double c = rsqrt(fma(t, t, 1.0));
+    if (!rot) {
+        t = 0.0;
+        c = 1.0;
+    }
+    const double s = c * t;
+    const double na = rot ? fmax(fma(-t, g, al), 0.0) : al, nb = rot ? fmax(fma(t, g, be), 0.0) : be;
+    const double co = __shfl_xor_sync(0xffffffffu, c, 16), so = __shfl_xor_sync(0xffffffffu, s, 16);
+    const double nao = __shfl_xor_sync(0xffffffffu, na, 16), nbo = __shfl_xor_sync(0xffffffffu, nb, 16);
+    const double c0 = jc_pick(hi, c, co), s0 = jc_pick(hi, s, so), c1 = jc_pick(hi, co, c), s1 = jc_pick(hi, so, s);
+    nx0 = jc_pick(hi, na, nao);
+    ny0 = jc_pick(hi, nb, nbo);
+    nx1 = jc_pick(hi, nao, na);
+    ny1 = jc_pick(hi, nbo, nb);
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        const double u0 = x0[q], v0 = y0[q], u1 = x1[q], v1 = y1[q];
+        x0[q] = fma(c0, u0, -s0 * v0);
+        y0[q] = fma(s0, u0, c0 * v0);
+        x1[q] = fma(c1, u1, -s1 * v1);
+        y1[q] = fma(s1, u1, c1 * v1);
+    }
+    return true;
+}
+
+template <int E>
+__device__ __forceinline__ double jc_norm2(const double (&x)[E], int ET) {
+    double a = 0, b = 0;
+#pragma unroll
+    for (int q = 0; q < E; q += 2) {
+        if (q < ET) a = fma(x[q], x[q], a);
+        if (q + 1 < E && q + 1 < ET) b = fma(x[q + 1], x[q + 1], b);
+    }
+    return wsum(a + b);
+}
+
+// Doubles of one inbox slot: a block's two columns interleaved by lane (16-byte
+// accesses, no bank conflicts) and its two norms.
+template <int E> __host__ __device__ constexpr int jc_slot() { return 64 * E + 2; }
+
+template <int E>
+size_t jc_smem_bytes(int warps, int parities, int nmax) {
+    return sizeof(double) * ((size_t)jc_slot<E>() * 2 * warps * parities + (size_t)nmax + 2) + sizeof(int) * nmax;
+}
+
+template <int E>
+__global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __restrict__ jobs, SvdJob one,
+                                                                 int vectors, int parities, int nmax) {
+    extern __shared__ __align__(16) double smem[];
+    cg::cluster_group cl = cg::this_cluster();
+    const int ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const SvdJob jb = jobs ? jobs[blockIdx.x / ncta] : one;
+    const int m = jb.m, n = jb.n;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+    const int gw = rank * nw + wid;          // warp of the cluster
+    const int NW = max(1, (n + 3) / 4);      // warps that hold columns
+    const int ET = (m + 31) / 32;
+    const bool on = gw < NW;
+    __shared__ int flags[3];                 // rank 0's are used: "something rotated", by sweep modulo 3
+    __shared__ double red[32];
+    __shared__ int at[32];
+    constexpr int SLOT = jc_slot<E>();
+    double* inbox = smem;                    // [parity][warp][top, bottom][SLOT]
+    double* sig = smem + (size_t)SLOT * 2 * nw * parities;  // nmax
+    int* rk = reinterpret_cast<int*>(sig + nmax + 2);
+    if (tid < 3) flags[tid] = 0;
+    auto slot = [&](int dst, int which, int par) -> double* {  // inbox slot of cluster warp dst
+        const int r = dst / nw, w = dst - r * nw;
+        double* p = inbox + (size_t)SLOT * ((par * nw + w) * 2 + which);
+        return r == rank ? p : cl.map_shared_rank(p, r);
+    };
+    double x0[E], x1[E], y0[E], y1[E];       // top block, bottom block
+    double nx0, nx1, ny0, ny1;
+    auto load = [&](double(&v)[E], int col) -> double {
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            double e = 0.0;
+            if (on && col < n) {
+                const int row = lane + 32 * q;
+                if (q < ET) e = row < m ? jb.W[(size_t)col * m + row] : 0.0;
+                else if (vectors) e = (row - 32 * ET == col) ? 1.0 : 0.0;
+            }
+            v[q] = e;
+        }
+        return (on && col < n) ? 0.0 : -1.0;
+    };
+    nx0 = load(x0, 2 * gw);
+    nx1 = load(x1, 2 * gw + 1);
+    ny0 = load(y0, 2 * (NW + gw));
+    ny1 = load(y1, 2 * (NW + gw) + 1);
+    auto put = [&](double* p, const double(&a)[E], const double(&b)[E], double na, double nb) {
+#pragma unroll
+        for (int q = 0; q < E; ++q) reinterpret_cast<double2*>(p)[32 * q + lane] = make_double2(a[q], b[q]);
+        if (lane == 0) reinterpret_cast<double2*>(p)[32 * E] = make_double2(na, nb);
+    };
+    auto get = [&](const double* p, double(&a)[E], double(&b)[E], double& na, double& nb) {
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const double2 v = reinterpret_cast<const double2*>(p)[32 * q + lane];
+            a[q] = v.x;
+            b[q] = v.y;
+        }
+        const double2 v = reinterpret_cast<const double2*>(p)[32 * E];
+        na = v.x;
+        nb = v.y;
+    };
+    cl.sync();  // every CTA of the cluster runs before the first remote write; flags are zero
+
+    const double tol = 1e-15 * fmax(1.0, sqrt((double)m) / 4.0);
+    int sweep = 0, par = 0;
+    for (sweep = 0; sweep < SVD_MAX_SWEEPS && n > 1; ++sweep) {
+        bool rot = false;
+        if (on) {
+            if (nx0 >= 0) nx0 = jc_norm2(x0, ET);
+            if (nx1 >= 0) nx1 = jc_norm2(x1, ET);
+            if (ny0 >= 0) ny0 = jc_norm2(y0, ET);
+            if (ny1 >= 0) ny1 = jc_norm2(y1, ET);
+            rot |= jc_rotate2(x0, x1, y0, y1, nx0, nx1, ny0, ny1, ET, tol);  // inside the blocks
+        }
+        const int rounds = 2 * NW - 1;
+        for (int r = 0; r < rounds; ++r) {
+            if (on) {
+                rot |= jc_rotate2(x0, y0, x1, y1, nx0, ny0, nx1, ny1, ET, tol);
+                rot |= jc_rotate2(x0, y1, x1, y0, nx0, ny1, nx1, ny0, ET, tol);
+            }
+            if (parities == 1 && r + sweep > 0) cl.sync();  // the inboxes have been read
+            if (on && NW > 1) {
+                put(gw == 0 ? slot(1, 0, par) : slot(gw - 1, 1, par), y0, y1, ny0, ny1);
+                if (gw == NW - 1) {
+#pragma unroll
+                    for (int q = 0; q < E; ++q) {
+                        y0[q] = x0[q];
+                        y1[q] = x1[q];
+                    }
+                    ny0 = nx0;
+                    ny1 = nx1;
+                } else if (gw > 0) {
+                    put(slot(gw + 1, 0, par), x0, x1, nx0, nx1);
+                }
+            }
+            if (r == rounds - 1 && rot && lane == 0) *cl.map_shared_rank(&flags[sweep % 3], 0) = 1;
+            cl.sync();
+            if (r == 0 && rank == 0 && tid == 0) flags[(sweep + 2) % 3] = 0;  // read by all before this barrier
+            if (on && NW > 1) {
+                if (gw > 0) get(slot(gw, 0, par), x0, x1, nx0, nx1);
+                if (gw < NW - 1) get(slot(gw, 1, par), y0, y1, ny0, ny1);
+            }
+            if (parities > 1) par ^= 1;
+        }
+        if (!*cl.map_shared_rank(&flags[sweep % 3], 0)) break;  // the same value in every thread of the cluster
+    }
+
+    // singular values: every CTA gets all of them (slots 4 gw .. 4 gw + 3; padding columns -1)
+    if (on) {
+        const double s0 = nx0 < 0 ? -1.0 : sqrt(jc_norm2(x0, ET)), s1 = nx1 < 0 ? -1.0 : sqrt(jc_norm2(x1, ET));
+        const double s2 = ny0 < 0 ? -1.0 : sqrt(jc_norm2(y0, ET)), s3 = ny1 < 0 ? -1.0 : sqrt(jc_norm2(y1, ET));
+        if (lane < ncta) {
+            double* p = cl.map_shared_rank(sig, lane) + 4 * gw;
+            p[0] = s0;
+            p[1] = s1;
+            p[2] = s2;
+            p[3] = s3;
+        }
+    }
+    cl.sync();
+    // descending rank, ties broken by position
+    const int np = 4 * NW;
+    for (int j = tid; j < np; j += blockDim.x) {
+        const double sj = sig[j];
+        int k = 0;
+        for (int i = 0; i < np; ++i) {
+            const double si = sig[i];
+            k += (si > sj) || (si == sj && i < j);
+        }
+        rk[j] = sj < 0 ? -1 : k;
+        if (rank == 0 && !(sj < 0)) jb.s[min(k, n - 1)] = sj;
+    }
+    __syncthreads();
+    if (vectors) {
+        double smax = 0;
+        for (int j = 0; j < np; ++j) smax = fmax(smax, sig[j]);
+        const double cut = smax * 1e-13 * fmax(1.0, (double)m);
+        auto emit = [&](const double(&v)[E], int j) {
+            const int k = rk[j];
+            if (k < 0) return;
+            const double sj = sig[j];
+            const bool good = sj > cut && sj > 0.0;
+            double* uo = jb.U + (size_t)min(k, n - 1) * jb.ldu;
+            double* vo = jb.Vt + min(k, n - 1);
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+                const int row = lane + 32 * q;
+                if (q < ET) {
+                    if (row < m) uo[row] = good ? v[q] / sj : 0.0;
+                } else if (row - 32 * ET < n) {
+                    vo[(size_t)(row - 32 * ET) * jb.ldvt] = v[q];
+                }
+            }
+        };
+        if (on) {
+            emit(x0, 4 * gw);
+            emit(x1, 4 * gw + 1);
+            emit(y0, 4 * gw + 2);
+            emit(y1, 4 * gw + 3);
+        }
+        __threadfence();
+        cl.sync();
+        if (rank == 0) complete_u(jb, cut, red, sig, at);
+    }
+    if (rank == 0 && tid == 0 && jb.sweeps) *jb.sweeps = sweep;
+    cl.sync();  // no CTA leaves while its shared memory may still be addressed
+}
+
+// Cluster shape for the largest n and row-slot count of a batch; ncta = 0: not served.
+struct JcShape {
+    int ncta = 0, warps = 0;
+};
+JcShape jc_shape(int n, int slots) {
+    JcShape s;
+    if (slots > JC_SLOTS_MAX || n > 512) return s;
+    const int NW = std::max(1, (n + 3) / 4);
+    s.warps = NW <= 32 ? 4 : 8;
+    s.ncta = 1;
+    while (s.ncta * s.warps < NW) s.ncta *= 2;
+    return s;
+}
+
+template <int E>
+int jc_launch(Ctx& c, const SvdJob* dev_jobs, const SvdJob& one, int njobs, JcShape sh, int nmax, bool vectors,
+              bool* served) {
+    *served = false;
+    const size_t cap = 220 * 1024;
+    const int np = 4 * sh.ncta * sh.warps;
+    int parities = 2;
+    size_t smem = jc_smem_bytes<E>(sh.warps, 2, std::max(np, nmax));
+    if (smem > cap) {
+        parities = 1;
+        smem = jc_smem_bytes<E>(sh.warps, 1, std::max(np, nmax));
+    }
+    if (smem > cap) return TN_OK;
+    auto kern = jacobi_cluster_kernel<E>;
+    TN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    if (sh.ncta > 8) TN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(njobs * sh.ncta));
+    cfg.blockDim = dim3((unsigned)(32 * sh.warps));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)sh.ncta;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (sh.ncta > 8) {
+        int nc = 0;
+        if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) != cudaSuccess || nc < 1) {
+            cudaGetLastError();
+            return TN_OK;
+        }
+    }
+    TN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, dev_jobs, one, vectors ? 1 : 0, parities, std::max(np, nmax)));
+    TN_LAUNCH_CHECK();
+    *served = true;
+    return TN_OK;
 }
 
 }  // namespace
@@ -204,14 +593,44 @@ int svd_batched(Ctx& c, const std::vector<SvdJob>& jobs, bool vectors) {
             return TN_BAD_SHAPE;
         }
     }
-    TN_CHECK(c.svdw.ensure(sizeof(SvdJob) * jobs.size()));
-    TN_CUDA_CHECK(cudaMemcpyAsync(c.svdw.p, jobs.data(), sizeof(SvdJob) * jobs.size(), cudaMemcpyHostToDevice,
-                                  c.stream));
-    const size_t cap = 200 * 1024;
-    TN_CUDA_CHECK(cudaFuncSetAttribute(jacobi_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-    jacobi_svd_kernel<<<(unsigned)jobs.size(), SVD_THREADS, cap, c.stream>>>(c.svdw.as<SvdJob>(), vectors ? 1 : 0,
-                                                                             cap);
-    TN_LAUNCH_CHECK();
+    const SvdJob* dev = nullptr;  // a single job travels as a kernel argument
+    if (jobs.size() > 1) {
+        TN_CHECK(c.svdw.ensure(sizeof(SvdJob) * jobs.size()));
+        TN_CUDA_CHECK(cudaMemcpyAsync(c.svdw.p, jobs.data(), sizeof(SvdJob) * jobs.size(), cudaMemcpyHostToDevice,
+                                      c.stream));
+        dev = c.svdw.as<SvdJob>();
+    }
+    int nmax = 1, slots = 1;
+    for (const auto& j : jobs) {
+        nmax = std::max(nmax, j.n);
+        slots = std::max(slots, (j.m + 31) / 32 + (vectors ? (j.n + 31) / 32 : 0));
+    }
+    // Every job of the batch fits the cluster kernel (n <= 512 and at most 16
+    // slots of 32 rows per column, rows of U and V together): there it is the
+    // faster one at every size (150 x 128 with vectors: @@); otherwise one CTA
+    // per matrix with its columns in shared memory or L2.
+    const JcShape sh = jc_shape(nmax, slots);
+    bool served = false;
+    const int nj = (int)jobs.size();
+    if (sh.ncta > 0) {
+        if (slots <= 2) TN_CHECK(jc_launch<2>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
+        else if (slots <= 4) TN_CHECK(jc_launch<4>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
+        else if (slots <= 6) TN_CHECK(jc_launch<6>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
+        else if (slots <= 8) TN_CHECK(jc_launch<8>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
+        else if (slots <= 12) TN_CHECK(jc_launch<12>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
+        else TN_CHECK(jc_launch<16>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
+    }
+    if (!served) {
+        if (!dev) {
+            TN_CHECK(c.svdw.ensure(sizeof(SvdJob)));
+            TN_CUDA_CHECK(cudaMemcpyAsync(c.svdw.p, jobs.data(), sizeof(SvdJob), cudaMemcpyHostToDevice, c.stream));
+            dev = c.svdw.as<SvdJob>();
+        }
+        const size_t cap = 200 * 1024;
+        TN_CUDA_CHECK(cudaFuncSetAttribute(jacobi_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        jacobi_svd_kernel<<<(unsigned)jobs.size(), SVD_THREADS, cap, c.stream>>>(dev, vectors ? 1 : 0, cap);
+        TN_LAUNCH_CHECK();
+    }
     // the job array must stay valid until the kernel has read it
     TN_CUDA_CHECK(cudaStreamSynchronize(c.stream));
     return TN_OK;
