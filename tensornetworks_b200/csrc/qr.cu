@@ -991,10 +991,7 @@ int qr_persistent(Ctx& c, int m, int n, double* W, double* Qout, int ldq, double
     if (G < 2) return QRP_UNAVAILABLE;
     const size_t words = 4 + (size_t)nwb + (size_t)nqb;
     TN_CHECK(c.qrsync.ensure(sizeof(int) * words));
-    if (!c.derr.p) {
-        TN_CHECK(c.derr.ensure(sizeof(int)));
-        TN_CUDA_CHECK(cudaMemset(c.derr.p, 0, sizeof(int)));
-    }
+    TN_CHECK(ensure_device_error_word(c));
     double* Qt = nullptr;
     if (fwdq) {
         TN_CHECK(c.qaccum.ensure(sizeof(double) * (size_t)m * m));
@@ -1442,13 +1439,28 @@ int qr_tall(Ctx& c, int m, int n, double* W, double* Qout, int ldq, double* Rout
 
 }  // namespace
 
+int ensure_device_error_word(Ctx& c) {
+    if (c.derr.p) return TN_OK;
+    TN_CHECK(c.derr.ensure(sizeof(int)));
+    TN_CUDA_CHECK(cudaMemset(c.derr.p, 0, sizeof(int)));
+    return TN_OK;
+}
+
+int check_device_error_on_stream(Ctx& c) {
+    TN_CHECK(c.derr_host.ensure(sizeof(int)));
+    int* h = reinterpret_cast<int*>(c.derr_host.p);
+    TN_CUDA_CHECK(cudaMemcpyAsync(h, c.derr.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    TN_CUDA_CHECK(cudaStreamSynchronize(c.stream));
+    return *h ? check_device_error(c) : TN_OK;
+}
+
 int check_device_error(Ctx& c) {
     if (!c.derr.p) return TN_OK;
     int h = 0;
     TN_CUDA_CHECK(cudaMemcpy(&h, c.derr.p, sizeof(int), cudaMemcpyDeviceToHost));
     if (!h) return TN_OK;
     TN_CUDA_CHECK(cudaMemset(c.derr.p, 0, sizeof(int)));
-    set_error("a bounded wait between the CTAs of the persistent QR expired");
+    set_error("a bounded wait between the CTAs of a kernel expired");
     return TN_CUDA_ERROR;
 }
 

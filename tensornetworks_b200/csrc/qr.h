@@ -11,8 +11,12 @@ int qr_dense(Ctx& c, int m, int n, double* W, double* Qout, int ldq, double* Rou
 // Reads (and clears) the context's sticky device error word, raised when a
 // bounded wait between CTAs expired; waits for the device.
 int check_device_error(Ctx& c);
+// The same by a copy on the context stream, which it then waits for.
+int check_device_error_on_stream(Ctx& c);
+// The error word allocated and zero (before the first kernel that may raise it).
+int ensure_device_error_word(Ctx& c);
 
-// One job of the batched one-sided Jacobi SVD (one CTA per job).  W is the
+// One job of the batched one-sided Jacobi SVD (one cluster or CTA per job).  W is the
 // tall (m >= n) working copy, overwritten.  With vectors: U (m x n, ldu),
 // Vt (n x n, ldvt) and a scratch V (n x n, ld n).  s (n) is always written.
 struct SvdJob {

@@ -197,6 +197,7 @@ struct Ctx {
     DevBuf apiw[3];        // staging copies of the dense-solver entry points
     DevBuf cqr, rr1, rr2;  // RQ / QL factor staging; rank-revealing factorisations' full factors
     HostBuf pinned;
+    HostBuf derr_host;     // landing place of the error word
     int sm_count = 148;
     bool use_persistent_qr = true;  // TN_NO_PERSISTENT_QR=1: the two-stream look-ahead QR instead
     bool qr_forward_q = true;       // TN_QR_FORWARD_Q=0: the persistent QR forms the thin Q after the panels
