@@ -110,12 +110,17 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(GemmArgs g) {
 
 // ---------------------------------------------------------------------------
 // FP64 tensor-core path: mma.sync m8n8k4 (DMMA), for operands whose index maps
-// are plain strides over the ranges used (no split indices).  CTA tile 64x64,
-// 4 warps each owning a 32x32 quarter (4x4 MMA tiles, 32 accumulators per
-// thread), k-tiles of 16 staged in shared memory with the next tile
-// prefetched into registers.  The shared row stride 68 (= 4 mod 16 doubles)
-// makes the fragment loads of a half-warp hit 16 distinct bank pairs.
-constexpr int TBM = 64, TBN = 64, TBK = 16, TNT = 128, TLD = TBM + 4;
+// are plain strides over the ranges used (no split indices).  CTA tile
+// BM x BN, four warps in a 2 x 2 grid, k-tiles of 16 in a ring of DG_STAGES
+// shared-memory stages filled by asynchronous copies (one barrier per k-tile;
+// the copies of the next two tiles are in flight behind the products).  An
+// operand keeps its contiguous index contiguous in shared memory, [k][m] or
+// [m][k], with rows of 4 mod 16 doubles: the fragment loads of a half warp
+// then hit 16 distinct bank pairs in both forms, and copies are 16 bytes
+// where base, strides and batch strides allow it (V = 2), 8 otherwise.
+// Bound: the FP64 pipe (37 TFLOP/s); what keeps smaller products off it is
+// the number of tiles per SM and the pipeline's fill.
+constexpr int DG_BK = 16, DG_STAGES = 3, DG_NT = 128;
 
 struct LinGemm {
     int M, N, K, nb1;
@@ -133,81 +138,130 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-// WM: rows of a warp's tile (32: CTA tile 64 x 64; 16: 32 x 64, twice the
-// CTAs for grids that would leave SMs idle or run one latency-bound CTA each).
-template <int WM, bool A_MCONTIG, bool B_KCONTIG>
-__global__ void __launch_bounds__(TNT) gemm_f64_dmma_kernel(LinGemm g) {
-    constexpr int BMT = 2 * WM, LDA = BMT + 4, RA = BMT * TBK / TNT, MI = WM / 8;
+// V doubles to shared memory, the first `valid` of them read, zeros for the rest
+template <int V>
+__device__ __forceinline__ void dg_copy(double* dst, const double* src, int valid) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if (V == 2)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(8 * valid) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(8 * valid) : "memory");
+}
+
+// One operand's share of the pipeline.  X x DG_BK elements per stage, x the row
+// index of A or the column index of B; XC: x is the contiguous one.
+template <int X, bool XC, int V>
+struct DgOperand {
+    static constexpr int LD = XC ? X + 4 : DG_BK + 4;
+    static constexpr int STAGE = XC ? DG_BK * LD : X * LD;
+    static constexpr int N = X * DG_BK / V / DG_NT;  // copies per thread
+    const double* src[N];
+    int xleft[N];  // valid elements along x at the copy's place
+    int dst[N], kk[N];
+    long long step;
+    __device__ __forceinline__ void init(const double* base, long long sx, long long sk, int x0, int nx) {
+        step = DG_BK * sk;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int e = threadIdx.x + DG_NT * i;
+            int x, k;
+            if (XC) {
+                x = e % (X / V) * V;
+                k = e / (X / V);
+                dst[i] = k * LD + x;
+            } else {
+                k = e % (DG_BK / V) * V;
+                x = e / (DG_BK / V);
+                dst[i] = x * LD + k;
+            }
+            xleft[i] = nx - x0 - x;
+            kk[i] = k;
+            src[i] = base + (xleft[i] > 0 ? (long long)(x0 + x) * sx : 0) + (long long)k * sk;
+        }
+    }
+    // the stage of k-tile k0 (kleft = K - k0), then on to the next
+    __device__ __forceinline__ void load(double* stage, const double* safe, int kleft) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int along = XC ? xleft[i] : kleft - kk[i];
+            const bool in = xleft[i] > 0 && kk[i] < kleft;
+            const int valid = in ? (along < V ? along : V) : 0;
+            dg_copy<V>(stage + dst[i], valid > 0 ? src[i] : safe, valid);
+            src[i] += step;
+        }
+    }
+    __device__ static __forceinline__ double get(const double* stage, int x, int k) {
+        return XC ? stage[k * LD + x] : stage[x * LD + k];
+    }
+};
+
+template <int BM, int BN, bool A_MC, bool B_KC, int V>
+constexpr int dg_smem_bytes() {
+    return (int)sizeof(double) * DG_STAGES * (DgOperand<BM, A_MC, V>::STAGE + DgOperand<BN, !B_KC, V>::STAGE);
+}
+
+template <int BM, int BN, bool A_MC, bool B_KC, int V>
+__global__ void __launch_bounds__(DG_NT) gemm_f64_dmma_kernel(LinGemm g) {
+    constexpr int WM = BM / 2, WN = BN / 2, MI = WM / 8, NI = WN / 8;
+    using OpA = DgOperand<BM, A_MC, V>;
+    using OpB = DgOperand<BN, !B_KC, V>;
     if (g.skip && *g.skip) return;
-    __shared__ double As[TBK][LDA];
-    __shared__ double Bs[TBK][TLD];
+    extern __shared__ __align__(16) double dg_smem[];
+    double* As = dg_smem;
+    double* Bs = dg_smem + DG_STAGES * OpA::STAGE;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int gid = lane >> 2, tig = lane & 3;
-    const int wm = (warp >> 1) * WM, wn = (warp & 1) * 32;
-    const int m0 = blockIdx.y * BMT, n0 = blockIdx.x * TBN;
+    const int wm = (warp >> 1) * WM, wn = (warp & 1) * WN;
+    const int mt = (g.M + BM - 1) / BM;  // tiles of one column of C in a row
+    const int m0 = blockIdx.x % mt * BM, n0 = blockIdx.x / mt * BN;
     const int b = blockIdx.z;
     const int b0 = b / g.nb1, b1 = b - b0 * g.nb1;
     const double* Ab = g.A + b0 * g.sA0 + b1 * g.sA1;
     const double* Bb = g.B + b0 * g.sB0 + b1 * g.sB1;
-    // tile slots: RA per thread for A (TBK x BMT), 8 for B (TBK x TBN)
-    double ra[RA], rb[8];
-    auto load = [&](int k0) {
-#pragma unroll
-        for (int r = 0; r < RA; ++r) {
-            const int e = t + TNT * r;
-            int am, ak;
-            if (A_MCONTIG) { am = e % BMT; ak = e / BMT; } else { ak = e % TBK; am = e / TBK; }
-            const int gm = m0 + am, gk = k0 + ak;
-            ra[r] = (gm < g.M && gk < g.K) ? __ldg(Ab + gm * g.sAm + gk * g.sAk) : 0.0;
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int e = t + TNT * r;
-            int bk, bn;
-            if (B_KCONTIG) { bk = e % TBK; bn = e / TBK; } else { bn = e % TBN; bk = e / TBN; }
-            const int hk = k0 + bk, gn = n0 + bn;
-            rb[r] = (gn < g.N && hk < g.K) ? __ldg(Bb + hk * g.sBk + gn * g.sBn) : 0.0;
-        }
-    };
-    auto store = [&]() {
-#pragma unroll
-        for (int r = 0; r < RA; ++r) {
-            const int e = t + TNT * r;
-            int am, ak;
-            if (A_MCONTIG) { am = e % BMT; ak = e / BMT; } else { ak = e % TBK; am = e / TBK; }
-            As[ak][am] = ra[r];
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int e = t + TNT * r;
-            int bk, bn;
-            if (B_KCONTIG) { bk = e % TBK; bn = e / TBK; } else { bn = e % TBN; bk = e / TBN; }
-            Bs[bk][bn] = rb[r];
-        }
-    };
-    double acc[MI][4][2];
+    OpA oa;
+    OpB ob;
+    oa.init(Ab, g.sAm, g.sAk, m0, g.M);
+    ob.init(Bb, g.sBn, g.sBk, n0, g.N);
+    double acc[MI][NI][2];
 #pragma unroll
     for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    load(0);
-    for (int k0 = 0; k0 < g.K; k0 += TBK) {
-        store();
-        __syncthreads();
-        if (k0 + TBK < g.K) load(k0 + TBK);
+        for (int j = 0; j < NI; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    const int ntile = (g.K + DG_BK - 1) / DG_BK;
 #pragma unroll
-        for (int ks = 0; ks < TBK; ks += 4) {
-            double af[MI], bf[4];
+    for (int s = 0; s < DG_STAGES - 1; ++s) {
+        if (s < ntile) {
+            oa.load(As + s * OpA::STAGE, Ab, g.K - s * DG_BK);
+            ob.load(Bs + s * OpB::STAGE, Bb, g.K - s * DG_BK);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    int rd = 0, wr = DG_STAGES - 1;
+    for (int kt = 0; kt < ntile; ++kt) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(DG_STAGES - 2) : "memory");
+        __syncthreads();  // tile kt has arrived for all threads, and stage wr has been read by all
+        if (kt + DG_STAGES - 1 < ntile) {
+            const int kleft = g.K - (kt + DG_STAGES - 1) * DG_BK;
+            oa.load(As + wr * OpA::STAGE, Ab, kleft);
+            ob.load(Bs + wr * OpB::STAGE, Bb, kleft);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const double* a = As + rd * OpA::STAGE;
+        const double* bb = Bs + rd * OpB::STAGE;
 #pragma unroll
-            for (int i = 0; i < MI; ++i) af[i] = As[ks + tig][wm + i * 8 + gid];  // A(row gid, col tig)
+        for (int ks = 0; ks < DG_BK; ks += 4) {
+            double af[MI], bf[NI];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) bf[j] = Bs[ks + tig][wn + j * 8 + gid];  // B(row tig, col gid)
+            for (int i = 0; i < MI; ++i) af[i] = OpA::get(a, wm + i * 8 + gid, ks + tig);  // A(row gid, col tig)
+#pragma unroll
+            for (int j = 0; j < NI; ++j) bf[j] = OpB::get(bb, wn + j * 8 + gid, ks + tig);  // B(row tig, col gid)
 #pragma unroll
             for (int i = 0; i < MI; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dmma(acc[i][j], af[i], bf[j]);
+                for (int j = 0; j < NI; ++j) dmma(acc[i][j], af[i], bf[j]);
         }
-        __syncthreads();
+        rd = rd + 1 == DG_STAGES ? 0 : rd + 1;
+        wr = wr + 1 == DG_STAGES ? 0 : wr + 1;
     }
     double* Cb = g.C + b0 * g.sC0 + b1 * g.sC1;
 #pragma unroll
@@ -215,7 +269,7 @@ __global__ void __launch_bounds__(TNT) gemm_f64_dmma_kernel(LinGemm g) {
         const int gm = m0 + wm + i * 8 + gid;
         if (gm >= g.M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < NI; ++j)
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int gn = n0 + wn + j * 8 + tig * 2 + q;
@@ -226,6 +280,50 @@ __global__ void __launch_bounds__(TNT) gemm_f64_dmma_kernel(LinGemm g) {
                 *c = v;
             }
     }
+}
+
+template <int BM, int BN, bool A_MC, bool B_KC, int V>
+int dg_launch(const LinGemm& l, int batches, cudaStream_t st) {
+    constexpr int bytes = dg_smem_bytes<BM, BN, A_MC, B_KC, V>();
+    auto kern = gemm_f64_dmma_kernel<BM, BN, A_MC, B_KC, V>;
+    if (bytes > 48 * 1024) {
+        static thread_local int dev_set = -1;
+        int dev = 0;
+        TN_CUDA_CHECK(cudaGetDevice(&dev));
+        if (dev_set != dev) {
+            TN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            dev_set = dev;
+        }
+    }
+    const long long tiles = (long long)((l.N + BN - 1) / BN) * ((l.M + BM - 1) / BM);
+    if (tiles > 0x7fffffffLL) {
+        set_error("gemm_f64: grid too large");
+        return TN_BAD_SHAPE;
+    }
+    const dim3 grid((unsigned)tiles, 1, batches);
+    kern<<<grid, DG_NT, bytes, st>>>(l);
+    TN_LAUNCH_CHECK();
+    return TN_OK;
+}
+
+template <int BM, int BN>
+int dg_dispatch(const LinGemm& l, int batches, bool amc, bool bkc, bool wide, cudaStream_t st) {
+    if (wide) {
+        if (amc && bkc) return dg_launch<BM, BN, true, true, 2>(l, batches, st);
+        if (amc) return dg_launch<BM, BN, true, false, 2>(l, batches, st);
+        if (bkc) return dg_launch<BM, BN, false, true, 2>(l, batches, st);
+        return dg_launch<BM, BN, false, false, 2>(l, batches, st);
+    }
+    if (amc && bkc) return dg_launch<BM, BN, true, true, 1>(l, batches, st);
+    if (amc) return dg_launch<BM, BN, true, false, 1>(l, batches, st);
+    if (bkc) return dg_launch<BM, BN, false, true, 1>(l, batches, st);
+    return dg_launch<BM, BN, false, false, 1>(l, batches, st);
+}
+
+// 16-byte copies: the contiguous index has stride 1, and the base and every
+// other stride keep 16-byte alignment.
+inline bool wide_operand(const double* p, long long contiguous, long long other, long long s0, long long s1) {
+    return contiguous == 1 && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ((other | s0 | s1) & 1) == 0;
 }
 
 // An index map that is a plain stride over [0, n).
@@ -255,29 +353,23 @@ int gemm_f64(const GemmArgs& g, cudaStream_t st) {
         l.sAm = g.A.mn.s; l.sAk = g.A.k.s; l.sBk = g.B.k.s; l.sBn = g.B.mn.s; l.sCm = g.C.m.s; l.sCn = g.C.n.s;
         l.sA0 = g.A.sb0; l.sA1 = g.A.sb1; l.sB0 = g.B.sb0; l.sB1 = g.B.sb1; l.sC0 = g.C.sb0; l.sC1 = g.C.sb1;
         l.A = g.A.ptr; l.B = g.B.ptr; l.C = g.C.ptr; l.alpha = g.alpha; l.beta = g.beta; l.skip = g.skip;
-        // 64 x 64 CTA tiles, or 32 x 64 when that grid would not fill two CTAs per SM
+        const bool wide = wide_operand(l.A, amc ? l.sAm : l.sAk, amc ? l.sAk : l.sAm, l.sA0, l.sA1) &&
+                          wide_operand(l.B, bkc ? l.sBk : l.sBn, bkc ? l.sBn : l.sBk, l.sB0, l.sB1);
         static int sms = 0;
         if (sms == 0) {
             int dev = 0;
             cudaGetDevice(&dev);
             if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
         }
-        const long long tiles64 = (long long)((g.N + TBN - 1) / TBN) * ((g.M + TBM - 1) / TBM) * g.nb0 * g.nb1;
-        if (tiles64 < 2LL * sms) {
-            dim3 tg((g.N + TBN - 1) / TBN, (g.M + 31) / 32, g.nb0 * g.nb1);
-            if (amc && bkc) gemm_f64_dmma_kernel<16, true, true><<<tg, TNT, 0, st>>>(l);
-            else if (amc && !bkc) gemm_f64_dmma_kernel<16, true, false><<<tg, TNT, 0, st>>>(l);
-            else if (!amc && bkc) gemm_f64_dmma_kernel<16, false, true><<<tg, TNT, 0, st>>>(l);
-            else gemm_f64_dmma_kernel<16, false, false><<<tg, TNT, 0, st>>>(l);
-        } else {
-            dim3 tg((g.N + TBN - 1) / TBN, (g.M + TBM - 1) / TBM, g.nb0 * g.nb1);
-            if (amc && bkc) gemm_f64_dmma_kernel<32, true, true><<<tg, TNT, 0, st>>>(l);
-            else if (amc && !bkc) gemm_f64_dmma_kernel<32, true, false><<<tg, TNT, 0, st>>>(l);
-            else if (!amc && bkc) gemm_f64_dmma_kernel<32, false, true><<<tg, TNT, 0, st>>>(l);
-            else gemm_f64_dmma_kernel<32, false, false><<<tg, TNT, 0, st>>>(l);
-        }
-        TN_LAUNCH_CHECK();
-        return TN_OK;
+        // 32 x 32 tiles until 32 x 64 ones give every SM eight: below that the
+        // finer split wins by what the last round of tiles leaves idle (10 x 256^3:
+        // 18.5 us against 20.5 with 32 x 64 and 24.6 with 64 x 64; 10 x 250 x 203 x 250:
+        // 16.4, 22.6, 24.6; 15 x 90^3: 6.2, 8.3, 10.3), above it the wider one by its
+        // operand reuse (15 x 512^3: 133 us against 137).
+        const int nb = g.nb0 * g.nb1;
+        const long long tiles = (long long)((g.N + 63) / 64) * ((g.M + 31) / 32) * nb;
+        if (tiles >= 8LL * sms) return dg_dispatch<32, 64>(l, nb, amc, bkc, wide, st);
+        return dg_dispatch<32, 32>(l, nb, amc, bkc, wide, st);
     }
     if (amc && bkc) gemm_f64_kernel<true, true><<<grid, NT, 0, st>>>(g);
     else if (amc && !bkc) gemm_f64_kernel<true, false><<<grid, NT, 0, st>>>(g);
