@@ -7,6 +7,7 @@
 #include <string>
 
 #include "engine.h"
+#include "lzsite.h"
 #include "mixed.h"
 #include "itebd.h"
 #include "ed.h"
@@ -636,8 +637,24 @@ int tn_eigensolve_heff(tn_ctx c, const tn_solver_options* opt, int d, int Dw1, i
         return r.converged ? TN_OK : TN_NOT_CONVERGED;
     }
     LzResult r{};
-    TN_CHECK(lanczos_solve(cx, N, x, krylov, restarts, tol, mv, &r));
-    TN_CUDA_CHECK(cudaStreamSynchronize(cx.stream));
+    TN_CHECK(cx.pinned.ensure(sizeof(LzSummary)));
+    LzSummary* sum = reinterpret_cast<LzSummary*>(cx.pinned.p);
+    const int rc = lanczos_site(cx, s, t, nt, F, G, x, krylov, restarts, tol, 0.0, sum);
+    if (rc == LZ_SITE_UNAVAILABLE) {
+        TN_CHECK(lanczos_solve(cx, N, x, krylov, restarts, tol, mv, &r));
+        TN_CUDA_CHECK(cudaStreamSynchronize(cx.stream));
+    } else {
+        TN_CHECK(rc);
+        TN_CHECK(check_device_error_on_stream(cx));
+        if (!std::isfinite(sum->theta)) {
+            set_error("lanczos: non-finite Ritz value");
+            return TN_NAN_DETECTED;
+        }
+        r.theta = sum->theta;
+        r.resid = sum->resid;
+        r.matvecs = sum->matvecs;
+        r.converged = sum->converged;
+    }
     if (theta) *theta = r.theta;
     if (residual) *residual = r.resid;
     if (matvecs) *matvecs = r.matvecs;

@@ -24,6 +24,7 @@
 #include <random>
 
 #include "engine.h"
+#include "lzsite.h"
 #include "host_linalg.h"
 
 namespace tnb {
@@ -963,8 +964,9 @@ int MPSState::refine_site(int ia, double epsEigen) {
         // (its FP64 Ritz value is the site energy) is read once per half-sweep
         TN_CHECK(rq_slots());
         LzSummary* slot = reinterpret_cast<LzSummary*>(reinterpret_cast<double*>(rqhost.p) + RQ_SLOT * (size_t)ia + 4);
-        const int rc = lanczos_solve_async(*ctx, N, A[ia]->as<double>(), krylov, restarts, epsEigen, mv, tol_rel, key,
-                                           slot);
+        int rc = lanczos_site(*ctx, s, t, op.nLR, F, G, A[ia]->as<double>(), krylov, restarts, epsEigen, tol_rel, slot);
+        if (rc == LZ_SITE_UNAVAILABLE)
+            rc = lanczos_solve_async(*ctx, N, A[ia]->as<double>(), krylov, restarts, epsEigen, mv, tol_rel, key, slot);
         if (rc == TN_OK) {
             rq_lz[ia] = 1;
             rq_exact[ia] = 1;

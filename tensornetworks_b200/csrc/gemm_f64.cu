@@ -7,6 +7,7 @@
 // Plain strided operands take the FP64 tensor-core (DMMA) kernel below;
 // split-index operands the SIMT kernel: tile 64x64x16, 256 threads, 4x4
 // outputs per thread, register-staged double buffering of the next k-tile.
+#include "dgemm.cuh"
 #include "tn_internal.h"
 
 namespace tnb {
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(GemmArgs g) {
 // where base, strides and batch strides allow it (V = 2), 8 otherwise.
 // Bound: the FP64 pipe (37 TFLOP/s); what keeps smaller products off it is
 // the number of tiles per SM and the pipeline's fill.
-constexpr int DG_BK = 16, DG_STAGES = 3, DG_NT = 128;
+constexpr int DG_STAGES = 3, DG_NT = 128;
 
 struct LinGemm {
     int M, N, K, nb1;
@@ -132,79 +133,16 @@ struct LinGemm {
     const int* skip;
 };
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
-
-// V doubles to shared memory, the first `valid` of them read, zeros for the rest
-template <int V>
-__device__ __forceinline__ void dg_copy(double* dst, const double* src, int valid) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    if (V == 2)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(8 * valid) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(8 * valid) : "memory");
-}
-
-// One operand's share of the pipeline.  X x DG_BK elements per stage, x the row
-// index of A or the column index of B; XC: x is the contiguous one.
-template <int X, bool XC, int V>
-struct DgOperand {
-    static constexpr int LD = XC ? X + 4 : DG_BK + 4;
-    static constexpr int STAGE = XC ? DG_BK * LD : X * LD;
-    static constexpr int N = X * DG_BK / V / DG_NT;  // copies per thread
-    const double* src[N];
-    int xleft[N];  // valid elements along x at the copy's place
-    int dst[N], kk[N];
-    long long step;
-    __device__ __forceinline__ void init(const double* base, long long sx, long long sk, int x0, int nx) {
-        step = DG_BK * sk;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const int e = threadIdx.x + DG_NT * i;
-            int x, k;
-            if (XC) {
-                x = e % (X / V) * V;
-                k = e / (X / V);
-                dst[i] = k * LD + x;
-            } else {
-                k = e % (DG_BK / V) * V;
-                x = e / (DG_BK / V);
-                dst[i] = x * LD + k;
-            }
-            xleft[i] = nx - x0 - x;
-            kk[i] = k;
-            src[i] = base + (xleft[i] > 0 ? (long long)(x0 + x) * sx : 0) + (long long)k * sk;
-        }
-    }
-    // the stage of k-tile k0 (kleft = K - k0), then on to the next
-    __device__ __forceinline__ void load(double* stage, const double* safe, int kleft) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const int along = XC ? xleft[i] : kleft - kk[i];
-            const bool in = xleft[i] > 0 && kk[i] < kleft;
-            const int valid = in ? (along < V ? along : V) : 0;
-            dg_copy<V>(stage + dst[i], valid > 0 ? src[i] : safe, valid);
-            src[i] += step;
-        }
-    }
-    __device__ static __forceinline__ double get(const double* stage, int x, int k) {
-        return XC ? stage[k * LD + x] : stage[x * LD + k];
-    }
-};
-
 template <int BM, int BN, bool A_MC, bool B_KC, int V>
 constexpr int dg_smem_bytes() {
-    return (int)sizeof(double) * DG_STAGES * (DgOperand<BM, A_MC, V>::STAGE + DgOperand<BN, !B_KC, V>::STAGE);
+    return (int)sizeof(double) * DG_STAGES * (DgOperand<BM, A_MC, V, DG_NT>::STAGE + DgOperand<BN, !B_KC, V, DG_NT>::STAGE);
 }
 
 template <int BM, int BN, bool A_MC, bool B_KC, int V>
 __global__ void __launch_bounds__(DG_NT) gemm_f64_dmma_kernel(LinGemm g) {
     constexpr int WM = BM / 2, WN = BN / 2, MI = WM / 8, NI = WN / 8;
-    using OpA = DgOperand<BM, A_MC, V>;
-    using OpB = DgOperand<BN, !B_KC, V>;
+    using OpA = DgOperand<BM, A_MC, V, DG_NT>;
+    using OpB = DgOperand<BN, !B_KC, V, DG_NT>;
     if (g.skip && *g.skip) return;
     extern __shared__ __align__(16) double dg_smem[];
     double* As = dg_smem;
@@ -220,8 +158,8 @@ __global__ void __launch_bounds__(DG_NT) gemm_f64_dmma_kernel(LinGemm g) {
     const double* Bb = g.B + b0 * g.sB0 + b1 * g.sB1;
     OpA oa;
     OpB ob;
-    oa.init(Ab, g.sAm, g.sAk, m0, g.M);
-    ob.init(Bb, g.sBn, g.sBk, n0, g.N);
+    oa.init(t, Ab, g.sAm, g.sAk, m0, g.M);
+    ob.init(t, Bb, g.sBn, g.sBk, n0, g.N);
     double acc[MI][NI][2];
 #pragma unroll
     for (int i = 0; i < MI; ++i)

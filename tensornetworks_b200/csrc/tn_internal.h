@@ -185,6 +185,7 @@ struct Ctx {
     DevBuf lz;             // Lanczos basis + work vectors
     DevBuf lzsum;          // summary of a device-driven Lanczos solve
     DevBuf lzstate;        // Lanczos device state
+    DevBuf lzbar;          // barrier counter of the one-launch site solve
     DevBuf rq;             // Rayleigh-quotient state + partials
     DevBuf dv, dvstate;    // Davidson basis + work vectors, device state
     DevBuf qrw;            // QR workspace
