@@ -63,9 +63,42 @@ int DevBuf::ensure(size_t nbytes) {
 }
 
 void DevBuf::release() {
-    if (p) cudaFree(p);
+    if (p && !part) cudaFree(p);
     p = nullptr;
     bytes = 0;
+    part = false;
+}
+
+int slab_reserve(const std::vector<DevBuf*>& v, const std::vector<size_t>& need, DevBuf& slab) {
+    bool enough = true;
+    size_t total = 0;
+    std::vector<size_t> size(v.size());
+    for (size_t i = 0; i < v.size(); ++i) {
+        enough = enough && v[i]->bytes >= need[i];
+        size[i] = std::max(need[i], v[i]->bytes);
+        total += (size[i] + 255) / 256 * 256;
+    }
+    if (enough) return TN_OK;
+    TN_CUDA_CHECK(cudaDeviceSynchronize());  // whatever still uses the buffers, on any stream
+    DevBuf fresh;
+    TN_CHECK(fresh.ensure(total));
+    char* at = fresh.as<char>();
+    for (size_t i = 0; i < v.size(); ++i) {
+        if (v[i]->p) TN_CUDA_CHECK(cudaMemcpy(at, v[i]->p, v[i]->bytes, cudaMemcpyDeviceToDevice));
+        at += (size[i] + 255) / 256 * 256;
+    }
+    TN_CUDA_CHECK(cudaDeviceSynchronize());
+    at = fresh.as<char>();
+    for (size_t i = 0; i < v.size(); ++i) {
+        v[i]->release();
+        v[i]->p = at;
+        v[i]->bytes = size[i];
+        v[i]->part = true;
+        at += (size[i] + 255) / 256 * 256;
+    }
+    std::swap(slab.p, fresh.p);
+    std::swap(slab.bytes, fresh.bytes);
+    return TN_OK;
 }
 
 int HostBuf::ensure(size_t nbytes) {
@@ -297,6 +330,7 @@ int tn_mps_destroy(tn_mps m) {
     if (!m) return TN_BAD_ARG;
     TN_ON_DEVICE(m->m.ctx->device);
     cudaStreamSynchronize(m->m.ctx->stream);
+    if (m->m.ctx->aux2) cudaStreamSynchronize(m->m.ctx->aux2);
     delete m;
     return TN_OK;
 }

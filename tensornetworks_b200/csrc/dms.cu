@@ -103,7 +103,7 @@ int MPSState::two_site_dms(double* out_host) {
             TN_CHECK(gemm_f64(g, st));
             // rho(m, m2; n, n2) = <A_m2, T[(mn) d + n2]>                       (FinializeTwoSiteDM)
             // dots[m2 * (dd d) + (mn) d + n2]
-            DevBuf& dots = tmp;
+            DevBuf& dots = scratch->tmp;
             TN_CHECK(dots.ensure(sizeof(double) * (size_t)d * dd * d));
             pair_dot_kernel<<<d * dd * d, 256, 0, st>>>(A[ib]->as<double>(), blk, d, Tb.as<double>(), blk, dd * d,
                                                         blk, dots.as<double>());
@@ -119,6 +119,7 @@ int MPSState::two_site_dms(double* out_host) {
                 TN_CHECK(gemm_f64(h, st));
                 std::swap(Cb.p, Cn.p);
                 std::swap(Cb.bytes, Cn.bytes);
+                std::swap(Cb.part, Cn.part);
             }
         }
         TN_CHECK(normalize_site(ia, true));

@@ -281,7 +281,13 @@ int Hamiltonian::build() {
 // ---------------------------------------------------------------------------
 // MPS
 // ---------------------------------------------------------------------------
+void MpsScratchDelete::operator()(MpsScratch* s) const { delete s; }
+
 MPSState::~MPSState() {
+    if (ctx && scratch) {  // the work buffers go to the next MPS of this context
+        std::lock_guard<std::mutex> lk(ctx->spare_mu);
+        ctx->spare = std::move(scratch);
+    }
     for (auto e : phase_ev) cudaEventDestroy(e);
     for (auto p : A) delete p;
     for (auto p : Lenv) delete p;
@@ -294,6 +300,10 @@ MPSState::~MPSState() {
 int MPSState::init(Hamiltonian* h, int D) {
     H = h;
     ctx = h->ctx;
+    {
+        std::lock_guard<std::mutex> lk(ctx->spare_mu);
+        if (ctx->spare) scratch = std::move(ctx->spare);
+    }
     L = h->L;
     d = h->d;
     D1.assign(L + 2, 1);
@@ -345,18 +355,33 @@ int MPSState::init(Hamiltonian* h, int D) {
 }
 
 int MPSState::ensure_capacity(int D) {
-    size_t site = sizeof(double) * (size_t)d * D * D;
+    const size_t site = sizeof(double) * (size_t)d * D * D;
+    return slab_reserve(std::vector<DevBuf*>(A.begin() + 1, A.begin() + L + 1), std::vector<size_t>(L, site), siteSlab);
+}
+
+// The environments that a sweep at the current bonds fills, in one allocation.
+int MPSState::reserve_environments() {
+    std::vector<DevBuf*> v;
+    std::vector<size_t> need;
     for (int ia = 1; ia <= L; ++ia) {
-        if (A[ia]->bytes < site) {
-            // grow preserving contents
-            DevBuf nb;
-            TN_CHECK(nb.ensure(site));
-            if (A[ia]->p) TN_CUDA_CHECK(cudaMemcpy(nb.p, A[ia]->p, A[ia]->bytes, cudaMemcpyDeviceToDevice));
-            std::swap(A[ia]->p, nb.p);
-            std::swap(A[ia]->bytes, nb.bytes);
-        }
+        const SiteMPO& op = H->ops[ia];
+        v.push_back(Lenv[ia]);
+        need.push_back(ia < L ? sizeof(double) * (size_t)op.Dw2 * D2[ia] * D2[ia] : 0);
+        v.push_back(Renv[ia]);
+        need.push_back(ia > 1 ? sizeof(double) * (size_t)op.Dw1 * D1[ia] * D1[ia] : 0);
     }
-    return TN_OK;
+    return slab_reserve(v, need, envSlab);
+}
+
+// The triangular factors that a half-sweep in direction dir leaves, in one allocation.
+int MPSState::reserve_factors(int dir) {
+    std::vector<DevBuf*> v;
+    std::vector<size_t> need;
+    for (int b = 1; b < L; ++b) {
+        v.push_back(bondR[dir][b]);
+        need.push_back(sizeof(double) * (size_t)D2[b] * D2[b]);
+    }
+    return v.empty() ? TN_OK : slab_reserve(v, need, factorSlab[dir]);
 }
 
 // MPSSite::InitializeWith(Random) (MPSSite.C:119-127) with mt19937_64(seed),
@@ -387,12 +412,12 @@ int MPSState::max_D() const {
 int MPSState::site_resize(int ia, int nD1, int nD2) {
     if (nD1 == D1[ia] && nD2 == D2[ia]) return TN_OK;
     size_t cnt = (size_t)d * nD1 * nD2;
-    TN_CHECK(tmp.ensure(sizeof(double) * cnt));
+    TN_CHECK(scratch->tmp.ensure(sizeof(double) * cnt));
     if (A[ia]->bytes < sizeof(double) * cnt) TN_CHECK(ensure_capacity(std::max(nD1, nD2)));
     resize_kernel<<<g1d((long long)cnt), 256, 0, ctx->stream>>>(A[ia]->as<double>(), d, D1[ia], D2[ia],
-                                                                tmp.as<double>(), nD1, nD2);
+                                                                scratch->tmp.as<double>(), nD1, nD2);
     TN_LAUNCH_CHECK();
-    TN_CUDA_CHECK(cudaMemcpyAsync(A[ia]->p, tmp.p, sizeof(double) * cnt, cudaMemcpyDeviceToDevice, ctx->stream));
+    TN_CUDA_CHECK(cudaMemcpyAsync(A[ia]->p, scratch->tmp.p, sizeof(double) * cnt, cudaMemcpyDeviceToDevice, ctx->stream));
     D1[ia] = nD1;
     D2[ia] = nD2;
     return TN_OK;
@@ -401,10 +426,10 @@ int MPSState::site_resize(int ia, int nD1, int nD2) {
 // MPSSite::Rescale(sqrt(GetNorm(lr)(1,1))) of HandleEdges: divide by the 2-norm.
 int MPSState::rescale_site(int ia) {
     long long n = (long long)d * D1[ia] * D2[ia];
-    TN_CHECK(tmp.ensure(sizeof(double) * 2));
-    sumsq_kernel<<<1, 512, 0, ctx->stream>>>(A[ia]->as<double>(), n, tmp.as<double>());
+    TN_CHECK(scratch->tmp.ensure(sizeof(double) * 2));
+    sumsq_kernel<<<1, 512, 0, ctx->stream>>>(A[ia]->as<double>(), n, scratch->tmp.as<double>());
     TN_LAUNCH_CHECK();
-    scale_by_norm_kernel<<<g1d(n), 256, 0, ctx->stream>>>(A[ia]->as<double>(), n, tmp.as<double>());
+    scale_by_norm_kernel<<<g1d(n), 256, 0, ctx->stream>>>(A[ia]->as<double>(), n, scratch->tmp.as<double>());
     TN_LAUNCH_CHECK();
     return TN_OK;
 }
@@ -440,27 +465,27 @@ int MPSState::normalize_site(int ia, bool left) {
     double* Aia = A[ia]->as<double>();
     if (left) {
         const int m = d * a1, n = a2, k = std::min(m, n);
-        TN_CHECK(Wqr.ensure(sizeof(double) * (size_t)m * n));
-        TN_CHECK(Qqr.ensure(sizeof(double) * (size_t)m * k));
+        TN_CHECK(scratch->Wqr.ensure(sizeof(double) * (size_t)m * n));
+        TN_CHECK(scratch->Qqr.ensure(sizeof(double) * (size_t)m * k));
         DevBuf* Rb = bondR[0][ia];
         TN_CHECK(Rb->ensure(sizeof(double) * (size_t)k * n));
         // W(r=(n_,i1), c=i2) = A(n_,i1,i2)
-        TN_CHECK(copy2d(m, n, Aia, idx2(1, a1, blk), idx(a1), Wqr.as<double>(), idx(1), idx(m), 1.0, st));
-        TN_CHECK(gauge_qr(m, n, Wqr.as<double>(), Qqr.as<double>(), Rb->as<double>(), k));
+        TN_CHECK(copy2d(m, n, Aia, idx2(1, a1, blk), idx(a1), scratch->Wqr.as<double>(), idx(1), idx(m), 1.0, st));
+        TN_CHECK(gauge_qr(m, n, scratch->Wqr.as<double>(), scratch->Qqr.as<double>(), Rb->as<double>(), k));
         // site := Q with D2 = k
         rq_order();
-        TN_CHECK(copy2d(m, k, Qqr.as<double>(), idx(1), idx(m), Aia, idx2(1, a1, (long long)a1 * k), idx(a1), 1.0, st));
+        TN_CHECK(copy2d(m, k, scratch->Qqr.as<double>(), idx(1), idx(m), Aia, idx2(1, a1, (long long)a1 * k), idx(a1), 1.0, st));
         D2[ia] = k;
         // right neighbour: M_n <- R M_n
         const int nb1 = D1[ia + 1], nb2 = D2[ia + 1];
-        TN_CHECK(tmp.ensure(sizeof(double) * (size_t)d * k * nb2));
+        TN_CHECK(scratch->tmp.ensure(sizeof(double) * (size_t)d * k * nb2));
         GemmArgs g;
         g.M = k; g.N = nb2; g.K = nb1; g.nb0 = d;
         g.A.ptr = Rb->as<double>(); g.A.mn = idx(1); g.A.k = idx(k);
         g.B.ptr = A[ia + 1]->as<double>(); g.B.k = idx(1); g.B.mn = idx(nb1); g.B.sb0 = (long long)nb1 * nb2;
-        g.C.ptr = tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(k); g.C.sb0 = (long long)k * nb2;
+        g.C.ptr = scratch->tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(k); g.C.sb0 = (long long)k * nb2;
         TN_CHECK(gemm_f64(g, st));
-        TN_CUDA_CHECK(cudaMemcpyAsync(A[ia + 1]->p, tmp.p, sizeof(double) * (size_t)d * k * nb2,
+        TN_CUDA_CHECK(cudaMemcpyAsync(A[ia + 1]->p, scratch->tmp.p, sizeof(double) * (size_t)d * k * nb2,
                                       cudaMemcpyDeviceToDevice, st));
         D1[ia + 1] = k;
         bondRm[0][ia] = k; bondRn[0][ia] = n; bondHave[0][ia] = 1; bondLatest[ia] = 0;
@@ -468,27 +493,27 @@ int MPSState::normalize_site(int ia, bool left) {
     } else {
         // LQ of the D1 x (d*D2) matrix as QR of its transpose (m = d*D2 rows, n = D1 cols)
         const int m = d * a2, n = a1, k = std::min(m, n);
-        TN_CHECK(Wqr.ensure(sizeof(double) * (size_t)m * n));
-        TN_CHECK(Qqr.ensure(sizeof(double) * (size_t)m * k));
+        TN_CHECK(scratch->Wqr.ensure(sizeof(double) * (size_t)m * n));
+        TN_CHECK(scratch->Qqr.ensure(sizeof(double) * (size_t)m * k));
         DevBuf* Rb = bondR[1][ia - 1];
         TN_CHECK(Rb->ensure(sizeof(double) * (size_t)k * n));
         // W(r=(n_,i2), c=i1) = A(n_,i1,i2)
-        TN_CHECK(copy2d(m, n, Aia, idx2(a1, a2, blk), idx(1), Wqr.as<double>(), idx(1), idx(m), 1.0, st));
-        TN_CHECK(gauge_qr(m, n, Wqr.as<double>(), Qqr.as<double>(), Rb->as<double>(), k));
+        TN_CHECK(copy2d(m, n, Aia, idx2(a1, a2, blk), idx(1), scratch->Wqr.as<double>(), idx(1), idx(m), 1.0, st));
+        TN_CHECK(gauge_qr(m, n, scratch->Wqr.as<double>(), scratch->Qqr.as<double>(), Rb->as<double>(), k));
         // site := Q^T with D1 = k: element (n_, i1', i2) = Q(n_*D2+i2, i1')
         rq_order();
-        TN_CHECK(copy2d(m, k, Qqr.as<double>(), idx(1), idx(m), Aia, idx2(k, a2, (long long)k * a2), idx(1), 1.0, st));
+        TN_CHECK(copy2d(m, k, scratch->Qqr.as<double>(), idx(1), idx(m), Aia, idx2(k, a2, (long long)k * a2), idx(1), 1.0, st));
         D1[ia] = k;
         // left neighbour: M_n <- M_n L, L = R^T (n x k)
         const int pb1 = D1[ia - 1], pb2 = D2[ia - 1];
-        TN_CHECK(tmp.ensure(sizeof(double) * (size_t)d * pb1 * k));
+        TN_CHECK(scratch->tmp.ensure(sizeof(double) * (size_t)d * pb1 * k));
         GemmArgs g;
         g.M = pb1; g.N = k; g.K = pb2; g.nb0 = d;
         g.A.ptr = A[ia - 1]->as<double>(); g.A.mn = idx(1); g.A.k = idx(pb1); g.A.sb0 = (long long)pb1 * pb2;
         g.B.ptr = Rb->as<double>(); g.B.k = idx(k); g.B.mn = idx(1);
-        g.C.ptr = tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(pb1); g.C.sb0 = (long long)pb1 * k;
+        g.C.ptr = scratch->tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(pb1); g.C.sb0 = (long long)pb1 * k;
         TN_CHECK(gemm_f64(g, st));
-        TN_CUDA_CHECK(cudaMemcpyAsync(A[ia - 1]->p, tmp.p, sizeof(double) * (size_t)d * pb1 * k,
+        TN_CUDA_CHECK(cudaMemcpyAsync(A[ia - 1]->p, scratch->tmp.p, sizeof(double) * (size_t)d * pb1 * k,
                                       cudaMemcpyDeviceToDevice, st));
         D2[ia - 1] = k;
         bondRm[1][ia - 1] = k; bondRn[1][ia - 1] = n; bondHave[1][ia - 1] = 1; bondLatest[ia - 1] = 1;
@@ -507,14 +532,14 @@ int MPSState::bond_values(const std::vector<std::pair<int, int>>& which, std::ve
         int r = bondRm[w.first][w.second], c = bondRn[w.first][w.second];
         total += (size_t)r * c + std::min(r, c);
     }
-    TN_CHECK(svdw.ensure(sizeof(double) * total));
+    TN_CHECK(scratch->svdw.ensure(sizeof(double) * total));
     std::vector<SvdJob> jobs;
     std::vector<size_t> soff;
     size_t off = 0;
     for (auto& w : which) {
         int r = bondRm[w.first][w.second], c = bondRn[w.first][w.second];
         int tm = std::max(r, c), tn = std::min(r, c);
-        double* Wb = svdw.as<double>() + off;
+        double* Wb = scratch->svdw.as<double>() + off;
         const double* R = bondR[w.first][w.second]->as<double>();
         if (r >= c)
             TN_CHECK(copy2d(r, c, R, idx(1), idx(r), Wb, idx(1), idx(r), 1.0, ctx->stream));
@@ -522,14 +547,14 @@ int MPSState::bond_values(const std::vector<std::pair<int, int>>& which, std::ve
             TN_CHECK(copy2d(r, c, R, idx(1), idx(r), Wb, idx(c), idx(1), 1.0, ctx->stream));
         off += (size_t)tm * tn;
         SvdJob j{};
-        j.W = Wb; j.m = tm; j.n = tn; j.s = svdw.as<double>() + off;
+        j.W = Wb; j.m = tm; j.n = tn; j.s = scratch->svdw.as<double>() + off;
         soff.push_back(off);
         off += tn;
         jobs.push_back(j);
     }
     TN_CHECK(svd_batched(*ctx, jobs, false));
     std::vector<double> hs(total);
-    TN_CUDA_CHECK(cudaMemcpy(hs.data(), svdw.p, sizeof(double) * total, cudaMemcpyDeviceToHost));
+    TN_CUDA_CHECK(cudaMemcpy(hs.data(), scratch->svdw.p, sizeof(double) * total, cudaMemcpyDeviceToHost));
     for (size_t q = 0; q < which.size(); ++q)
         out[q].assign(hs.begin() + soff[q], hs.begin() + soff[q] + jobs[q].n);
     return TN_OK;
@@ -628,6 +653,7 @@ int MPSState::compute_right_env(int ia) {
 }
 
 int MPSState::normalize_all(bool left) {
+    TN_CHECK(reserve_factors(left ? 0 : 1));
     if (left) for (int ia = 1; ia <= L; ++ia) TN_CHECK(normalize_site(ia, true));
     else for (int ia = L; ia >= 1; --ia) TN_CHECK(normalize_site(ia, false));
     return TN_OK;
@@ -635,6 +661,7 @@ int MPSState::normalize_all(bool left) {
 
 // MPSImp::LoadHeffCaches -> CalcHeffRight (MPSImp_Variational.C:120-149).
 int MPSState::load_heff_caches() {
+    TN_CHECK(reserve_environments());
     for (int ia = L; ia >= 2; --ia) TN_CHECK(compute_right_env(ia));
     return TN_OK;
 }
@@ -650,7 +677,7 @@ int MPSState::refine_site_mixed(int ia, double epsEigen) {
     size_t scr = sizeof(double) * contract_scratch_doubles(s);
     TN_CHECK(ctx->P.ensure(scr));
     TN_CHECK(ctx->Q.ensure(scr));
-    TN_CHECK(yvec.ensure(sizeof(double) * (size_t)N));
+    TN_CHECK(scratch->yvec.ensure(sizeof(double) * (size_t)N));
     const WTermDev* t = H->terms.as<WTermDev>() + op.offLR;
     const double* F = Lenv[ia - 1]->as<double>();
     const double* G = Renv[ia + 1]->as<double>();
@@ -668,10 +695,10 @@ int MPSState::refine_site_mixed(int ia, double epsEigen) {
         TN_CHECK(ctx->prof_events());
         TN_CUDA_CHECK(cudaEventRecord(ctx->pev[0], st));
     }
-    TN_CHECK(mixed_prepare_site(*ctx, msite, s, op.W.data(), F, G, wF, wG, ns));
+    TN_CHECK(mixed_prepare_site(*ctx, scratch->msite, s, op.W.data(), F, G, wF, wG, ns));
     if (ctx->prof) TN_CUDA_CHECK(cudaEventRecord(ctx->pev[1], st));
     MatvecFn mvm = [&](const double* x, double* y, const int* skip) {
-        return heff_matvec_mixed(*ctx, msite, x, y, skip);
+        return heff_matvec_mixed(*ctx, scratch->msite, x, y, skip);
     };
     int krylov = opt.krylov > 0 ? opt.krylov : 20;
     int restarts = opt.max_restarts > 0 ? opt.max_restarts : 10;
@@ -679,24 +706,25 @@ int MPSState::refine_site_mixed(int ia, double epsEigen) {
     unsigned long long key = hash_val(HASH_SEED, 0x6d69786564ULL);
     key = hash_val(key, s);
     key = hash_val(key, ns);
-    key = hash_val(key, (const void*)t);
-    key = hash_val(key, op.nLR);
-    for (const DevBuf* b : {&msite.Fs, &msite.Gc, &msite.Xs, &msite.Ps, &msite.segs, &msite.shifts, &msite.err})
+    key = tc_chain_hash(scratch->msite.plan1, key);
+    key = tc_chain_hash(scratch->msite.plan2, key);
+    MixedSite& ms = scratch->msite;
+    for (const DevBuf* b : {&ms.Fs, &ms.Gc, &ms.Xs, &ms.Ps, &ms.segs, &ms.shifts, &ms.err})
         key = hash_val(key, b->p);
     // the Lanczos kernels that produce each Krylov vector also write its BF16
     // pieces, so the matvec starts with its first GEMM
-    const VecSplit vsp{msite.Xs.as<uint16_t>(), ns, (long long)msite.nX};
+    const VecSplit vsp{scratch->msite.Xs.as<uint16_t>(), ns, (long long)scratch->msite.nX};
     struct PresplitScope {
         MixedSite& m;
         explicit PresplitScope(MixedSite& mm) : m(mm) { m.presplit = true; }
         ~PresplitScope() { m.presplit = false; }
-    } presplit_scope(msite);
+    } presplit_scope(scratch->msite);
     const bool deferred = opt.refine_tol <= 0 && opt.verbose < 3 && ctx->aux2;
     if (deferred) {
         // nothing here waits for the host: restarts decided on the device, the
         // FP64 check beside the gauge move, both read back once per half-sweep
         TN_CHECK(rq_slots());
-        LzSummary* slot = reinterpret_cast<LzSummary*>(reinterpret_cast<double*>(rqhost.p) + RQ_SLOT * (size_t)ia + 4);
+        LzSummary* slot = reinterpret_cast<LzSummary*>(reinterpret_cast<double*>(scratch->rqhost.p) + RQ_SLOT * (size_t)ia + 4);
         const int rc = lanczos_solve_async(*ctx, N, A[ia]->as<double>(), krylov, restarts, epsEigen, mvm, tol_rel,
                                            key, slot, &vsp);
         if (rc == TN_OK) {
@@ -727,11 +755,11 @@ int MPSState::refine_site_mixed(int ia, double epsEigen) {
         if (!rm.converged) ++not_converged;
         return TN_OK;
     }
-    TN_CHECK(mixed_check_error(msite, st));
+    TN_CHECK(mixed_check_error(scratch->msite, st));
     // FP64 Rayleigh quotient and residual of the Ritz vector
-    TN_CHECK(heff_matvec_f64(s, t, op.nLR, F, G, A[ia]->as<double>(), yvec.as<double>(), P, Q, nullptr, st));
+    TN_CHECK(heff_matvec_f64(s, t, op.nLR, F, G, A[ia]->as<double>(), scratch->yvec.as<double>(), P, Q, nullptr, st));
     double theta = 0, resid = 0;
-    TN_CHECK(rayleigh_residual(*ctx, N, A[ia]->as<double>(), yvec.as<double>(), &theta, &resid));
+    TN_CHECK(rayleigh_residual(*ctx, N, A[ia]->as<double>(), scratch->yvec.as<double>(), &theta, &resid));
     matvecs += 1;
     matvecs_fp64 += 1;
     heff_flop += heff_flops(s);
@@ -764,7 +792,7 @@ int MPSState::refine_site_mixed(int ia, double epsEigen) {
 // second side stream once the Lanczos solve has finished; the result (and the
 // split operator's error flag) is read by rq_collect().
 int MPSState::rq_slots() {
-    TN_CHECK(rqhost.ensure(sizeof(double) * RQ_SLOT * (size_t)(L + 2)));
+    TN_CHECK(scratch->rqhost.ensure(sizeof(double) * RQ_SLOT * (size_t)(L + 2)));
     if ((int)rq_pending.size() != L + 2) {
         rq_pending.assign(L + 2, 0);
         rq_lz.assign(L + 2, 0);
@@ -780,17 +808,17 @@ int MPSState::rq_launch(int ia, const ContractShape& s, const WTermDev* t, int n
     cudaStream_t st = ctx->stream, sx = ctx->aux2;
     TN_CHECK(rq_slots());
     const size_t scr = sizeof(double) * contract_scratch_doubles(s);
-    TN_CHECK(rqP.ensure(scr));
-    TN_CHECK(rqQ.ensure(scr));
-    TN_CHECK(yvec.ensure(sizeof(double) * (size_t)N));
-    TN_CHECK(rqbuf.ensure(rayleigh_scratch_bytes(N, ctx->sm_count)));
-    double* slot = reinterpret_cast<double*>(rqhost.p) + RQ_SLOT * (size_t)ia;
-    TN_CUDA_CHECK(cudaMemcpyAsync(slot + 3, msite.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TN_CHECK(scratch->rqP.ensure(scr));
+    TN_CHECK(scratch->rqQ.ensure(scr));
+    TN_CHECK(scratch->yvec.ensure(sizeof(double) * (size_t)N));
+    TN_CHECK(scratch->rqbuf.ensure(rayleigh_scratch_bytes(N, ctx->sm_count)));
+    double* slot = reinterpret_cast<double*>(scratch->rqhost.p) + RQ_SLOT * (size_t)ia;
+    TN_CUDA_CHECK(cudaMemcpyAsync(slot + 3, scratch->msite.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     TN_CUDA_CHECK(cudaEventRecord(ctx->ev_y[0], st));
     TN_CUDA_CHECK(cudaStreamWaitEvent(sx, ctx->ev_y[0], 0));
     const double* x = A[ia]->as<double>();
-    TN_CHECK(heff_matvec_f64(s, t, nLR, F, G, x, yvec.as<double>(), rqP.as<double>(), rqQ.as<double>(), nullptr, sx));
-    TN_CHECK(rayleigh_residual_async(sx, ctx->sm_count, N, x, yvec.as<double>(), rqbuf.p, slot));
+    TN_CHECK(heff_matvec_f64(s, t, nLR, F, G, x, scratch->yvec.as<double>(), scratch->rqP.as<double>(), scratch->rqQ.as<double>(), nullptr, sx));
+    TN_CHECK(rayleigh_residual_async(sx, ctx->sm_count, N, x, scratch->yvec.as<double>(), scratch->rqbuf.p, slot));
     TN_CUDA_CHECK(cudaEventRecord(ctx->ev_y[1], sx));
     rq_pending[ia] = 1;
     rq_dtheta[ia] = dtheta;
@@ -811,7 +839,7 @@ int MPSState::rq_collect() {
     for (int ia = 1; ia <= L; ++ia) {
         if (!rq_pending[ia]) continue;
         rq_pending[ia] = 0;
-        const double* slot = reinterpret_cast<double*>(rqhost.p) + RQ_SLOT * (size_t)ia;
+        const double* slot = reinterpret_cast<double*>(scratch->rqhost.p) + RQ_SLOT * (size_t)ia;
         const bool exact = rq_exact[ia] != 0;  // an FP64 solve: its Ritz value is the energy, no check ran
         rq_exact[ia] = 0;
         int err = 0;
@@ -861,15 +889,15 @@ int MPSState::refine_site_davidson(int ia, double epsEigen) {
     size_t scr = sizeof(double) * contract_scratch_doubles(s);
     TN_CHECK(ctx->P.ensure(scr));
     TN_CHECK(ctx->Q.ensure(scr));
-    TN_CHECK(yvec.ensure(sizeof(double) * (size_t)N));
-    TN_CHECK(diagbuf.ensure(sizeof(double) * (size_t)N));
+    TN_CHECK(scratch->yvec.ensure(sizeof(double) * (size_t)N));
+    TN_CHECK(scratch->diagbuf.ensure(sizeof(double) * (size_t)N));
     const WTermDev* t = H->terms.as<WTermDev>() + op.offLR;
     const double* F = Lenv[ia - 1]->as<double>();
     const double* G = Renv[ia + 1]->as<double>();
     double* P = ctx->P.as<double>();
     double* Q = ctx->Q.as<double>();
     cudaStream_t st = ctx->stream;
-    TN_CHECK(heff_diag(s, H->Wdev.as<double>() + op.offW, F, G, diagbuf.as<double>(), st));
+    TN_CHECK(heff_diag(s, H->Wdev.as<double>() + op.offW, F, G, scratch->diagbuf.as<double>(), st));
     const bool mixed = opt.precision != TN_PREC_FP64 && mixed_supported(s);
     const int ns = opt.precision == TN_PREC_MIXED_HI ? 3 : 2;
     MatvecFn mv;
@@ -881,14 +909,15 @@ int MPSState::refine_site_davidson(int ia, double epsEigen) {
     if (mixed) {
         const int wF = H->form == TN_FORM_REGULAR_LOWER ? 0 : op.Dw1 - 1;
         const int wG = H->form == TN_FORM_REGULAR_LOWER ? op.Dw2 - 1 : 0;
-        TN_CHECK(mixed_prepare_site(*ctx, msite, s, op.W.data(), F, G, wF, wG, ns));
+        TN_CHECK(mixed_prepare_site(*ctx, scratch->msite, s, op.W.data(), F, G, wF, wG, ns));
         // the split operator is Heff - sigma I: shift the diagonal the same way
-        const double sigma = mixed_shift_host(msite, st);
-        TN_CHECK(shift_vector(diagbuf.as<double>(), N, -sigma, st));
-        mv = [&](const double* x, double* y, const int* skip) { return heff_matvec_mixed(*ctx, msite, x, y, skip); };
+        const double sigma = mixed_shift_host(scratch->msite, st);
+        TN_CHECK(shift_vector(scratch->diagbuf.as<double>(), N, -sigma, st));
+        mv = [&](const double* x, double* y, const int* skip) { return heff_matvec_mixed(*ctx, scratch->msite, x, y, skip); };
         tol_rel = opt.mixed_tol > 0 ? opt.mixed_tol : (ns == 3 ? 1e-9 : 2e-6);
         key = hash_val(key, ns);
-        for (const DevBuf* b : {&msite.Fs, &msite.Gc, &msite.Xs, &msite.Ps, &msite.segs, &msite.shifts, &msite.err})
+        MixedSite& ms = scratch->msite;
+        for (const DevBuf* b : {&ms.Fs, &ms.Gc, &ms.Xs, &ms.Ps, &ms.segs, &ms.shifts, &ms.err})
             key = hash_val(key, b->p);
     } else {
         mv = [&](const double* x, double* y, const int* skip) {
@@ -902,9 +931,9 @@ int MPSState::refine_site_davidson(int ia, double epsEigen) {
     const int kmax = opt.krylov > 0 ? std::min(opt.krylov, DV_MAXK) : 16;
     const int maxit = std::max(8, (opt.max_restarts > 0 ? opt.max_restarts : 10) * kmax);
     DvResult r{};
-    TN_CHECK(davidson_solve(*ctx, N, A[ia]->as<double>(), kmax, maxit, epsEigen, mv, diagbuf.as<double>(), model, pos,
+    TN_CHECK(davidson_solve(*ctx, N, A[ia]->as<double>(), kmax, maxit, epsEigen, mv, scratch->diagbuf.as<double>(), model, pos,
                             &r, rec, key, tol_rel));
-    if (mixed) TN_CHECK(mixed_check_error(msite, st));
+    if (mixed) TN_CHECK(mixed_check_error(scratch->msite, st));
     matvecs += r.matvecs;
     if (!mixed) matvecs_fp64 += r.matvecs;
     heff_flop += heff_flops(s) * r.matvecs;
@@ -913,9 +942,9 @@ int MPSState::refine_site_davidson(int ia, double epsEigen) {
     double theta = r.theta;
     if (mixed) {
         // FP64 Rayleigh quotient of the Ritz vector
-        TN_CHECK(heff_matvec_f64(s, t, op.nLR, F, G, A[ia]->as<double>(), yvec.as<double>(), P, Q, nullptr, st));
+        TN_CHECK(heff_matvec_f64(s, t, op.nLR, F, G, A[ia]->as<double>(), scratch->yvec.as<double>(), P, Q, nullptr, st));
         double resid = 0;
-        TN_CHECK(rayleigh_residual(*ctx, N, A[ia]->as<double>(), yvec.as<double>(), &theta, &resid));
+        TN_CHECK(rayleigh_residual(*ctx, N, A[ia]->as<double>(), scratch->yvec.as<double>(), &theta, &resid));
         matvecs += 1;
         matvecs_fp64 += 1;
         heff_flop += heff_flops(s);
@@ -963,7 +992,7 @@ int MPSState::refine_site(int ia, double epsEigen) {
         // device-driven restarts, nothing waits for the host: the solve's summary
         // (its FP64 Ritz value is the site energy) is read once per half-sweep
         TN_CHECK(rq_slots());
-        LzSummary* slot = reinterpret_cast<LzSummary*>(reinterpret_cast<double*>(rqhost.p) + RQ_SLOT * (size_t)ia + 4);
+        LzSummary* slot = reinterpret_cast<LzSummary*>(reinterpret_cast<double*>(scratch->rqhost.p) + RQ_SLOT * (size_t)ia + 4);
         int rc = lanczos_site(*ctx, s, t, op.nLR, F, G, A[ia]->as<double>(), krylov, restarts, epsEigen, tol_rel, slot);
         if (rc == LZ_SITE_UNAVAILABLE)
             rc = lanczos_solve_async(*ctx, N, A[ia]->as<double>(), krylov, restarts, epsEigen, mv, tol_rel, key, slot);
@@ -998,6 +1027,7 @@ int MPSState::sweep(bool left, double epsEigen) {
     auto secs = [](std::chrono::steady_clock::time_point a, std::chrono::steady_clock::time_point b) {
         return std::chrono::duration<double>(b - a).count();
     };
+    TN_CHECK(reserve_factors(left ? 0 : 1));
     const bool dev_phases = opt.phase_timing != 0;
     if (dev_phases) TN_CHECK(phase_events_ensure((size_t)4 * L));
     auto mark = [&](int step, int k) -> int {
@@ -1102,10 +1132,10 @@ int MPSState::increase_bond_dims(int D) {
 int MPSState::expectation(const std::vector<SiteMPO>& ops, double* E) {
     cudaStream_t st = ctx->stream;
     double one = 1.0;
-    TN_CHECK(envA.ensure(sizeof(double)));
-    TN_CUDA_CHECK(cudaMemcpyAsync(envA.p, &one, sizeof(double), cudaMemcpyHostToDevice, st));
-    DevBuf* cur = &envA;
-    DevBuf* nxt = &envB;
+    TN_CHECK(scratch->envA.ensure(sizeof(double)));
+    TN_CUDA_CHECK(cudaMemcpyAsync(scratch->envA.p, &one, sizeof(double), cudaMemcpyHostToDevice, st));
+    DevBuf* cur = &scratch->envA;
+    DevBuf* nxt = &scratch->envB;
     for (int ia = 1; ia <= L; ++ia) {
         const SiteMPO& op = ops[ia];
         ContractShape s{d, op.Dw1, op.Dw2, D1[ia], D2[ia]};

@@ -36,6 +36,19 @@ struct SiteSet {
     std::vector<int> D1, D2;
 };
 
+// Work buffers of an MPS's sweeps, which the context hands from one MPS to the next.
+struct MpsScratch {
+    DevBuf tmp, Wqr, Qqr, svdw, envA, envB, yvec, diagbuf;
+    // FP64 check of the split-precision eigenvector on the context's second side
+    // stream (refine_tol = 0): contraction scratch, reduction state, and per site
+    // (theta, -, resid, error flag) in pinned memory, applied by rq_collect().
+    // With the device-driven Lanczos solve (lanczos_solve_async) its summary
+    // goes to the same slot (doubles 4 ..) and is applied there too.
+    DevBuf rqP, rqQ, rqbuf;
+    HostBuf rqhost;
+    MixedSite msite;
+};
+
 struct MPSState {
     Ctx* ctx = nullptr;
     Hamiltonian* H = nullptr;
@@ -59,19 +72,12 @@ struct MPSState {
     std::vector<int> bondK;                   // current bond dimension (Bond::GetD)
     std::vector<char> bondDirty;              // bond_s lags behind the latest factor
     std::vector<double> Emin, iterDE, gapE;
-    DevBuf tmp, Wqr, Qqr, svdw, envA, envB, yvec, diagbuf;
-    // FP64 check of the split-precision eigenvector on the context's second side
-    // stream (refine_tol = 0): contraction scratch, reduction state, and per site
-    // (theta, -, resid, error flag) in pinned memory, applied by rq_collect().
-    // With the device-driven Lanczos solve (lanczos_solve_async) its summary
-    // goes to the same slot (doubles 4 ..) and is applied there too.
+    std::unique_ptr<MpsScratch, MpsScratchDelete> scratch{new MpsScratch};
+    DevBuf siteSlab, envSlab, factorSlab[2];  // what the tensors, environments and factors are parts of
     static constexpr int RQ_SLOT = 12;  // doubles per site
-    DevBuf rqP, rqQ, rqbuf;
-    HostBuf rqhost;
     std::vector<char> rq_pending, rq_lz, rq_exact;  // rq_exact: an FP64 solve, no separate check
     std::vector<double> rq_dtheta, rq_flop;
     bool rq_inflight = false;
-    MixedSite msite;
     long long matvecs = 0, matvecs_fp64 = 0;
     double heff_flop = 0;
     int not_converged = 0, fallbacks = 0;
@@ -93,6 +99,8 @@ struct MPSState {
     int initialize_random(unsigned long long seed);
     int max_D() const;
     int ensure_capacity(int D);
+    int reserve_environments();
+    int reserve_factors(int dir);
     int normalize_site(int ia, bool left);
     int normalize_all(bool left);
     int bond_values(const std::vector<std::pair<int, int>>& which, std::vector<std::vector<double>>& out);

@@ -187,6 +187,7 @@ int MPSState::site_reserve(int ia, size_t n) {
     TN_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
     std::swap(A[ia]->p, nb.p);
     std::swap(A[ia]->bytes, nb.bytes);
+    std::swap(A[ia]->part, nb.part);
     return TN_OK;
 }
 
@@ -247,12 +248,12 @@ int MPSState::apply_mpo_inplace(const std::vector<SiteMPO>& W) {
         const size_t n = (size_t)d * E1 * E2;
         TN_CHECK(wd.ensure(sizeof(double) * op.W.size()));
         TN_CUDA_CHECK(cudaMemcpyAsync(wd.p, op.W.data(), sizeof(double) * op.W.size(), cudaMemcpyHostToDevice, st));
-        TN_CHECK(tmp.ensure(sizeof(double) * n));
+        TN_CHECK(scratch->tmp.ensure(sizeof(double) * n));
         apply_mpo_kernel<<<g1d((long long)n), 256, 0, st>>>(A[ia]->as<double>(), d, D1[ia], D2[ia], wd.as<double>(),
-                                                            op.Dw1, op.Dw2, tmp.as<double>());
+                                                            op.Dw1, op.Dw2, scratch->tmp.as<double>());
         TN_LAUNCH_CHECK();
         TN_CHECK(site_reserve(ia, n));
-        TN_CUDA_CHECK(cudaMemcpyAsync(A[ia]->p, tmp.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+        TN_CUDA_CHECK(cudaMemcpyAsync(A[ia]->p, scratch->tmp.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
         TN_CUDA_CHECK(cudaStreamSynchronize(st));  // wd and tmp are reused by the next site
         D1[ia] = E1;
         D2[ia] = E2;
@@ -279,13 +280,13 @@ int MPSState::svd_compress_sweep(bool left, int Dmax, double eps, std::vector<st
         const int m = left ? d * a1 : a1, n = left ? a2 : d * a2;
         const bool tall = m >= n;
         const int tm = tall ? m : n, tn = tall ? n : m;  // the SVD runs on the tall orientation
-        TN_CHECK(Wqr.ensure(sizeof(double) * (size_t)tm * tn));
-        TN_CHECK(svdw.ensure(sizeof(double) * ((size_t)tm * tn + 2 * (size_t)tn * tn + tn)));
-        double* Ut = svdw.as<double>();      // tm x tn
+        TN_CHECK(scratch->Wqr.ensure(sizeof(double) * (size_t)tm * tn));
+        TN_CHECK(scratch->svdw.ensure(sizeof(double) * ((size_t)tm * tn + 2 * (size_t)tn * tn + tn)));
+        double* Ut = scratch->svdw.as<double>();      // tm x tn
         double* Vw = Ut + (size_t)tm * tn;   // tn x tn (work)
         double* Vt = Vw + (size_t)tn * tn;   // tn x tn
         double* sv = Vt + (size_t)tn * tn;   // tn
-        double* Mw = Wqr.as<double>();
+        double* Mw = scratch->Wqr.as<double>();
         const double* Aia = A[ia]->as<double>();
         if (left) {
             if (tall) TN_CHECK(copy2d(m, n, Aia, idx2(1, a1, blk), idx(a1), Mw, idx(1), idx(tm), 1.0, st));
@@ -326,8 +327,8 @@ int MPSState::svd_compress_sweep(bool left, int Dmax, double eps, std::vector<st
             D2[ia] = k;
             // next site: A'[n](c, j2) = sum_i2 s_c R(c, i2) A[n](i2, j2)
             const int b1 = D1[ia + 1], b2 = D2[ia + 1];
-            TN_CHECK(tmp.ensure(sizeof(double) * ((size_t)k * n + (size_t)d * k * b2)));
-            double* SR = tmp.as<double>();
+            TN_CHECK(scratch->tmp.ensure(sizeof(double) * ((size_t)k * n + (size_t)d * k * b2)));
+            double* SR = scratch->tmp.as<double>();
             double* nxt = SR + (size_t)k * n;
             TN_CHECK(copy2d(k, n, Rf, rf_row, rf_col, SR, idx(1), idx(k), 1.0, st));
             TN_CHECK(scale_rows(SR, k, n, sk.as<double>(), st));
@@ -348,8 +349,8 @@ int MPSState::svd_compress_sweep(bool left, int Dmax, double eps, std::vector<st
             D1[ia] = k;
             // previous site: A'[n](i1, c) = sum_j A[n](i1, j) L(j, c) s_c
             const int p1 = D1[ia - 1], p2 = D2[ia - 1];
-            TN_CHECK(tmp.ensure(sizeof(double) * ((size_t)m * k + (size_t)d * p1 * k)));
-            double* LS = tmp.as<double>();
+            TN_CHECK(scratch->tmp.ensure(sizeof(double) * ((size_t)m * k + (size_t)d * p1 * k)));
+            double* LS = scratch->tmp.as<double>();
             double* prv = LS + (size_t)m * k;
             TN_CHECK(copy2d(m, k, Lf, lr_row, lr_col, LS, idx(1), idx(m), 1.0, st));
             TN_CHECK(scale_cols(LS, m, k, sk.as<double>(), st));
@@ -375,20 +376,20 @@ int MPSState::svd_compress_sweep(bool left, int Dmax, double eps, std::vector<st
 int MPSState::overlap_left(int ia, const SiteSet& P2, std::vector<DevBuf*>& Lo) {
     cudaStream_t st = ctx->stream;
     const int a1 = D1[ia], a2 = D2[ia], b1 = P2.D1[ia], b2 = P2.D2[ia];
-    TN_CHECK(tmp.ensure(sizeof(double) * (size_t)d * a1 * b2));
+    TN_CHECK(scratch->tmp.ensure(sizeof(double) * (size_t)d * a1 * b2));
     // T[n](i1, j2) = Lo[ia-1](i1, j1) B_n(j1, j2)
     GemmArgs g;
     g.M = a1; g.N = b2; g.K = b1; g.nb0 = d;
     g.A.ptr = Lo[ia - 1]->as<double>(); g.A.mn = idx(1); g.A.k = idx(a1);
     g.B.ptr = P2.A[ia]->as<double>(); g.B.k = idx(1); g.B.mn = idx(b1); g.B.sb0 = (long long)b1 * b2;
-    g.C.ptr = tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(a1); g.C.sb0 = (long long)a1 * b2;
+    g.C.ptr = scratch->tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(a1); g.C.sb0 = (long long)a1 * b2;
     TN_CHECK(gemm_f64(g, st));
     TN_CHECK(Lo[ia]->ensure(sizeof(double) * (size_t)a2 * b2));
     // Lo[ia](i2, j2) = sum_{(i1, n)} A_n(i1, i2) T[n](i1, j2)
     GemmArgs h;
     h.M = a2; h.N = b2; h.K = d * a1;
     h.A.ptr = A[ia]->as<double>(); h.A.mn = idx(a1); h.A.k = idx2(1, a1, (long long)a1 * a2);
-    h.B.ptr = tmp.as<double>(); h.B.k = idx2(1, a1, (long long)a1 * b2); h.B.mn = idx(a1);
+    h.B.ptr = scratch->tmp.as<double>(); h.B.k = idx2(1, a1, (long long)a1 * b2); h.B.mn = idx(a1);
     h.C.ptr = Lo[ia]->as<double>(); h.C.m = idx(1); h.C.n = idx(a2);
     return gemm_f64(h, st);
 }
@@ -397,19 +398,19 @@ int MPSState::overlap_left(int ia, const SiteSet& P2, std::vector<DevBuf*>& Lo) 
 int MPSState::overlap_right(int ia, const SiteSet& P2, std::vector<DevBuf*>& Ro) {
     cudaStream_t st = ctx->stream;
     const int a1 = D1[ia], a2 = D2[ia], b1 = P2.D1[ia], b2 = P2.D2[ia];
-    TN_CHECK(tmp.ensure(sizeof(double) * (size_t)d * a1 * b2));
+    TN_CHECK(scratch->tmp.ensure(sizeof(double) * (size_t)d * a1 * b2));
     // T[n](i1, j2) = A_n(i1, i2) Ro[ia+1](i2, j2)
     GemmArgs g;
     g.M = a1; g.N = b2; g.K = a2; g.nb0 = d;
     g.A.ptr = A[ia]->as<double>(); g.A.mn = idx(1); g.A.k = idx(a1); g.A.sb0 = (long long)a1 * a2;
     g.B.ptr = Ro[ia + 1]->as<double>(); g.B.k = idx(1); g.B.mn = idx(a2);
-    g.C.ptr = tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(a1); g.C.sb0 = (long long)a1 * b2;
+    g.C.ptr = scratch->tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(a1); g.C.sb0 = (long long)a1 * b2;
     TN_CHECK(gemm_f64(g, st));
     TN_CHECK(Ro[ia]->ensure(sizeof(double) * (size_t)a1 * b1));
     // Ro[ia](i1, j1) = sum_{(j2, n)} T[n](i1, j2) B_n(j1, j2)
     GemmArgs h;
     h.M = a1; h.N = b1; h.K = d * b2;
-    h.A.ptr = tmp.as<double>(); h.A.mn = idx(1); h.A.k = idx2(a1, b2, (long long)a1 * b2);
+    h.A.ptr = scratch->tmp.as<double>(); h.A.mn = idx(1); h.A.k = idx2(a1, b2, (long long)a1 * b2);
     h.B.ptr = P2.A[ia]->as<double>(); h.B.k = idx2(b1, b2, (long long)b1 * b2); h.B.mn = idx(1);
     h.C.ptr = Ro[ia]->as<double>(); h.C.m = idx(1); h.C.n = idx(a1);
     return gemm_f64(h, st);
@@ -420,16 +421,16 @@ int MPSState::overlap_right(int ia, const SiteSet& P2, std::vector<DevBuf*>& Ro)
 int MPSState::overlap_site(int ia, const SiteSet& P2, std::vector<DevBuf*>& Lo, std::vector<DevBuf*>& Ro) {
     cudaStream_t st = ctx->stream;
     const int a1 = D1[ia], a2 = D2[ia], b1 = P2.D1[ia], b2 = P2.D2[ia];
-    TN_CHECK(tmp.ensure(sizeof(double) * (size_t)d * a1 * b2));
+    TN_CHECK(scratch->tmp.ensure(sizeof(double) * (size_t)d * a1 * b2));
     GemmArgs g;  // T[n] = Lo B_n   (a1 x b2)
     g.M = a1; g.N = b2; g.K = b1; g.nb0 = d;
     g.A.ptr = Lo[ia - 1]->as<double>(); g.A.mn = idx(1); g.A.k = idx(a1);
     g.B.ptr = P2.A[ia]->as<double>(); g.B.k = idx(1); g.B.mn = idx(b1); g.B.sb0 = (long long)b1 * b2;
-    g.C.ptr = tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(a1); g.C.sb0 = (long long)a1 * b2;
+    g.C.ptr = scratch->tmp.as<double>(); g.C.m = idx(1); g.C.n = idx(a1); g.C.sb0 = (long long)a1 * b2;
     TN_CHECK(gemm_f64(g, st));
     GemmArgs h;  // A_n = T[n] Ro^T   (a1 x a2): Ro is a2 x b2
     h.M = a1; h.N = a2; h.K = b2; h.nb0 = d;
-    h.A.ptr = tmp.as<double>(); h.A.mn = idx(1); h.A.k = idx(a1); h.A.sb0 = (long long)a1 * b2;
+    h.A.ptr = scratch->tmp.as<double>(); h.A.mn = idx(1); h.A.k = idx(a1); h.A.sb0 = (long long)a1 * b2;
     h.B.ptr = Ro[ia + 1]->as<double>(); h.B.k = idx(a2); h.B.mn = idx(1);
     h.C.ptr = A[ia]->as<double>(); h.C.m = idx(1); h.C.n = idx(a1); h.C.sb0 = (long long)a1 * a2;
     return gemm_f64(h, st);

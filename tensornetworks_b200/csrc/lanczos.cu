@@ -550,7 +550,6 @@ int lanczos_solve(Ctx& c, long long N, double* x, int m, int maxRestarts, double
         key = hash_val(key, (const void*)V);
         key = hash_val(key, (const void*)s);
         key = hash_val(key, st);
-        key = hash_val(key, alloc_generation());
         auto it = c.lzgraphs.find(key);
         if (it == c.lzgraphs.end()) {
             if (c.lzgraphs.size() >= 256) c.clear_graphs();
@@ -712,13 +711,14 @@ int lanczos_solve_async(Ctx& c, long long N, double* x, int m, int maxRestarts, 
     LzSummary* sum = c.lzsum.as<LzSummary>();
     unsigned long long key = hash_val(graph_key, 0x6e65737465644c5aULL);
     for (unsigned long long v : {(unsigned long long)N, (unsigned long long)mm, (unsigned long long)maxR,
-                                 (unsigned long long)grid, alloc_generation()})
+                                 (unsigned long long)grid})
         key = hash_val(key, v);
     key = hash_val(key, tol);
     key = hash_val(key, tol_rel);
     key = hash_val(key, (const void*)V);
     key = hash_val(key, (const void*)s);
     key = hash_val(key, (const void*)sp.out);
+    key = hash_val(key, (const void*)sum);
     key = hash_val(key, st);
     auto it = c.lzgraphs.find(key);
     if (it == c.lzgraphs.end()) {

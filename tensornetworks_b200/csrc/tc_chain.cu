@@ -366,4 +366,20 @@ int tc_chain_run(const TcChainPlan& pl, cudaStream_t st) {
     return p.nsplit == 3 ? launch_chain<3, TCC_OUT_F64_COLMAJOR>(pl, st) : launch_chain<2, TCC_OUT_F64_COLMAJOR>(pl, st);
 }
 
+unsigned long long tc_chain_hash(const TcChainPlan& pl, unsigned long long h) {
+    const TcChainArgs& p = pl.args;
+    for (int q = 0; q < p.nsplit; ++q) {
+        h = hash_val(h, pl.maps.a[q]);
+        h = hash_val(h, pl.maps.b[q]);
+    }
+    for (long long v : {(long long)p.M, (long long)p.N, (long long)p.K, (long long)p.nbatch, (long long)p.splitk,
+                        (long long)p.nsplit, p.lda, p.a_batch, p.ldb, p.b_batch, (long long)p.a_nbatch,
+                        (long long)p.b_nbatch, (long long)p.out_mode, p.c16_piece, p.ldc16, p.c16_batch, p.ldc64,
+                        p.c64_batch})
+        h = hash_val(h, v);
+    for (const void* v : {(const void*)p.seg_start, (const void*)p.segs, (const void*)p.c16, (const void*)p.err})
+        h = hash_val(h, v);
+    return h;
+}
+
 }  // namespace tnb

@@ -50,5 +50,7 @@ struct TcChainPlan {
 int tc_chain_splitk(int tiles, int chunks, int sm_count);
 int tc_chain_plan(const TcChainArgs& a, TcChainPlan* plan);
 int tc_chain_run(const TcChainPlan& plan, cudaStream_t st);
+// Every launch parameter of the plan but the output and skip pointers, hashed into h.
+unsigned long long tc_chain_hash(const TcChainPlan& plan, unsigned long long h);
 
 }  // namespace tnb

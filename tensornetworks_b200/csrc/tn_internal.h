@@ -5,6 +5,8 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -70,8 +72,9 @@ unsigned long long launch_count();
         TN_CUDA_CHECK(cudaGetLastError()); \
     } while (0)
 
-// Incremented by every device (re)allocation of a DevBuf: captured CUDA graphs
-// hold raw pointers, so a graph recorded under another generation is stale.
+// Incremented by every device (re)allocation of a DevBuf: a captured CUDA graph
+// holds raw pointers, so one whose key does not name them all is stale under
+// another generation.
 unsigned long long alloc_generation();
 
 // FNV-1a over raw bytes (graph-cache keys).
@@ -89,6 +92,7 @@ constexpr unsigned long long HASH_SEED = 1469598103934665603ULL;
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool part = false;  // a part of another buffer (slab_reserve), not freed by itself
     int ensure(size_t nbytes);
     void release();
     template <class T> T* as() const { return reinterpret_cast<T*>(p); }
@@ -97,6 +101,10 @@ struct DevBuf {
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
 };
+
+// Every buffer of v gets its need[] bytes (where it has less) as a part of one
+// allocation, which replaces the slab they were parts of before; contents are kept.
+int slab_reserve(const std::vector<DevBuf*>& v, const std::vector<size_t>& need, DevBuf& slab);
 
 // Pinned host buffer for small device->host reads.
 struct HostBuf {
@@ -160,6 +168,11 @@ struct LzGraph {
     unsigned long long kernels_per_iter = 0;
 };
 
+struct MpsScratch;
+struct MpsScratchDelete {
+    void operator()(MpsScratch* s) const;
+};
+
 // Execution context (one per tn_ctx handle).
 struct Ctx {
     int device = 0;
@@ -213,6 +226,12 @@ struct Ctx {
     std::unordered_map<unsigned long long, LzGraph> lzgraphs;
     bool use_graphs = true;
     void clear_graphs();
+    // work buffers of the last MPS that was destroyed, for the next one (its graphs' addresses
+    // then stay the same, and nothing is allocated again); at most one set, freed with the
+    // context.  The lock: an MPS may be destroyed by another thread than the one that uses
+    // the context.
+    std::mutex spare_mu;
+    std::unique_ptr<MpsScratch, MpsScratchDelete> spare;
 };
 
 }  // namespace tnb
