@@ -206,6 +206,7 @@ struct Ctx {
     DevBuf qrsync;         // QR: progress words of the persistent kernel
     DevBuf derr;           // sticky error word of kernels with bounded waits (zero until one expires)
     DevBuf svdw;           // SVD workspace
+    DevBuf wterms;         // MPO term lists
     DevBuf misc;
     DevBuf apiw[3];        // staging copies of the dense-solver entry points
     DevBuf cqr, rr1, rr2;  // RQ / QL factor staging; rank-revealing factorisations' full factors
@@ -215,13 +216,10 @@ struct Ctx {
     bool use_persistent_qr = true;  // TN_NO_PERSISTENT_QR=1: the two-stream look-ahead QR instead
     bool qr_forward_q = true;       // TN_QR_FORWARD_Q=0: the persistent QR forms the thin Q after the panels
     long long qr_spin_limit = 1LL << 21;  // polls per wait in the persistent QR (TN_QR_SPIN_LIMIT)
-    // the last MPO term list of each direction uploaded through the C ABI
-    struct TermCache {
-        DevBuf terms;
-        std::vector<double> W;
-        int key[3] = {0, 0, 0};
-        int n = 0;
-    } wcache[2];
+    // cache of the last MPO term list uploaded through the C ABI
+    std::vector<double> wcache_W;
+    int wcache_key[4] = {0, 0, 0, 0};
+    int wcache_n = 0;
     // device-looped Lanczos graphs by operator key (TN_NO_GRAPHS=1 disables)
     std::unordered_map<unsigned long long, LzGraph> lzgraphs;
     bool use_graphs = true;
