@@ -149,6 +149,24 @@ int upload_terms(Ctx& c, const double* W_host, int d, int Dw1, int Dw2, bool lr,
     return TN_OK;
 }
 
+// The term list for one call: as a kernel argument where it fits, else uploaded.
+struct CallTerms {
+    WTermArg arg;
+    bool fits = false;
+    const WTermDev* dev = nullptr;
+    int n = 0;
+    int make(Ctx& c, const double* W_host, int d, int Dw1, int Dw2, bool lr) {
+        const auto t = build_terms(W_host, d, Dw1, Dw2, lr);
+        n = (int)t.size();
+        fits = n <= WT_ARG_TERMS;
+        if (!fits) return upload_terms(c, W_host, d, Dw1, Dw2, lr, &dev, &n);
+        arg.n = n;
+        std::copy(t.begin(), t.end(), arg.t);
+        return TN_OK;
+    }
+    const WTermArg* as_arg() const { return fits ? &arg : nullptr; }
+};
+
 bool valid_shape(int d, int Dw1, int Dw2, int D1, int D2) {
     return d >= 1 && Dw1 >= 1 && Dw2 >= 1 && D1 >= 1 && D2 >= 1;
 }
@@ -486,7 +504,9 @@ struct tn_heff_s {
     tn_ctx ctx = nullptr;
     int precision = TN_PREC_FP64;
     tnb::ContractShape s{};
-    tnb::DevBuf terms, P, Q;
+    tnb::DevBuf P, Q;
+    tnb::DevBuf terms;     // the term list where it does not fit an argument
+    tnb::WTermArg arg;
     int nterms = 0;
     const double* F = nullptr;
     const double* G = nullptr;
@@ -514,9 +534,16 @@ int tn_heff_create(tn_ctx c, int precision, int d, int Dw1, int Dw2, int D1, int
     h->F = F;
     h->G = G;
     auto t = build_terms(W_host, d, Dw1, Dw2, true);
-    int st = h->terms.ensure(sizeof(WTermDev) * t.size());
-    if (st == TN_OK && cudaMemcpy(h->terms.p, t.data(), sizeof(WTermDev) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-        st = TN_CUDA_ERROR;
+    int st = TN_OK;
+    if (t.size() <= (size_t)WT_ARG_TERMS) {
+        h->arg.n = (int)t.size();
+        std::copy(t.begin(), t.end(), h->arg.t);
+    } else {
+        st = h->terms.ensure(sizeof(WTermDev) * t.size());
+        if (st == TN_OK &&
+            cudaMemcpy(h->terms.p, t.data(), sizeof(WTermDev) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            st = TN_CUDA_ERROR;
+    }
     h->nterms = (int)t.size();
     if (st == TN_OK) {
         if (precision == TN_PREC_FP64) {
@@ -544,7 +571,7 @@ int tn_heff_apply(tn_heff h, const double* x, double* y) {
     Ctx& cx = h->ctx->c;
     if (h->precision == TN_PREC_FP64)
         return heff_matvec_f64(h->s, h->terms.as<WTermDev>(), h->nterms, h->F, h->G, x, y, h->P.as<double>(),
-                               h->Q.as<double>(), nullptr, cx.stream);
+                               h->Q.as<double>(), nullptr, cx.stream, h->terms.p ? nullptr : &h->arg);
     return heff_matvec_mixed(cx, h->ms, x, y, nullptr);
 }
 
@@ -571,14 +598,14 @@ int tn_heff_matvec(tn_ctx c, int precision, int d, int Dw1, int Dw2, int D1, int
         return st != TN_OK ? st : st2;
     }
     Ctx& cx = c->c;
-    const WTermDev* t;
-    int nt;
-    TN_CHECK(upload_terms(cx, W_host, d, Dw1, Dw2, true, &t, &nt));
+    CallTerms t;
+    TN_CHECK(t.make(cx, W_host, d, Dw1, Dw2, true));
     ContractShape s{d, Dw1, Dw2, D1, D2};
     size_t scr = sizeof(double) * contract_scratch_doubles(s);
     TN_CHECK(cx.P.ensure(scr));
     TN_CHECK(cx.Q.ensure(scr));
-    TN_CHECK(heff_matvec_f64(s, t, nt, F, G, x, y, cx.P.as<double>(), cx.Q.as<double>(), nullptr, cx.stream));
+    TN_CHECK(heff_matvec_f64(s, t.dev, t.n, F, G, x, y, cx.P.as<double>(), cx.Q.as<double>(), nullptr, cx.stream,
+                             t.as_arg()));
     return TN_OK;
 }
 
@@ -604,14 +631,13 @@ int tn_env_left(tn_ctx c, int precision, int d, int Dw1, int Dw2, int D1, int D2
     if (!valid_shape(d, Dw1, Dw2, D1, D2)) return TN_BAD_SHAPE;
     if (precision != TN_PREC_FP64) return TN_BAD_ARG;
     Ctx& cx = c->c;
-    const WTermDev* t;
-    int nt;
-    TN_CHECK(upload_terms(cx, W_host, d, Dw1, Dw2, true, &t, &nt));
+    CallTerms t;
+    TN_CHECK(t.make(cx, W_host, d, Dw1, Dw2, true));
     ContractShape s{d, Dw1, Dw2, D1, D2};
     size_t scr = sizeof(double) * contract_scratch_doubles(s);
     TN_CHECK(cx.P.ensure(scr));
     TN_CHECK(cx.Q.ensure(scr));
-    return env_left_f64(s, t, nt, A, F, Fout, cx.P.as<double>(), cx.Q.as<double>(), cx.stream);
+    return env_left_f64(s, t.dev, t.n, A, F, Fout, cx.P.as<double>(), cx.Q.as<double>(), cx.stream, t.as_arg());
 }
 
 int tn_env_right(tn_ctx c, int precision, int d, int Dw1, int Dw2, int D1, int D2, const double* W_host,
@@ -621,14 +647,13 @@ int tn_env_right(tn_ctx c, int precision, int d, int Dw1, int Dw2, int D1, int D
     if (!valid_shape(d, Dw1, Dw2, D1, D2)) return TN_BAD_SHAPE;
     if (precision != TN_PREC_FP64) return TN_BAD_ARG;
     Ctx& cx = c->c;
-    const WTermDev* t;
-    int nt;
-    TN_CHECK(upload_terms(cx, W_host, d, Dw1, Dw2, false, &t, &nt));
+    CallTerms t;
+    TN_CHECK(t.make(cx, W_host, d, Dw1, Dw2, false));
     ContractShape s{d, Dw1, Dw2, D1, D2};
     size_t scr = sizeof(double) * contract_scratch_doubles(s);
     TN_CHECK(cx.P.ensure(scr));
     TN_CHECK(cx.Q.ensure(scr));
-    return env_right_f64(s, t, nt, A, G, Gout, cx.P.as<double>(), cx.Q.as<double>(), cx.stream);
+    return env_right_f64(s, t.dev, t.n, A, G, Gout, cx.P.as<double>(), cx.Q.as<double>(), cx.stream, t.as_arg());
 }
 
 int tn_eigensolve_heff(tn_ctx c, const tn_solver_options* opt, int d, int Dw1, int Dw2, int D1, int D2,

@@ -12,25 +12,44 @@ namespace tnb {
 
 namespace {
 
-__global__ void wcombine_kernel(const double* __restrict__ P, double* __restrict__ Q,
-                                const WTermDev* __restrict__ terms, int nterms, long long blk,
-                                const int* skip) {
-    if (skip && *skip) return;
+// Q[out] = sum over the terms of out of c P[in], in list order (sorted by out).
+__device__ __forceinline__ void combine_terms(const double* __restrict__ P, double* __restrict__ Q,
+                                              const WTermDev* terms, int nterms, long long blk) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < blk;
          e += (long long)gridDim.x * blockDim.x) {
         int cur = terms[0].out;
         double acc = 0.0;
-        for (int t = 0; t < nterms; ++t) {
-            WTermDev tm = terms[t];
-            if (tm.out != cur) {
-                Q[(long long)cur * blk + e] = acc;
-                acc = 0.0;
-                cur = tm.out;
+        for (int t0 = 0; t0 < nterms; t0 += 8) {  // eight blocks' loads in flight
+            double v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = t0 + q < nterms ? P[(long long)terms[t0 + q].in * blk + e] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                if (t0 + q >= nterms) break;
+                const WTermDev tm = terms[t0 + q];
+                if (tm.out != cur) {
+                    Q[(long long)cur * blk + e] = acc;
+                    acc = 0.0;
+                    cur = tm.out;
+                }
+                acc = fma(tm.c, v[q], acc);
             }
-            acc = fma(tm.c, P[(long long)tm.in * blk + e], acc);
         }
         Q[(long long)cur * blk + e] = acc;
     }
+}
+
+__global__ void wcombine_kernel(const double* __restrict__ P, double* __restrict__ Q,
+                                const WTermDev* __restrict__ terms, int nterms, long long blk,
+                                const int* skip) {
+    if (skip && *skip) return;
+    combine_terms(P, Q, terms, nterms, blk);
+}
+
+__global__ void wcombine_arg_kernel(const double* __restrict__ P, double* __restrict__ Q,
+                                    const __grid_constant__ WTermArg a, long long blk, const int* skip) {
+    if (skip && *skip) return;
+    combine_terms(P, Q, a.t, a.n, blk);
 }
 
 __global__ void heff_diag_kernel(int d, int Dw1, int Dw2, int D1, int D2, const double* __restrict__ Wd,
@@ -116,6 +135,15 @@ int wcombine(const double* P, double* Q, const WTermDev* terms, int nterms, long
              const int* skip, cudaStream_t st) {
     if (blk <= 0) return TN_OK;
     wcombine_kernel<<<grid_for(blk), 256, 0, st>>>(P, Q, terms, nterms, blk, skip);
+    TN_LAUNCH_CHECK();
+    return TN_OK;
+}
+
+static int combine(const double* P, double* Q, const WTermDev* terms, int nterms, const WTermArg* arg, long long blk,
+                   const int* skip, cudaStream_t st) {
+    if (!arg) return wcombine(P, Q, terms, nterms, blk, skip, st);
+    if (blk <= 0) return TN_OK;
+    wcombine_arg_kernel<<<grid_for(blk), 256, 0, st>>>(P, Q, *arg, blk, skip);
     TN_LAUNCH_CHECK();
     return TN_OK;
 }
@@ -223,7 +251,8 @@ int heff_diag(const ContractShape& s, const double* Wdev, const double* F, const
 
 // y = Heff x  (FP64).  P, Q: scratch of d*max(Dw1,Dw2)*D1*D2 doubles each.
 int heff_matvec_f64(const ContractShape& s, const WTermDev* termsLR, int nLR, const double* F, const double* G,
-                    const double* x, double* y, double* P, double* Q, const int* skip, cudaStream_t st) {
+                    const double* x, double* y, double* P, double* Q, const int* skip, cudaStream_t st,
+                    const WTermArg* arg) {
     const int d = s.d, Dw1 = s.Dw1, Dw2 = s.Dw2, D1 = s.D1, D2 = s.D2;
     const long long blk = (long long)D1 * D2;
     // Stage 1: P[w1][n] = F_w1 x_n
@@ -235,7 +264,7 @@ int heff_matvec_f64(const ContractShape& s, const WTermDev* termsLR, int nLR, co
     g1.skip = skip;
     TN_CHECK(gemm_f64(g1, st));
     // Stage 2: Q[m][w2] = sum W P
-    TN_CHECK(wcombine(P, Q, termsLR, nLR, blk, skip, st));
+    TN_CHECK(combine(P, Q, termsLR, nLR, arg, blk, skip, st));
     // Stage 3: y_m = sum_w2 Q[m][w2] G_w2^T, split over w2 for parallelism:
     // partial P[w2][m] = Q[m][w2] G_w2^T (the stage-1 buffer is free again), then a
     // deterministic sum over w2.
@@ -263,7 +292,7 @@ int heff_matvec_f64(const ContractShape& s, const WTermDev* termsLR, int nLR, co
 }
 
 int env_left_f64(const ContractShape& s, const WTermDev* termsLR, int nLR, const double* A, const double* F,
-                 double* Fout, double* P, double* Q, cudaStream_t st) {
+                 double* Fout, double* P, double* Q, cudaStream_t st, const WTermArg* arg) {
     const int d = s.d, Dw1 = s.Dw1, Dw2 = s.Dw2, D1 = s.D1, D2 = s.D2;
     const long long blk = (long long)D1 * D2;
     GemmArgs g1;
@@ -272,7 +301,7 @@ int env_left_f64(const ContractShape& s, const WTermDev* termsLR, int nLR, const
     g1.B.ptr = A; g1.B.k = idx(1); g1.B.mn = idx(D1); g1.B.sb1 = blk;
     g1.C.ptr = P; g1.C.m = idx(1); g1.C.n = idx(D1); g1.C.sb0 = d * blk; g1.C.sb1 = blk;
     TN_CHECK(gemm_f64(g1, st));
-    TN_CHECK(wcombine(P, Q, termsLR, nLR, blk, nullptr, st));
+    TN_CHECK(combine(P, Q, termsLR, nLR, arg, blk, nullptr, st));
     // F'_w2(i2,j2) = sum_{m,i1} A_m(i1,i2) Q[m][w2](i1,j2), split over m:
     // partial P[m][w2] = A_m^T Q[m][w2] (D2 x D2), then a sum over m.
     GemmArgs g3;
@@ -290,7 +319,7 @@ int env_left_f64(const ContractShape& s, const WTermDev* termsLR, int nLR, const
 }
 
 int env_right_f64(const ContractShape& s, const WTermDev* termsRL, int nRL, const double* A, const double* G,
-                  double* Gout, double* P, double* Q, cudaStream_t st) {
+                  double* Gout, double* P, double* Q, cudaStream_t st, const WTermArg* arg) {
     const int d = s.d, Dw1 = s.Dw1, Dw2 = s.Dw2, D1 = s.D1, D2 = s.D2;
     const long long blk = (long long)D1 * D2;
     // P[w2][n] = G_w2 A_n^T   (D2 x D1, column-major)
@@ -300,7 +329,7 @@ int env_right_f64(const ContractShape& s, const WTermDev* termsRL, int nRL, cons
     g1.B.ptr = A; g1.B.k = idx(D1); g1.B.mn = idx(1); g1.B.sb1 = blk;
     g1.C.ptr = P; g1.C.m = idx(1); g1.C.n = idx(D2); g1.C.sb0 = d * blk; g1.C.sb1 = blk;
     TN_CHECK(gemm_f64(g1, st));
-    TN_CHECK(wcombine(P, Q, termsRL, nRL, blk, nullptr, st));
+    TN_CHECK(combine(P, Q, termsRL, nRL, arg, blk, nullptr, st));
     // G'_w1(i1,j1) = sum_{m,i2} A_m(i1,i2) Q[m][w1](i2,j1), split over m:
     // partial P[m][w1] = A_m Q[m][w1] (D1 x D1), then a sum over m.
     GemmArgs g3;

@@ -14,6 +14,13 @@ struct WTermDev {
     double c;
 };
 
+// A term list that travels as a kernel argument: nothing to upload, wait for or keep.
+constexpr int WT_ARG_TERMS = 128;  // 2 KB of the 4 KB a kernel's arguments may take (Dw = 5: 16 terms at d = 2, 23 at d = 3)
+struct WTermArg {
+    int n;
+    WTermDev t[WT_ARG_TERMS];
+};
+
 std::vector<WTermDev> build_terms(const double* W, int d, int Dw1, int Dw2, bool leftToRight);
 
 int wcombine(const double* P, double* Q, const WTermDev* terms, int nterms, long long blk, const int* skip,
@@ -31,12 +38,14 @@ int slab_sum(const double* in, int nslab, long long slab, double* out, const int
 int slab_sum_skip(const double* in, int nslab, long long slab, double* out, const int* skip, cudaStream_t st);
 int heff_diag(const ContractShape& s, const double* Wdev, const double* F, const double* G, double* diag,
               cudaStream_t st);
+// With arg the terms come from it, else from the device list.
 int heff_matvec_f64(const ContractShape& s, const WTermDev* termsLR, int nLR, const double* F, const double* G,
-                    const double* x, double* y, double* P, double* Q, const int* skip, cudaStream_t st);
+                    const double* x, double* y, double* P, double* Q, const int* skip, cudaStream_t st,
+                    const WTermArg* arg = nullptr);
 int env_left_f64(const ContractShape& s, const WTermDev* termsLR, int nLR, const double* A, const double* F,
-                 double* Fout, double* P, double* Q, cudaStream_t st);
+                 double* Fout, double* P, double* Q, cudaStream_t st, const WTermArg* arg = nullptr);
 int env_right_f64(const ContractShape& s, const WTermDev* termsRL, int nRL, const double* A, const double* G,
-                  double* Gout, double* P, double* Q, cudaStream_t st);
+                  double* Gout, double* P, double* Q, cudaStream_t st, const WTermArg* arg = nullptr);
 
 // Doubles each of the two contraction scratch buffers (P, Q) must hold.
 inline size_t contract_scratch_doubles(const ContractShape& s) {
