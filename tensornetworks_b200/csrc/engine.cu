@@ -437,6 +437,10 @@ int MPSState::rescale_site(int ia) {
 // Thin QR of the gauge matrix W (m x n, ld m; overwritten) into Q (m x k, ld m)
 // and R (k x n, ld ldr): blocked Householder.
 int MPSState::gauge_qr(int m, int n, double* W, double* Q, double* R, int ldr) {
+    if (opt.precision != TN_PREC_FP64) {
+        const int st = qr_cluster(*ctx, m, n, W, 1, m, Q, 1, m, R, 1, ldr);
+        if (st != QR_UNAVAILABLE) return st;
+    }
     return qr_dense(*ctx, m, n, W, Q, m, R, ldr);
 }
 
