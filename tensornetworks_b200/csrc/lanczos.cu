@@ -4,7 +4,7 @@
 // LapackEigenSolver.C:62-109).  Everything except the decision to restart stays
 // on the device: the dots, the full reorthogonalisation (classical Gram-Schmidt
 // applied twice, FP64 coefficients), the norm, the tridiagonal eigenproblem
-// (multisection on Sturm counts over a whole thread block) and the convergence
+// (multisection on Sturm counts by one warp) and the convergence
 // flag.  Kernels launched after convergence see the flag and return at once.
 // Vector passes are grid-stride, coalesced, FP64, with warp-shuffle block
 // reductions and a deterministic last-block final reduction.
@@ -13,6 +13,7 @@
 #include "tridiag.cuh"
 #include "pdl.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 #include <vector>
@@ -66,27 +67,125 @@ __device__ void reduce_partials(const double* partial, int nb, int stride, int n
     }
 }
 
-// acc + sgn * sum_{k < nk} c[k] V[k N + i] with the basis loads issued eight at
+// Many sums over a block at once.  A butterfly that halves the values instead of repeating every step for each
+// (31 exchanges for 32 values instead of 160), the same additions in the same order as block_sum_chunk, so the
+// same sums bit for bit.  warp_sums leaves value lane / (32 / NV) in each lane.
+template <int NV, int O = 16, int LEN>
+__device__ __forceinline__ double warp_sums(double (&v)[LEN]) {
+    if constexpr (O == 0) {
+        return v[0];
+    } else if constexpr (NV > 1) {
+        const bool up = threadIdx.x & O;
+#pragma unroll
+        for (int q = 0; q < NV / 2; ++q) {
+            const double mine = up ? v[q + NV / 2] : v[q], other = up ? v[q] : v[q + NV / 2];
+            v[q] = mine + __shfl_xor_sync(0xffffffffu, other, O);
+        }
+        return warp_sums<NV / 2, O / 2>(v);
+    } else {
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+        return warp_sums<1, O / 2>(v);
+    }
+}
+
+constexpr int LZ_CHUNK = 32;                    // sums a thread keeps in registers
+constexpr int LZ_WARPS = LZ_THREADS / 32;
+constexpr int LZ_SUMS = LZ_CHUNK * (LZ_WARPS + 1);  // shared memory of block_sums
+
+// Threads q < nq end with the block's sum of value q (nq <= NV).
+template <int NV>
+__device__ __forceinline__ double block_sums_n(double (&v)[LZ_CHUNK], double* sh) {
+    static_assert(LZ_WARPS == 16, "the tree below");
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const double s = warp_sums<NV>(v);
+    __syncthreads();  // sh may still be read
+    if (lane % (32 / NV) == 0) sh[lane / (32 / NV) * (LZ_WARPS + 1) + wid] = s;
+    __syncthreads();
+    if (threadIdx.x >= NV) return 0.0;
+    double t[LZ_WARPS];
+#pragma unroll
+    for (int i = 0; i < LZ_WARPS; ++i) t[i] = sh[threadIdx.x * (LZ_WARPS + 1) + i];
+#pragma unroll
+    for (int o = LZ_WARPS / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; ++i) t[i] += t[i + o];
+    return t[0];
+}
+__device__ __forceinline__ double block_sums(double (&v)[LZ_CHUNK], int nq, double* sh) {
+    if (nq <= 8) return block_sums_n<8>(v, sh);
+    if (nq <= 16) return block_sums_n<16>(v, sh);
+    return block_sums_n<32>(v, sh);
+}
+
+// out[k] = sum over the nv blocks' partials partial[k nv + b], k < nk <= LZ_MAXK, by the whole block, a warp per k:
+// the order of reduce_partials, so its values (nv <= LZ_MAXBLOCKS, one partial per thread there).
+constexpr int LZ_MAXBLOCKS = 256;
+__device__ __forceinline__ void sum_partials(const double* partial, int nv, int nk, double* out) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int U = 2;
+    for (int k0 = wid; k0 < nk; k0 += U * LZ_WARPS) {
+        double x[U][LZ_MAXBLOCKS / 32];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * LZ_WARPS;
+#pragma unroll
+            for (int i = 0; i < LZ_MAXBLOCKS / 32; ++i) {
+                const int b = 32 * i + lane;
+                x[u][i] = k < nk && b < nv ? __ldcg(partial + (long long)k * nv + b) : 0.0;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            double t = warp_sums<LZ_MAXBLOCKS / 32>(x[u]);  // of the 32 blocks of lane / 4
+            t += __shfl_xor_sync(0xffffffffu, t, 16);
+            t += __shfl_xor_sync(0xffffffffu, t, 8);
+            t += __shfl_xor_sync(0xffffffffu, t, 4);
+            if (lane == 0 && k0 + u * LZ_WARPS < nk) out[k0 + u * LZ_WARPS] = t;
+        }
+    }
+    __syncthreads();
+}
+
+// acc + sgn * sum_{k < nk} c[k] V[k N + i] with the basis loads issued sixteen at
 // a time (independent, all in flight before their FMAs): a thread touches only a
 // few elements, so without this the loop is one load latency per basis vector.
 __device__ __forceinline__ double basis_combine(const double* __restrict__ V, long long N, long long i,
                                                 const double* c, int nk, double sgn, double acc) {
+    constexpr int B = 16;
     int k = 0;
-    for (; k + 8 <= nk; k += 8) {
-        double v[8];
+    for (; k + B <= nk; k += B) {
+        double v[B];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = __ldg(V + (long long)(k + q) * N + i);
+        for (int q = 0; q < B; ++q) v[q] = __ldg(V + (long long)(k + q) * N + i);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc = fma(sgn * c[k + q], v[q], acc);
+        for (int q = 0; q < B; ++q) acc = fma(sgn * c[k + q], v[q], acc);
     }
-    double v[8];
+    double v[B];
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < B; ++q)
         if (k + q < nk) v[q] = __ldg(V + (long long)(k + q) * N + i);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < B; ++q)
         if (k + q < nk) acc = fma(sgn * c[k + q], v[q], acc);
     return acc;
+}
+
+// s[q] += V[(k0 + q) N + i] x, q < LZ_CHUNK, k0 + q < nk, eight loads at a time
+__device__ __forceinline__ void basis_dots(const double* __restrict__ V, long long N, long long i, int k0, int nk,
+                                           double x, double (&s)[LZ_CHUNK]) {
+    constexpr int B = 8;
+#pragma unroll
+    for (int c0 = 0; c0 < LZ_CHUNK; c0 += B) {
+        if (k0 + c0 < nk) {
+            double v[B];
+#pragma unroll
+            for (int q = 0; q < B; ++q)
+                if (k0 + c0 + q < nk) v[q] = __ldg(V + (long long)(k0 + c0 + q) * N + i);
+#pragma unroll
+            for (int q = 0; q < B; ++q)
+                if (k0 + c0 + q < nk) s[c0 + q] = fma(v[q], x, s[c0 + q]);
+        }
+    }
 }
 
 // Step j's tridiagonal problem (alpha, beta of steps 0..j in the state), by the
@@ -104,17 +203,21 @@ __device__ void lz_decide_step(LzState* st, int j, cudaGraphConditionalHandle co
     }
     __syncthreads();
     if (threadIdx.x >= 32) return;  // warp 0 decides (the callers' next barrier waits for it)
-    const double th = warp_eig_k(nk, a, b, 0);
+    __shared__ double2 rows[LZ_MAXK];
+    const double th = warp_eig_exact(nk, a, b, rows, 0, [] {});
+    double tn = 0;
+    if (st->tol_rel > 0) {
+        for (int i = threadIdx.x; i < nk; i += 32)
+            tn = fmax(tn, fabs(a[i]) + fabs(b[i]) + (i > 0 ? fabs(b[i - 1]) : 0.0));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) tn = fmax(tn, __shfl_xor_sync(0xffffffffu, tn, o));
+    }
     if (threadIdx.x == 0) {
-        const double yl = last_component(nk, a, b, th);
+        const double yl = last_component_rows(nk, rows, a, b, th);
         const double bj = b[j];
         const double resid = bj * yl;
         double tolEff = fmax(st->tol, 1e-13 * fmax(1.0, fabs(th)));
-        if (st->tol_rel > 0) {
-            double tn = 0;
-            for (int i = 0; i < nk; ++i) tn = fmax(tn, fabs(a[i]) + fabs(b[i]) + (i > 0 ? fabs(b[i - 1]) : 0.0));
-            tolEff = fmax(tolEff, st->tol_rel * tn);
-        }
+        if (st->tol_rel > 0) tolEff = fmax(tolEff, st->tol_rel * tn);
         st->theta = th;
         st->resid = resid;
         st->nb = nk;
@@ -245,105 +348,102 @@ __global__ void lz_scale_kernel(const double* x, double* v0, long long N, const 
 // of a last block reducing them at the end of the previous kernel while the
 // other SMs idle.
 
+// Vector passes: what bounds them is the basis, nk N doubles from L2 for each of the three kernels, and the
+// sums that end them.  All sums of a pass stay in registers (LZ_CHUNK at a time) and are reduced together, the
+// update reads the basis once from L2 (a second time from L1), and the step's tridiagonal
+// problem has a block of its own beside the vector's.  N = 262144, 40 vectors (20 on average): dots, update and
+// next 9.0, 14.6 and 14.7 us where they took 16.1, 23.1 and 30.3.
+
 // Partials of h_k = V_k . w, k = 0..j, into partA.
-__global__ void lz_dots_kernel(const double* __restrict__ V, const double* __restrict__ w, long long N,
-                               double* partA, LzState* st) {
+__global__ void __launch_bounds__(LZ_THREADS) lz_dots_kernel(const double* __restrict__ V,
+                                                             const double* __restrict__ w, long long N, double* partA,
+                                                             LzState* st) {
     pdl_wait();
     if (st->done) return;
-    __shared__ double sh[KCHUNK * 32];
-    __shared__ double res[KCHUNK];
-    const int j = st->j;
-    const int nk = j + 1;
-    for (int k0 = 0; k0 < nk; k0 += KCHUNK) {
-        double v[KCHUNK] = {0};
+    __shared__ double sh[LZ_SUMS];
+    const int nk = st->j + 1;
+    for (int k0 = 0; k0 < nk; k0 += LZ_CHUNK) {
+        const int nq = min(LZ_CHUNK, nk - k0);
+        double v[LZ_CHUNK] = {0};
         for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
-             i += (long long)gridDim.x * blockDim.x) {
-            double wi = w[i];
-#pragma unroll
-            for (int q = 0; q < KCHUNK; ++q)
-                if (k0 + q < nk) v[q] = fma(V[(long long)(k0 + q) * N + i], wi, v[q]);
-        }
-        block_sum_chunk(v, res, sh);
-        if (threadIdx.x < KCHUNK && k0 + threadIdx.x < nk)
-            partA[(long long)blockIdx.x * LZ_MAXK + k0 + threadIdx.x] = res[threadIdx.x];
+             i += (long long)gridDim.x * blockDim.x)
+            basis_dots(V, N, i, k0, nk, w[i], v);
+        const double t = block_sums(v, nq, sh);
+        if ((int)threadIdx.x < nq) partA[(long long)(k0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
     }
 }
 
 // h from partA; w' = w - V h; partials of h2 = V^T w' and |w'|^2 into partB.
 // Block 0 keeps h in the state (alpha_j = h_j + h2_j is formed next).
-__global__ void lz_update_kernel(const double* __restrict__ V, double* __restrict__ w, long long N,
-                                 const double* partA, double* partB, LzState* st) {
+__global__ void __launch_bounds__(LZ_THREADS) lz_update_kernel(const double* __restrict__ V, double* __restrict__ w,
+                                                               long long N, const double* partA, double* partB,
+                                                               LzState* st) {
     pdl_wait();
     if (st->done) return;
-    __shared__ double sh[KCHUNK * 32];
-    __shared__ double res[KCHUNK];
-    __shared__ double hs[LZ_MAXK + KCHUNK];
-    const int j = st->j;
-    const int nk = j + 1;
-    reduce_partials(partA, gridDim.x, LZ_MAXK, nk, hs, sh);
+    __shared__ double sh[LZ_SUMS];
+    __shared__ double hs[LZ_MAXK];
+    const int nk = st->j + 1;
+    sum_partials(partA, gridDim.x, nk, hs);
     if (blockIdx.x == 0)
         for (int k = threadIdx.x; k < nk; k += blockDim.x) st->h[k] = hs[k];
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        double wi = w[i];
-        wi = basis_combine(V, N, i, hs, nk, -1.0, wi);
-        w[i] = wi;
-    }
-    for (int k0 = 0; k0 < nk + 1; k0 += KCHUNK) {
-        double v[KCHUNK] = {0};
+    for (int k0 = 0; k0 < nk + 1; k0 += LZ_CHUNK) {
+        const int nq = min(LZ_CHUNK, nk + 1 - k0);
+        double v[LZ_CHUNK] = {0};
         for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
              i += (long long)gridDim.x * blockDim.x) {
             double wi = w[i];
+            if (k0 == 0) w[i] = wi = basis_combine(V, N, i, hs, nk, -1.0, wi);
+            basis_dots(V, N, i, k0, nk, wi, v);
 #pragma unroll
-            for (int q = 0; q < KCHUNK; ++q) {
-                int k = k0 + q;
-                if (k < nk) v[q] = fma(V[(long long)k * N + i], wi, v[q]);
-                else if (k == nk) v[q] = fma(wi, wi, v[q]);
-            }
+            for (int q = 0; q < LZ_CHUNK; ++q)
+                if (k0 + q == nk) v[q] = fma(wi, wi, v[q]);
         }
-        block_sum_chunk(v, res, sh);
-        if (threadIdx.x < KCHUNK && k0 + (int)threadIdx.x <= nk)
-            partB[(long long)blockIdx.x * LZ_MAXK + k0 + threadIdx.x] = res[threadIdx.x];
+        const double t = block_sums(v, nq, sh);
+        if ((int)threadIdx.x < nq) partB[(long long)(k0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
     }
 }
 
 // h2 and |w'|^2 from partB, beta_j; V_{j+1} = (w' - V h2) / beta_j, also into
-// the matvec input xcur.  Block 0 records alpha_j and beta_j, then solves the
+// the matvec input xcur.  Block 0 records alpha_j and beta_j, solves the
 // tridiagonal problem of step j and decides whether the restart ends (and,
-// inside a graph loop, whether the loop runs another step), after its share
-// of the vector.  The last block to finish advances the step index.  Blocks
+// inside a graph loop, whether the loop runs another step); the others have the
+// vector.  The last block to finish advances the step index.  Blocks
 // that start after block 0 has ended the restart return at once; the step's
 // vector is then unused (and the half-counted ticket is cleared by the next
 // reset).
-__global__ void lz_next_kernel(double* __restrict__ V, const double* __restrict__ w, long long N,
-                               const double* partB, LzState* st, double* __restrict__ xcur, VecSplit sp,
-                               cudaGraphConditionalHandle cond = 0) {
+__global__ void __launch_bounds__(LZ_THREADS) lz_next_kernel(double* __restrict__ V, const double* __restrict__ w,
+                                                             long long N, const double* partB, LzState* st,
+                                                             double* __restrict__ xcur, VecSplit sp,
+                                                             cudaGraphConditionalHandle cond = 0) {
     pdl_wait();
     if (st->done) {
         if (cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
         return;
     }
-    __shared__ double sh[KCHUNK * 32];
-    __shared__ double h2s[LZ_MAXK + KCHUNK];
+    __shared__ double h2s[LZ_MAXK];
     __shared__ bool last;
     const int j = st->j;
     const int nk = j + 1;
-    reduce_partials(partB, gridDim.x, LZ_MAXK, nk + 1, h2s, sh);
+    const int nv = gridDim.x - 1;  // vector blocks
+    sum_partials(partB, nv, nk + 1, h2s);
     double ss = 0;
     for (int k = 0; k < nk; ++k) ss = fma(h2s[k], h2s[k], ss);
     const double beta = sqrt(fmax(h2s[nk] - ss, 0.0));
-    const double inv = beta > 0 ? 1.0 / beta : 0.0;
-    double* vn = V + (long long)(j + 1) * N;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        double wi = w[i];
-        wi = basis_combine(V, N, i, h2s, nk, -1.0, wi);
-        wi *= inv;
-        vn[i] = wi;
-        xcur[i] = wi;
-        if (sp.out) split_bf16((float)wi, sp.ns, sp.out, sp.stride, i);
-    }
-    if (blockIdx.x == 0) {
+    if (blockIdx.x > 0) {
+        const double inv = beta > 0 ? 1.0 / beta : 0.0;
+        double* vn = V + (long long)(j + 1) * N;
+        for (long long i = (blockIdx.x - 1) * (long long)blockDim.x + threadIdx.x; i < N;
+             i += (long long)nv * blockDim.x) {
+            double wi = w[i];
+            wi = basis_combine(V, N, i, h2s, nk, -1.0, wi);
+            wi *= inv;
+            vn[i] = wi;
+            xcur[i] = wi;
+            if (sp.out) split_bf16((float)wi, sp.ns, sp.out, sp.stride, i);
+        }
+    } else {
+        for (int k = threadIdx.x; k < nk; k += blockDim.x) st->h2[k] = h2s[k];
         if (threadIdx.x == 0) {
-            for (int k = 0; k < nk; ++k) st->h2[k] = h2s[k];
             st->alpha[j] = st->h[j] + h2s[j];
             st->beta[j] = beta;
             st->matvecs += 1;
@@ -365,47 +465,27 @@ __global__ void lz_next_kernel(double* __restrict__ V, const double* __restrict_
     }
 }
 
-// Ritz coefficients y of the lowest eigenpair of T_nb (inverse iteration), and theta2.
-__global__ void lz_ritz_coeffs_kernel(LzState* st) {
+// Ritz coefficients y of the lowest eigenpair of T_nb (inverse iteration; its eigenvalue is the last
+// decision's theta), and theta2: a warp each.
+__global__ void __launch_bounds__(64) lz_ritz_coeffs_kernel(LzState* st) {
     const int n = st->nb;
     if (n <= 0) return;
-    __shared__ double a[LZ_MAXK], b[LZ_MAXK];
+    __shared__ double a[LZ_MAXK], b[LZ_MAXK], y[LZ_MAXK], work[6 * LZ_MAXK];
+    __shared__ double2 rows[LZ_MAXK];
+    __shared__ int piv[LZ_MAXK];
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         a[i] = st->alpha[i];
         b[i] = st->beta[i];
     }
     __syncthreads();
-    // warp 0 the lowest eigenvalue, warp 1 the next (the gap, for the statistics)
-    __shared__ double ths[2];
-    const int wv = threadIdx.x >> 5;
-    if (wv < 2) {
-        const double e = (wv == 0 || n > 1) ? warp_eig_k(n, a, b, wv) : 0.0;
-        if ((threadIdx.x & 31) == 0) ths[wv] = e;
+    const double th = st->theta;
+    if (threadIdx.x >= 32) {
+        const double th2 = n > 1 ? warp_eig_exact(n, a, b, rows, 1, [] {}) : th;
+        if (threadIdx.x == 32) st->theta2 = th2;
+        return;
     }
-    __syncthreads();
-    const double th = ths[0], th2 = n > 1 ? ths[1] : th;
-    if (threadIdx.x != 0) return;
-    st->theta = th;
-    st->theta2 = th2;
-    __shared__ double y[LZ_MAXK], dl[LZ_MAXK], dd[LZ_MAXK], du[LZ_MAXK], du2[LZ_MAXK];
-    __shared__ int piv[LZ_MAXK];
-    double scale = 0;
-    for (int i = 0; i < n; ++i) scale = fmax(scale, fabs(a[i]) + (i < n - 1 ? fabs(b[i]) : 0.0));
-    scale = fmax(scale, 1e-300);
-    for (int i = 0; i < n; ++i) y[i] = 1.0 + 0.1 * ((i * 7919) % 97) / 97.0;
-    for (int it = 0; it < 3; ++it) {
-        tri_solve(n, a, b, th + 4e-15 * scale, 2.2e-16 * scale, y, dl, dd, du, du2, piv);
-        double mx = 0;
-        for (int i = 0; i < n; ++i) mx = fmax(mx, fabs(y[i]));
-        if (mx > 0) for (int i = 0; i < n; ++i) y[i] /= mx;
-    }
-    double nr = 0;
-    for (int i = 0; i < n; ++i) nr += y[i] * y[i];
-    nr = sqrt(nr);
-    int im = 0;
-    for (int i = 1; i < n; ++i) if (fabs(y[i]) > fabs(y[im])) im = i;
-    double sg = (y[im] < 0) ? -1.0 : 1.0;
-    for (int i = 0; i < n; ++i) st->y[i] = sg * y[i] / nr;
+    tri_ritz_exact(n, a, b, th, y, work, piv);
+    for (int i = threadIdx.x; i < n; i += 32) st->y[i] = y[i];
 }
 
 // x = V y
@@ -484,7 +564,7 @@ __global__ void rq_resid_kernel(const double* __restrict__ x, const double* __re
 
 inline int vec_grid(long long N, int sm) {
     long long b = (N + LZ_THREADS - 1) / LZ_THREADS;
-    long long cap = (long long)sm;
+    long long cap = std::min(sm, LZ_MAXBLOCKS);
     if (b > cap) b = cap;
     if (b < 1) b = 1;
     return (int)b;
@@ -509,7 +589,7 @@ static int enqueue_lz_step(Ctx& c, const MatvecFn& mv, int grid, double* V, doub
     TN_CHECK(step_matvec_dots(c, mv, grid, V, w, xcur, N, partial, s));
     TN_CHECK(launch_pdl(lz_update_kernel, grid, LZ_THREADS, 0, c.stream, (const double*)V, w, N,
                         (const double*)partial, partB, s));
-    return launch_pdl(lz_next_kernel, grid, LZ_THREADS, 0, c.stream, V, (const double*)w, N, (const double*)partB, s,
+    return launch_pdl(lz_next_kernel, grid + 1, LZ_THREADS, 0, c.stream, V, (const double*)w, N, (const double*)partB, s,
                       xcur, sp, cond);
 }
 
@@ -605,7 +685,7 @@ int lanczos_solve(Ctx& c, long long N, double* x, int m, int maxRestarts, double
             for (int j = 0; j < mm; ++j) TN_CHECK(enqueue_step(0));
         }
         if (c.prof) TN_CUDA_CHECK(cudaEventRecord(c.pev[4], st));
-        lz_ritz_coeffs_kernel<<<1, LZ_THREADS, 0, st>>>(s);
+        lz_ritz_coeffs_kernel<<<1, 64, 0, st>>>(s);
         TN_LAUNCH_CHECK();
         lz_ritz_vector_kernel<<<grid, LZ_THREADS, 0, st>>>(V, x, N, s);
         TN_LAUNCH_CHECK();
@@ -768,7 +848,7 @@ int lanczos_solve_async(Ctx& c, long long N, double* x, int m, int maxRestarts, 
         const unsigned long long kpi = launch_count() - n0;
         if (rc != TN_OK) return fail(rc);
         rc = capture_into(st, b_out, {n_in}, [&]() -> int {
-            lz_ritz_coeffs_kernel<<<1, LZ_THREADS, 0, st>>>(s);
+            lz_ritz_coeffs_kernel<<<1, 64, 0, st>>>(s);
             lz_ritz_vector_kernel<<<grid, LZ_THREADS, 0, st>>>(V, xw, N, s);
             lz_decide_kernel<<<1, 32, 0, st>>>(s, h_out, maxR, N, mm);
             return cudaGetLastError() == cudaSuccess ? TN_OK : TN_CUDA_ERROR;
