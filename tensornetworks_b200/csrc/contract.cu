@@ -6,7 +6,13 @@
 // G'_w1 = sum_{m,n,w2} W(w1,w2)(m,n) A_m G_w2 A_n^T       (IterateRightF, :352-400)
 // Each is three stages: a batched GEMM, the sparse W combination (memory
 // bound, one pass), and a GEMM over the concatenated (w, bond) index.
+// These kernels, the GEMM, the copies and the slab sums are launched as programmatic dependents: each
+// waits for its predecessor before it reads memory, and is launched and set up
+// while the predecessor drains.  None lets its own dependent go early: waiting CTAs
+// placed beside a GEMM's spread unevenly over the SMs.  Environment updates
+// 250 x 203, two directions: 84 us with ordinary launches, 68 so, 102 with early triggers.
 #include "contract.h"
+#include "pdl.cuh"
 
 namespace tnb {
 
@@ -42,12 +48,14 @@ __device__ __forceinline__ void combine_terms(const double* __restrict__ P, doub
 __global__ void wcombine_kernel(const double* __restrict__ P, double* __restrict__ Q,
                                 const WTermDev* __restrict__ terms, int nterms, long long blk,
                                 const int* skip) {
+    pdl_wait();
     if (skip && *skip) return;
     combine_terms(P, Q, terms, nterms, blk);
 }
 
 __global__ void wcombine_arg_kernel(const double* __restrict__ P, double* __restrict__ Q,
                                     const __grid_constant__ WTermArg a, long long blk, const int* skip) {
+    pdl_wait();
     if (skip && *skip) return;
     combine_terms(P, Q, a.t, a.n, blk);
 }
@@ -75,6 +83,7 @@ __global__ void heff_diag_kernel(int d, int Dw1, int Dw2, int D1, int D2, const 
 
 __global__ void copy2d_kernel(int rows, int cols, const double* __restrict__ src, IdxMap sr, IdxMap sc,
                               double* __restrict__ dst, IdxMap dr, IdxMap dc, double scale) {
+    pdl_wait();
     long long total = (long long)rows * cols;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
@@ -85,6 +94,7 @@ __global__ void copy2d_kernel(int rows, int cols, const double* __restrict__ src
 
 // out[e] = sum_s in[s*slab + e]  (deterministic split-K reduction)
 __global__ void slab_sum_kernel(const double* __restrict__ in, int nslab, long long slab, double* __restrict__ out) {
+    pdl_wait();
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < slab;
          e += (long long)gridDim.x * blockDim.x) {
         double s = 0.0;
@@ -134,18 +144,14 @@ std::vector<WTermDev> build_terms(const double* W, int d, int Dw1, int Dw2, bool
 int wcombine(const double* P, double* Q, const WTermDev* terms, int nterms, long long blk,
              const int* skip, cudaStream_t st) {
     if (blk <= 0) return TN_OK;
-    wcombine_kernel<<<grid_for(blk), 256, 0, st>>>(P, Q, terms, nterms, blk, skip);
-    TN_LAUNCH_CHECK();
-    return TN_OK;
+    return launch_pdl(wcombine_kernel, grid_for(blk), 256, 0, st, P, Q, terms, nterms, blk, skip);
 }
 
 static int combine(const double* P, double* Q, const WTermDev* terms, int nterms, const WTermArg* arg, long long blk,
                    const int* skip, cudaStream_t st) {
     if (!arg) return wcombine(P, Q, terms, nterms, blk, skip, st);
     if (blk <= 0) return TN_OK;
-    wcombine_arg_kernel<<<grid_for(blk), 256, 0, st>>>(P, Q, *arg, blk, skip);
-    TN_LAUNCH_CHECK();
-    return TN_OK;
+    return launch_pdl(wcombine_arg_kernel, grid_for(blk), 256, 0, st, P, Q, *arg, blk, skip);
 }
 
 namespace {
@@ -191,13 +197,13 @@ int dense_shift_spd(int N, const double* A, int lda, double* W, double* sigma, c
 int copy2d(int rows, int cols, const double* src, IdxMap sr, IdxMap sc, double* dst, IdxMap dr, IdxMap dc,
            double scale, cudaStream_t st) {
     if (rows <= 0 || cols <= 0) return TN_OK;
-    copy2d_kernel<<<grid_for((long long)rows * cols), 256, 0, st>>>(rows, cols, src, sr, sc, dst, dr, dc, scale);
-    TN_LAUNCH_CHECK();
-    return TN_OK;
+    return launch_pdl(copy2d_kernel, grid_for((long long)rows * cols), 256, 0, st, rows, cols, src, sr, sc, dst, dr, dc,
+                      scale);
 }
 
 __global__ void slab_sum_skip_kernel(const double* __restrict__ in, int nslab, long long slab, double* __restrict__ out,
                                      const int* skip) {
+    pdl_wait();
     if (*skip) return;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < slab;
          e += (long long)gridDim.x * blockDim.x) {
@@ -209,17 +215,13 @@ __global__ void slab_sum_skip_kernel(const double* __restrict__ in, int nslab, l
 
 int slab_sum_skip(const double* in, int nslab, long long slab, double* out, const int* skip, cudaStream_t st) {
     if (slab <= 0) return TN_OK;
-    slab_sum_skip_kernel<<<grid_for(slab), 256, 0, st>>>(in, nslab, slab, out, skip);
-    TN_LAUNCH_CHECK();
-    return TN_OK;
+    return launch_pdl(slab_sum_skip_kernel, grid_for(slab), 256, 0, st, in, nslab, slab, out, skip);
 }
 
 int slab_sum(const double* in, int nslab, long long slab, double* out, const int* skip, cudaStream_t st) {
     if (slab <= 0) return TN_OK;
     (void)skip;
-    slab_sum_kernel<<<grid_for(slab), 256, 0, st>>>(in, nslab, slab, out);
-    TN_LAUNCH_CHECK();
-    return TN_OK;
+    return launch_pdl(slab_sum_kernel, grid_for(slab), 256, 0, st, in, nslab, slab, out);
 }
 
 __global__ void shift_vector_kernel(double* p, long long n, double v) {

@@ -8,6 +8,7 @@
 // split-index operands the SIMT kernel: tile 64x64x16, 256 threads, 4x4
 // outputs per thread, register-staged double buffering of the next k-tile.
 #include "dgemm.cuh"
+#include "pdl.cuh"
 #include "tn_internal.h"
 
 namespace tnb {
@@ -143,7 +144,6 @@ __global__ void __launch_bounds__(DG_NT) gemm_f64_dmma_kernel(LinGemm g) {
     constexpr int WM = BM / 2, WN = BN / 2, MI = WM / 8, NI = WN / 8;
     using OpA = DgOperand<BM, A_MC, V, DG_NT>;
     using OpB = DgOperand<BN, !B_KC, V, DG_NT>;
-    if (g.skip && *g.skip) return;
     extern __shared__ __align__(16) double dg_smem[];
     double* As = dg_smem;
     double* Bs = dg_smem + DG_STAGES * OpA::STAGE;
@@ -160,6 +160,9 @@ __global__ void __launch_bounds__(DG_NT) gemm_f64_dmma_kernel(LinGemm g) {
     OpB ob;
     oa.init(t, Ab, g.sAm, g.sAk, m0, g.M);
     ob.init(t, Bb, g.sBn, g.sBk, n0, g.N);
+    // nothing above reads memory: launch and prologue run beside the predecessor's tail
+    pdl_wait();
+    if (g.skip && *g.skip) return;
     double acc[MI][NI][2];
 #pragma unroll
     for (int i = 0; i < MI; ++i)
@@ -239,9 +242,7 @@ int dg_launch(const LinGemm& l, int batches, cudaStream_t st) {
         return TN_BAD_SHAPE;
     }
     const dim3 grid((unsigned)tiles, 1, batches);
-    kern<<<grid, DG_NT, bytes, st>>>(l);
-    TN_LAUNCH_CHECK();
-    return TN_OK;
+    return launch_pdl(kern, grid, DG_NT, bytes, st, l);
 }
 
 template <int BM, int BN>
