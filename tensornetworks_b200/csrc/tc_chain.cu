@@ -8,15 +8,22 @@
 // form one thread-block cluster.  Each CTA runs the usual tcgen05 pipeline on
 // its chunk range (warp 0: TMA loads into a 128-byte-swizzled ring; warp 1:
 // one elected thread issues the BF16 piece products into a TMEM accumulator;
-// warps 2-5: tcgen05.ld of the accumulator into shared memory).  The cluster
-// then reduces: CTA r sums rows [r*128/splitk, (r+1)*128/splitk) of the tile
-// over the partials of all CTAs of the cluster, read through distributed
-// shared memory in a fixed order (deterministic), and writes them either as
+// warps 2-5: tcgen05.ld of the accumulator).  With splitk > 1 CTA r sums rows
+// [r*128/splitk, (r+1)*128/splitk) of the tile: warps 2-5 send every row of their CTA's
+// partial to the CTA that sums it (st.async, counted by an mbarrier there) and each
+// CTA adds the partials in rank order (deterministic).  The results are written either as
 // BF16 pieces (row-major: the A operand of the next GEMM) or as FP64
-// (column-major: the site-tensor layout).  No partial ever goes to HBM.
+// (column-major: the site-tensor layout); with splitk = 1 straight from the
+// accumulator.  No partial ever goes to HBM.
 //
-// Every mbarrier wait is bounded; on expiry the CTA records an error code and
-// still takes both cluster barriers, so no CTA of a cluster waits for a peer
+// What bounds it at the sizes of a sweep (2 to 6 chunks per CTA) is a chain of latencies:
+// first TMA ~0.9 us, ~0.6 us per chunk (48 KB), the accumulator 0.5, then the exchange.  Staging the
+// partial, a cluster barrier, reading the peers' staging and a second barrier took 4.4 of
+// 7.6 us; with the partials sent the d = 2, D = 256 matvec (two of these kernels and the splitting of x)
+// went from 26.7 to 22.8 us.
+//
+// Every mbarrier wait is bounded; on expiry the CTA records an error code, still
+// sends its partial and takes the cluster barriers, so no CTA of a cluster waits for a peer
 // that has left.
 #include <cuda_bf16.h>
 
@@ -44,17 +51,14 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
     return out;
 }
 
-// Not volatile: the loads of one thread are free to overlap; the cluster
-// barriers around the reduction order them against the peers' writes.
-__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
-    float4 v;
-    asm("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-    return v;
+__device__ __forceinline__ void st_async_v4(uint32_t addr, float a, float b, float c, float d, uint32_t mbar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "f"(a), "f"(b), "f"(c), "f"(d), "r"(mbar)
+                 : "memory");
 }
 
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 template <int NS>
 struct ChainSmem {
@@ -62,33 +66,60 @@ struct ChainSmem {
     static constexpr int B_BYTES = CBN * BK * 2;  // 8 KB per piece
     static constexpr int STAGE_BYTES = NS * (A_BYTES + B_BYTES);
     static constexpr int NSTAGE = (4 * STAGE_BYTES + 1024 <= 220 * 1024) ? 4 : ((3 * STAGE_BYTES + 1024 <= 220 * 1024) ? 3 : 2);
-    static constexpr int SROW = CBN + 4;  // staging row stride (floats): 16-byte rows, float4 traffic conflict-free
-    static constexpr int STAGING_BYTES = BM * SROW * 4;
     static constexpr int RING = NSTAGE * STAGE_BYTES;
-    static constexpr int TOTAL = (RING > STAGING_BYTES ? RING : STAGING_BYTES) + 1024;
+    // landing place of the partials: behind the ring where both fit, else over it (once no CTA's MMA reads it)
+    static constexpr int LAND_BYTES = BM * CBN * 4;
+    static constexpr bool OWN_LAND = RING + LAND_BYTES + 2048 <= 227 * 1024;
+    static constexpr int LAND = OWN_LAND ? RING : 0;
+    static constexpr int TOTAL = (OWN_LAND ? RING + LAND_BYTES : RING) + 1024;
 };
 
-template <int NS, int OUT>
+// Four columns of a row as BF16 pieces (`left` of them exist): one 8-byte store per piece (row pitch and first
+// column are multiples of 4).
+template <int NS>
+__device__ __forceinline__ void store_pieces(uint16_t* dst, long long piece, const float* v, int left) {
+    float rem[4] = {v[0], v[1], v[2], v[3]};
+#pragma unroll
+    for (int pc = 0; pc < NS; ++pc) {
+        uint16_t h[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __nv_bfloat16 b = __float2bfloat16_rn(rem[i]);
+            h[i] = __bfloat16_as_ushort(b);
+            rem[i] -= __bfloat162float(b);
+        }
+        uint16_t* d = dst + (long long)pc * piece;
+        if (left >= 4) {
+            *reinterpret_cast<uint2*>(d) =
+                make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                if (i < left) d[i] = h[i];
+        }
+    }
+}
+
+template <int NS, int OUT, int SK>
 __global__ void __launch_bounds__(THREADS, 1)
     tc_chain_kernel(const __grid_constant__ TcMaps maps, TcChainArgs p) {
     using SL = ChainSmem<NS>;
     constexpr int STAGES = SL::NSTAGE;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full_bar[4], empty_bar[4], accum_bar;
+    __shared__ uint64_t full_bar[4], empty_bar[4], accum_bar, land_bar;
     __shared__ uint32_t tmem_base_sh;
     __shared__ int s_fail;
 
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    float* stg = reinterpret_cast<float*>(smem);  // staging of the FP32 tile, reuses the ring
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * CBN;
-    const int split = p.splitk > 1 ? (int)cluster_ctarank() : 0;
-    const int ob = blockIdx.z / p.splitk;
+    const int split = SK > 1 ? (int)cluster_ctarank() : 0;
+    const int ob = blockIdx.z / SK;
     const int nkseg = (p.K + BK - 1) / BK;
     const int sbeg = p.seg_start[ob], send = p.seg_start[ob + 1];
     const int nchunk = (send - sbeg) * nkseg;
-    const int q0 = (int)((long long)split * nchunk / p.splitk);
-    const int q1 = (int)((long long)(split + 1) * nchunk / p.splitk);
+    const int q0 = (int)((long long)split * nchunk / SK);
+    const int q1 = (int)((long long)(split + 1) * nchunk / SK);
     const bool has_work = q1 > q0;
 
     if (threadIdx.x == 32) {
@@ -105,8 +136,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             mbar_init(&empty_bar[s], 1);
         }
         mbar_init(&accum_bar, 1);
+        mbar_init(&land_bar, 1);
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (SK > 1) mbar_expect_tx(&land_bar, SL::LAND_BYTES);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
@@ -117,9 +150,13 @@ __global__ void __launch_bounds__(THREADS, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = tmem_base_sh;
+    if (SK > 1) cluster_arrive();  // land_bar is ready for the peers' messages
+    TcSeg sg = {};                 // the segment tables are the plan's, not the predecessor's
+    if (threadIdx.x == 0 && has_work) sg = p.segs[sbeg + q0 / nkseg];
     // the prologue above touched nothing the predecessor writes
     pdl_launch_dependents();
     pdl_wait();
+    if (SK > 1) cluster_wait();
     // the flag is read by every CTA of a cluster alike, so a skipped launch leaves no peer waiting
     if (p.skip && *p.skip) {
         if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)CBN));
@@ -133,8 +170,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const int s = it % STAGES;
                 const uint32_t ph = (it / STAGES) & 1;
                 if (!mbar_wait(&empty_bar[s], ph ^ 1)) { s_fail = 1; break; }
-                const TcSeg sg = p.segs[sbeg + q / nkseg];
                 const int kc = q % nkseg;
+                if (q > q0 && kc == 0) sg = p.segs[sbeg + q / nkseg];
                 uint8_t* st = smem + s * SL::STAGE_BYTES;
                 mbar_expect_tx(&full_bar[s], SL::STAGE_BYTES);
 #pragma unroll
@@ -179,21 +216,48 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (has_work) ok = __all_sync(0xffffffffu, mbar_wait(&accum_bar, 0) ? 1 : 0) != 0;
         fence_after();
         if (!ok) s_fail = 1;
-        float* srow = stg + r * SL::SROW;
-        if (has_work && ok) {
-            const uint32_t tbase = tmem + ((uint32_t)(qd * 32) << 16);
-#pragma unroll
-            for (int c0 = 0; c0 < CBN; c0 += 16) {
-                float v[16];
+        if (SK > 1 && !SL::OWN_LAND) {
+            cluster_arrive();  // this CTA's MMA has read the ring (warps 0 and 1 below)
+            cluster_wait();
+        }
+        constexpr int RB = BM / SK;
+        const uint32_t tbase = tmem + ((uint32_t)(qd * 32) << 16);
+        const int row = m0 + r;
+        uint32_t dst = 0, bar = 0;
+        if (SK > 1) {
+            dst = mapa_shared(smem_u32(smem + SL::LAND), r / RB) + (split * RB + r % RB) * (CBN * 4);
+            bar = mapa_shared(smem_u32(&land_bar), r / RB);
+        }
+#pragma unroll 1
+        for (int c0 = 0; c0 < CBN; c0 += 16) {
+            float v[16];
+            if (has_work && ok)
                 tmem_ld16(tbase + (uint32_t)c0, v);
+            else
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = 0.f;
+            if (SK > 1) {  // granules of 16 bytes, swizzled by the row so that neither side has bank conflicts
 #pragma unroll
                 for (int i = 0; i < 16; i += 4)
-                    *reinterpret_cast<float4*>(srow + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-            }
-        } else {
+                    st_async_v4(dst + (((c0 + i) / 4) ^ (r % RB & 15)) * 16, v[i], v[i + 1], v[i + 2], v[i + 3], bar);
+            } else if (row < p.M) {
+                if (OUT == TCC_OUT_F64_COLMAJOR) {
+                    double* d64 = p.c64 + (long long)ob * p.c64_batch + (long long)(n0 + c0) * p.ldc64 + row;
 #pragma unroll
-            for (int c = 0; c < CBN; c += 4) *reinterpret_cast<float4*>(srow + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int i = 0; i < 16; ++i)
+                        if (n0 + c0 + i < p.N) d64[(long long)i * p.ldc64] = (double)v[i];
+                } else {
+                    uint16_t* d16 = p.c16 + (long long)ob * p.c16_batch + (long long)row * p.ldc16 + n0 + c0;
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4) store_pieces<NS>(d16 + i, p.c16_piece, v + i, p.N - (n0 + c0 + i));
+                }
+            }
         }
+    }
+    if (SK > 1 && !SL::OWN_LAND && warp < 2) {
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
     }
     fence_before();
     __syncthreads();
@@ -201,104 +265,63 @@ __global__ void __launch_bounds__(THREADS, 1)
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)CBN));
     }
-    if (p.splitk > 1) cluster_sync_all();
-
-    // cluster reduction of this CTA's rows and the output: work item = one row
-    // and four consecutive columns; the partial of every CTA of the cluster is
-    // read with one 16-byte load each (all issued before the sum), in rank order.
-    const int RB = BM / p.splitk;
-    const int rbase = split * RB;
-    const uint32_t stg_addr = smem_u32(stg);
-    constexpr int CG = CBN / 4;
-    const int items = RB * CG;
-    for (int e = threadIdx.x; e < items; e += THREADS) {
-        int rl, cg;
-        if (OUT == TCC_OUT_F64_COLMAJOR) {  // consecutive threads: consecutive rows (coalesced column writes)
-            rl = rbase + e % RB;
-            cg = e / RB;
-        } else {                            // consecutive threads: consecutive column groups of a row
-            rl = rbase + e / CG;
-            cg = e % CG;
-        }
-        const uint32_t off = (uint32_t)((rl * SL::SROW + 4 * cg) * 4);
-        float4 part[8];
+    if (SK > 1) {
+        cluster_arrive();  // this CTA's messages are on their way
+        if (!mbar_wait(&land_bar, 0)) s_fail = 2;
+        // this CTA's rows: work item = one row and four consecutive columns
+        constexpr int RB = BM / SK, CG = CBN / 4;
+        const uint8_t* land = smem + SL::LAND;
+#pragma unroll 1
+        for (int e = threadIdx.x; e < RB * CG; e += THREADS) {
+            // FP64: consecutive threads consecutive rows (coalesced column writes); BF16: column groups of a row
+            const int lr = OUT == TCC_OUT_F64_COLMAJOR ? e % RB : e / CG, cg = OUT == TCC_OUT_F64_COLMAJOR ? e / RB : e % CG;
+            float4 part[SK];
 #pragma unroll
-        for (int pr = 0; pr < 8; ++pr)
-            if (pr < p.splitk)
-                part[pr] = p.splitk > 1 ? ld_cluster_v4(mapa_shared(stg_addr + off, pr))
-                                        : *reinterpret_cast<const float4*>(stg + rl * SL::SROW + 4 * cg);
-        const int row = m0 + rl, col0 = n0 + 4 * cg;
-        if (OUT == TCC_OUT_F64_COLMAJOR) {
-            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int pr = 0; pr < SK; ++pr)
+                part[pr] = *reinterpret_cast<const float4*>(land + (pr * RB + lr) * (CBN * 4) + (cg ^ (lr & 15)) * 16);
+            const int row = m0 + split * RB + lr, col0 = n0 + 4 * cg;
+            if (row >= p.M) continue;
+            if (OUT == TCC_OUT_F64_COLMAJOR) {
+                double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-            for (int pr = 0; pr < 8; ++pr)
-                if (pr < p.splitk) {
+                for (int pr = 0; pr < SK; ++pr) {
                     acc[0] += (double)part[pr].x;
                     acc[1] += (double)part[pr].y;
                     acc[2] += (double)part[pr].z;
                     acc[3] += (double)part[pr].w;
                 }
-            if (row < p.M) {
-                double* dst = p.c64 + (long long)ob * p.c64_batch + row;
+                double* dst = p.c64 + (long long)ob * p.c64_batch + (long long)col0 * p.ldc64 + row;
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    if (col0 + i < p.N) dst[(long long)(col0 + i) * p.ldc64] = acc[i];
-            }
-        } else {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                    if (col0 + i < p.N) dst[(long long)i * p.ldc64] = acc[i];
+            } else {
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int pr = 0; pr < 8; ++pr)
-                if (pr < p.splitk) {
+                for (int pr = 0; pr < SK; ++pr) {
                     acc[0] += part[pr].x;
                     acc[1] += part[pr].y;
                     acc[2] += part[pr].z;
                     acc[3] += part[pr].w;
                 }
-            if (row < p.M) {
-                uint16_t* dst = p.c16 + (long long)ob * p.c16_batch + (long long)row * p.ldc16 + col0;
-                if (col0 + 4 <= p.N) {
-                    // four columns per piece in one 8-byte store (row pitch and col0 are multiples of 4)
-#pragma unroll
-                    for (int pc = 0; pc < NS; ++pc) {
-                        uint16_t h[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const __nv_bfloat16 b = __float2bfloat16_rn(acc[i]);
-                            h[i] = __bfloat16_as_ushort(b);
-                            acc[i] -= __bfloat162float(b);
-                        }
-                        uint2 w;
-                        w.x = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
-                        w.y = (uint32_t)h[2] | ((uint32_t)h[3] << 16);
-                        *reinterpret_cast<uint2*>(dst + (long long)pc * p.c16_piece) = w;
-                    }
-                } else {
-                    for (int i = 0; i < 4 && col0 + i < p.N; ++i) {
-                        float rem = acc[i];
-#pragma unroll
-                        for (int pc = 0; pc < NS; ++pc) {
-                            const __nv_bfloat16 b = __float2bfloat16_rn(rem);
-                            dst[(long long)pc * p.c16_piece + i] = __bfloat16_as_ushort(b);
-                            rem -= __bfloat162float(b);
-                        }
-                    }
-                }
+                store_pieces<NS>(p.c16 + (long long)ob * p.c16_batch + (long long)row * p.ldc16 + col0, p.c16_piece, acc,
+                                 p.N - col0);
             }
         }
+        if (s_fail == 2) __nanosleep(200000);  // messages that were given up may still be on their way
+        __syncwarp();
+        cluster_wait();                        // no CTA leaves before its peers have sent
     }
-    // peers may still be reading this CTA's staging tile
-    if (p.splitk > 1) cluster_sync_all();
     if (threadIdx.x == 0 && s_fail && p.err) atomicExch(p.err, 1);
 }
 
-template <int NS, int OUT>
+template <int NS, int OUT, int SK>
 int launch_chain(const TcChainPlan& pl, cudaStream_t st) {
     const TcChainArgs& p = pl.args;
     const int smem = ChainSmem<NS>::TOTAL;
-    auto kern = tc_chain_kernel<NS, OUT>;
+    auto kern = tc_chain_kernel<NS, OUT, SK>;
     TN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((p.N + CBN - 1) / CBN, (p.M + BM - 1) / BM, p.nbatch * p.splitk);
+    cfg.gridDim = dim3((p.N + CBN - 1) / CBN, (p.M + BM - 1) / BM, p.nbatch * SK);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -307,11 +330,11 @@ int launch_chain(const TcChainPlan& pl, cudaStream_t st) {
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
-    if (p.splitk > 1) {
+    if (SK > 1) {
         attr[na].id = cudaLaunchAttributeClusterDimension;
         attr[na].val.clusterDim.x = 1;
         attr[na].val.clusterDim.y = 1;
-        attr[na].val.clusterDim.z = p.splitk;
+        attr[na].val.clusterDim.z = SK;
         ++na;
     }
     cfg.attrs = attr;
@@ -319,6 +342,16 @@ int launch_chain(const TcChainPlan& pl, cudaStream_t st) {
     TN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, pl.maps, p));
     count_launch();
     return TN_OK;
+}
+
+template <int NS, int OUT>
+int launch_chain(const TcChainPlan& pl, cudaStream_t st) {
+    switch (pl.args.splitk) {
+        case 1: return launch_chain<NS, OUT, 1>(pl, st);
+        case 2: return launch_chain<NS, OUT, 2>(pl, st);
+        case 4: return launch_chain<NS, OUT, 4>(pl, st);
+        default: return launch_chain<NS, OUT, 8>(pl, st);
+    }
 }
 
 }  // namespace
