@@ -11,12 +11,12 @@ int qr_dense(Ctx& c, int m, int n, double* W, double* Qout, int ldq, double* Rou
 // The QR of A (element (i, c) at A[i ars + c acs], left as it is) by thread-block clusters in one
 // launch: Q (m x k) and R (k x n, zeros written below the diagonal), each with
 // its own strides, when the pointers are non-null.  The same reflectors as qr_dense (dlarfg's signs),
-// sums in another order.  QR_UNAVAILABLE (nothing enqueued) for m > 1536, for more column
+// sums in another order.  colmap (device, may be null): column c of the matrix is column colmap[c] of A.  QR_UNAVAILABLE (nothing enqueued) for m > 1536, for more column
 // blocks of 32 than clusters fit on the device, and when the context's settings
 // ask for another path.
 constexpr int QR_UNAVAILABLE = -1;
 int qr_cluster(Ctx& c, int m, int n, const double* A, long long ars, long long acs, double* Q, long long qrs,
-               long long qcs, double* R, long long rrs, long long rcs);
+               long long qcs, double* R, long long rrs, long long rcs, const int* colmap = nullptr);
 
 // Reads (and clears) the context's sticky device error word, raised when a
 // bounded wait between CTAs expired; waits for the device.
@@ -39,6 +39,7 @@ struct SvdJob {
     int ldvt;
     double* s;
     int* sweeps;  // may be null
+    const int* perm = nullptr;  // set by svd_batched: W is R^T and V is Q of the permuted matrix
 };
 
 int svd_batched(Ctx& c, const std::vector<SvdJob>& jobs, bool vectors);

@@ -51,6 +51,7 @@ struct QcArgs {
     int nb;                       // column blocks of A; clusters past them take blocks of Q's rows
     const double* A;
     long long ars, acs;           // row and column strides
+    const int* colmap;            // columns of A in the matrix's order, or null
     double* Q;                    // m x k
     long long qrs, qcs;
     double* R;                    // k x n
@@ -179,7 +180,10 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
         each(L::rows * C, true, [&](int c, int lr, int i) { Cs[c * ldr + lr] = i == c0 + c ? 1.0 : 0.0; });
     else
         each(L::rows * C, a.ars == 1, [&](int c, int lr, int i) {
-            Cs[c * ldr + lr] = (i < a.m && c < ncol) ? a.A[(long long)i * a.ars + (long long)(c0 + c) * a.acs] : 0.0;
+            double v = 0.0;
+            if (i < a.m && c < ncol)
+                v = a.A[(long long)i * a.ars + (long long)(a.colmap ? a.colmap[c0 + c] : c0 + c) * a.acs];
+            Cs[c * ldr + lr] = v;
         });
     cl.sync();  // barriers are initialised before the first remote arrival
     // A wait that ran out raises the error words and marks the CTA; its threads go on
@@ -588,7 +592,7 @@ int qc_launch(Ctx& c, QcArgs a, bool* served) {
 }  // namespace
 
 int qr_cluster(Ctx& c, int m, int n, const double* A, long long ars, long long acs, double* Q, long long qrs,
-               long long qcs, double* R, long long rrs, long long rcs) {
+               long long qcs, double* R, long long rrs, long long rcs, const int* colmap) {
     if (!c.use_persistent_qr || !c.qr_forward_q || m < 1 || n < 1 || m > 1536) return QR_UNAVAILABLE;
     const int k = std::min(m, n);
     // a block of A is read when its cluster starts: outputs in A's memory take the path with a copy
@@ -605,7 +609,7 @@ int qr_cluster(Ctx& c, int m, int n, const double* A, long long ars, long long a
     a.m = m; a.n = n; a.k = k;
     a.K = (k + 31) / 32;
     a.nb = (n + 31) / 32;
-    a.A = A; a.ars = ars; a.acs = acs;
+    a.A = A; a.ars = ars; a.acs = acs; a.colmap = colmap;
     a.Q = Q; a.qrs = qrs; a.qcs = qcs;
     a.R = R; a.rrs = rrs; a.rcs = rcs;
     bool served = false;

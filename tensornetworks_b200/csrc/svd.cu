@@ -43,15 +43,16 @@ __device__ __forceinline__ int rr_pos(int q, int r, int ne) {
 // rest of the space may be spread evenly over them), the one with the largest
 // remainder 1 - sum_p U(e, p)^2 is taken, which is never zero while columns are
 // missing.  U is read by L2 loads: other CTAs may have written it in this
-// launch.  dots: n doubles of shared memory, red and at: 32 each.
-__device__ void complete_u(const SvdJob& jb, double cut, double* red, double* dots, int* at) {
-    const int m = jb.m, n = jb.n;
+// launch.  U(i, c), i < m, at U[i rs + c cs].  dots: n doubles of shared memory, red and at: 32 each.
+__device__ void complete_u(const SvdJob& jb, double* U, long long rs, long long cs, int m, double cut, double* red,
+                           double* dots, int* at) {
+    const int n = jb.n;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
     int next_e = 0;
     for (int c = 0; c < n; ++c) {
         const double sc = __ldcg(jb.s + c);
         if (sc > cut && sc > 0.0) continue;
-        double* uc = jb.U + (size_t)c * jb.ldu;
+        double* uc = U + c * cs;
         auto accepted = [&](int p) {
             const double sp = __ldcg(jb.s + p);
             return p != c && ((sp > cut && sp > 0.0) || p < c);
@@ -66,7 +67,7 @@ __device__ void complete_u(const SvdJob& jb, double cut, double* red, double* do
                     double r = 1.0;
                     for (int p = 0; p < n; ++p)
                         if (accepted(p)) {
-                            const double u = __ldcg(jb.U + (size_t)p * jb.ldu + i);
+                            const double u = __ldcg(U + p * cs + i * rs);
                             r = fma(-u, u, r);
                         }
                     if (r > best) { best = r; bi = i; }
@@ -90,29 +91,29 @@ __device__ void complete_u(const SvdJob& jb, double cut, double* red, double* do
                 __syncthreads();
                 e = at[0];
             }
-            for (int i = tid; i < m; i += blockDim.x) uc[i] = (i == e) ? 1.0 : 0.0;
+            for (int i = tid; i < m; i += blockDim.x) uc[i * rs] = (i == e) ? 1.0 : 0.0;
             __syncthreads();
             for (int pass = 0; pass < 2; ++pass) {
                 for (int p = wid; p < n; p += nw) {
                     double part = 0;
                     if (accepted(p)) {
-                        const double* up = jb.U + (size_t)p * jb.ldu;
-                        for (int i = lane; i < m; i += 32) part = fma(__ldcg(up + i), __ldcg(uc + i), part);
+                        const double* up = U + p * cs;
+                        for (int i = lane; i < m; i += 32) part = fma(__ldcg(up + i * rs), __ldcg(uc + i * rs), part);
                     }
                     part = wsum(part);
                     if (lane == 0) dots[p] = part;
                 }
                 __syncthreads();
                 for (int i = tid; i < m; i += blockDim.x) {
-                    double v = __ldcg(uc + i);
+                    double v = __ldcg(uc + i * rs);
                     for (int p = 0; p < n; ++p)
-                        if (dots[p] != 0.0) v = fma(-dots[p], __ldcg(jb.U + (size_t)p * jb.ldu + i), v);
-                    uc[i] = v;
+                        if (dots[p] != 0.0) v = fma(-dots[p], __ldcg(U + p * cs + i * rs), v);
+                    uc[i * rs] = v;
                 }
                 __syncthreads();
             }
             double part = 0;
-            for (int i = tid; i < m; i += blockDim.x) part = fma(__ldcg(uc + i), __ldcg(uc + i), part);
+            for (int i = tid; i < m; i += blockDim.x) part = fma(__ldcg(uc + i * rs), __ldcg(uc + i * rs), part);
             part = wsum(part);
             if (lane == 0) red[wid] = part;
             __syncthreads();
@@ -121,7 +122,7 @@ __device__ void complete_u(const SvdJob& jb, double cut, double* red, double* do
             __syncthreads();
             const double nr = sqrt(nr2);
             if (nr > 0.5 || last) {
-                for (int i = tid; i < m; i += blockDim.x) uc[i] = nr > 0.0 ? __ldcg(uc + i) / nr : 0.0;
+                for (int i = tid; i < m; i += blockDim.x) uc[i * rs] = nr > 0.0 ? __ldcg(uc + i * rs) / nr : 0.0;
                 placed = true;
             }
             __syncthreads();
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_svd_kernel(const SvdJob* _
             for (int i = lane; i < n; i += 32) jb.Vt[(size_t)i * jb.ldvt + rk] = vj[i];
         }
         __syncthreads();
-        complete_u(jb, cut, red, norms, at);
+        complete_u(jb, jb.U, 1, jb.ldu, m, cut, red, norms, at);
     }
     if (tid == 0 && jb.sweeps) *jb.sweeps = s_sweeps;
 }
@@ -270,10 +271,10 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_svd_kernel(const SvdJob* _
 //
 // What bounds it: the serial chain of a round -- inbox read, two times (dot,
 // butterfly, angle, update: 650-1000 cycles), write -- 1.3-1.9 us, times
-// n / 2 - 1 rounds, times 11-19 sweeps (150 x 128 graded over three decades: 17
-// sweeps, 2.1 ms).  One CTA per matrix spends that latency per pair of each
+// n / 2 - 1 rounds, times the sweeps (9-11 after a QR factorisation, 14-19 without).  One CTA per matrix spends that latency per pair of each
 // warp's share and reads every column from shared memory (or L2) three times
 // per round.
+constexpr int SVD_PRE_MIN = 25;   // columns from which a single matrix is factored first
 constexpr int JC_SLOTS_MAX = 16;  // row slots per column: four columns x 16 doubles = 128 registers
 
 __device__ __forceinline__ double jc_pick(bool hi, double a, double b) { return hi ? b : a; }
@@ -416,7 +417,9 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
     const int gw = rank * nw + wid;          // warp of the cluster
     const int NW = max(1, (n + 3) / 4);      // warps that hold columns
-    const int ET = (m + 31) / 32;
+    const bool pre = jb.perm != nullptr;     // on R^T (n x n) with Q's rows below, see svd_batched
+    const int mt = pre ? n : m, mb = pre ? m : n;  // rows that are orthogonalised, rows that follow
+    const int ET = (mt + 31) / 32;
     const bool on = gw < NW;
     __shared__ int flags[3];                 // rank 0's are used: "something rotated", by sweep modulo 3
     __shared__ double red[32];
@@ -451,8 +454,11 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
             double e = 0.0;
             if (on && col < n) {
                 const int row = lane + 32 * q;
-                if (q < ET) e = row < m ? jb.W[(size_t)col * m + row] : 0.0;
-                else if (vectors) e = (row - 32 * ET == col) ? 1.0 : 0.0;
+                const int low = row - 32 * ET;
+                if (q < ET) e = row < mt ? jb.W[(size_t)col * mt + row] : 0.0;
+                else if (!vectors) e = 0.0;
+                else if (pre) e = low < mb ? jb.V[(size_t)col * mb + low] : 0.0;
+                else e = low == col ? 1.0 : 0.0;
             }
             v[q] = e;
         }
@@ -575,15 +581,19 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
             if (k < 0) return;
             const double sj = sig[j];
             const bool good = sj > cut && sj > 0.0;
-            double* uo = jb.U + (size_t)min(k, n - 1) * jb.ldu;
-            double* vo = jb.Vt + min(k, n - 1);
+            const int kc = min(k, n - 1);
 #pragma unroll
             for (int q = 0; q < E; ++q) {
-                const int row = lane + 32 * q;
+                const int row = lane + 32 * q, low = row - 32 * ET;
                 if (q < ET) {
-                    if (row < m) uo[row] = good ? v[q] / sj : 0.0;
-                } else if (row - 32 * ET < n) {
-                    vo[(size_t)(row - 32 * ET) * jb.ldvt] = v[q];
+                    const double e = good ? v[q] / sj : 0.0;
+                    if (row < mt) {
+                        if (pre) jb.Vt[(size_t)jb.perm[row] * jb.ldvt + kc] = e;
+                        else jb.U[(size_t)kc * jb.ldu + row] = e;
+                    }
+                } else if (low < mb) {
+                    if (pre) jb.U[(size_t)kc * jb.ldu + low] = v[q];
+                    else jb.Vt[(size_t)low * jb.ldvt + kc] = v[q];
                 }
             }
         };
@@ -595,10 +605,37 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
         }
         __threadfence();
         cl.sync();
-        if (rank == 0) complete_u(jb, cut, red, sig, at);
+        if (rank == 0) {
+            if (pre) complete_u(jb, jb.Vt, jb.ldvt, 1, n, cut, red, sig, at);
+            else complete_u(jb, jb.U, 1, jb.ldu, m, cut, red, sig, at);
+        }
     }
     if (rank == 0 && tid == 0 && jb.sweeps) *jb.sweeps = sweep;
     cl.sync();  // no CTA leaves while its shared memory may still be addressed
+}
+
+// perm: the columns of W (m x n) by descending norm, ties by index (a norm that is not a number counts as infinite).
+__global__ void __launch_bounds__(1024) svd_order_kernel(const double* __restrict__ W, int m, int n, int* __restrict__ perm) {
+    extern __shared__ double nrm2[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int c = wid; c < n; c += 32) {
+        const double* w = W + (size_t)c * m;
+        double s = 0;
+#pragma unroll 4
+        for (int i = lane; i < m; i += 32) s = fma(w[i], w[i], s);
+        s = wsum(s);
+        if (lane == 0) nrm2[c] = s >= 0 ? s : __longlong_as_double(0x7ff0000000000000LL);
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        const double sj = nrm2[j];
+        int k = 0;
+        for (int i = 0; i < n; ++i) {
+            const double si = nrm2[i];
+            k += (si > sj) || (si == sj && i < j);
+        }
+        perm[k] = j;
+    }
 }
 
 // Cluster shapes for the largest n and row-slot count of a batch, best first;
@@ -691,21 +728,51 @@ int svd_batched(Ctx& c, const std::vector<SvdJob>& jobs, bool vectors) {
     }
     // Every job of the batch fits the cluster kernel (n <= 512 and at most 16
     // slots of 32 rows per column, rows of U and V together): there it is the
-    // faster one at every size (150 x 128 with vectors 1.95 ms against 26.7,
-    // 25 x 33 0.2 against 1.2); otherwise one CTA per matrix with its columns in
-    // shared memory or L2.
+    // faster one at every size (25 x 25 0.24 against 0.44 ms, 150 x 128 1.95 against
+    // 26.7, both without the factorisation below); otherwise one CTA per matrix with its columns in shared
+    // memory or L2.
     TN_CHECK(ensure_device_error_word(c));
     bool served = false;
     const int nj = (int)jobs.size();
-    for (const JcShape& sh : jc_shapes(nmax, slots)) {
-        if (served) break;
-        if (slots <= 2) TN_CHECK(jc_launch<2>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
-        else if (slots <= 4) TN_CHECK(jc_launch<4>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
-        else if (slots <= 6) TN_CHECK(jc_launch<6>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
-        else if (slots <= 8) TN_CHECK(jc_launch<8>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
-        else if (slots <= 12) TN_CHECK(jc_launch<12>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
-        else TN_CHECK(jc_launch<16>(c, dev, jobs[0], nj, sh, nmax, vectors, &served));
+    const auto shapes = jc_shapes(nmax, slots);
+    auto run = [&](const SvdJob& one) -> int {
+        for (const JcShape& sh : shapes) {
+            if (served) break;
+            if (slots <= 2) TN_CHECK(jc_launch<2>(c, dev, one, nj, sh, nmax, vectors, &served));
+            else if (slots <= 4) TN_CHECK(jc_launch<4>(c, dev, one, nj, sh, nmax, vectors, &served));
+            else if (slots <= 6) TN_CHECK(jc_launch<6>(c, dev, one, nj, sh, nmax, vectors, &served));
+            else if (slots <= 8) TN_CHECK(jc_launch<8>(c, dev, one, nj, sh, nmax, vectors, &served));
+            else if (slots <= 12) TN_CHECK(jc_launch<12>(c, dev, one, nj, sh, nmax, vectors, &served));
+            else TN_CHECK(jc_launch<16>(c, dev, one, nj, sh, nmax, vectors, &served));
+        }
+        return TN_OK;
+    };
+    // A single matrix of some size is factored first, its columns by descending norm: A P = Q R, and the rotations
+    // that orthogonalise the columns of R^T (Drmac and Veselic, SIAM J. Matrix Anal. Appl. 29, 2008: R^T is closer to
+    // diagonal than A) turn Q into U: R^T J = V' S gives A = (Q J) S (P V')^T.  The same kernel with R^T
+    // above and Q's rows below, 9-11 sweeps instead of 14-19.  Factored and not (graded over three decades, host to
+    // host): 16 x 16 140 and 150 us, 20 x 20 166 and 166, 25 x 25 205 and 240, 64 x 64 488 and 630,
+    // 150 x 128 1383 and 1947, 160 x 160 2255 and 3220; 150 x 128 26.7 ms with one CTA per matrix.
+    const SvdJob& j0 = jobs[0];
+    if (nj == 1 && j0.n >= SVD_PRE_MIN && !shapes.empty()) {
+        const size_t nq = vectors ? (size_t)j0.m * j0.n : 0, nr = (size_t)j0.n * j0.n;
+        TN_CHECK(c.svdpre.ensure(sizeof(double) * (nq + nr) + sizeof(int) * (size_t)j0.n));
+        double* Q = c.svdpre.as<double>();
+        double* X = Q + nq;
+        int* perm = reinterpret_cast<int*>(X + nr);
+        svd_order_kernel<<<1, 1024, sizeof(double) * j0.n, c.stream>>>(j0.W, j0.m, j0.n, perm);
+        TN_LAUNCH_CHECK();
+        const int st = qr_cluster(c, j0.m, j0.n, j0.W, 1, j0.m, vectors ? Q : nullptr, 1, j0.m, X, j0.n, 1, perm);
+        if (st != QR_UNAVAILABLE) {
+            TN_CHECK(st);
+            SvdJob p = j0;
+            p.W = X;
+            p.V = Q;
+            p.perm = perm;
+            TN_CHECK(run(p));
+        }
     }
+    if (!served) TN_CHECK(run(j0));
     if (!served) {
         if (!dev) {
             TN_CHECK(c.svdw.ensure(sizeof(SvdJob)));

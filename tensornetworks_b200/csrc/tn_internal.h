@@ -206,6 +206,7 @@ struct Ctx {
     DevBuf qrsync;         // QR: progress words of the persistent kernel
     DevBuf derr;           // sticky error word of kernels with bounded waits (zero until one expires)
     DevBuf svdw;           // SVD workspace
+    DevBuf svdpre;         // SVD of one matrix: Q, R^T and the column order
     DevBuf wterms;         // MPO term lists
     DevBuf misc;
     DevBuf apiw[3];        // staging copies of the dense-solver entry points
