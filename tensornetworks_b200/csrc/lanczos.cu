@@ -188,47 +188,47 @@ __device__ __forceinline__ void basis_dots(const double* __restrict__ V, long lo
     }
 }
 
-// Step j's tridiagonal problem (alpha, beta of steps 0..j in the state), by the
-// whole calling block: the lowest Ritz value, its residual estimate, and the
+// What a step's decision reads, in shared memory: alpha and beta of steps 0..j and fields of the state, the older
+// of them loaded while the step's sums are still on their way.
+struct LzDecision {
+    double a[LZ_MAXK], b[LZ_MAXK];
+    double2 rows[LZ_MAXK];
+    double tol, tol_rel, h, resid2;  // h_j; the residual estimate two steps ago
+    int mmax, matvecs;
+};
+
+// Step j's tridiagonal problem, by one warp: the lowest Ritz value, its residual estimate, and the
 // decision to stop the restart -- converged, the split-precision operator's
 // noise floor (a residual that no longer halves over two steps), or the basis
 // limit -- which, inside a graph loop (cond != 0), also ends the loop.  Every
 // step reaches it, so the loop ends at the latest at the basis limit.
-__device__ void lz_decide_step(LzState* st, int j, cudaGraphConditionalHandle cond) {
-    const int nk = j + 1;
-    __shared__ double a[LZ_MAXK], b[LZ_MAXK];
-    for (int i = threadIdx.x; i < nk; i += blockDim.x) {
-        a[i] = st->alpha[i];
-        b[i] = st->beta[i];
-    }
-    __syncthreads();
-    if (threadIdx.x >= 32) return;  // warp 0 decides (the callers' next barrier waits for it)
-    __shared__ double2 rows[LZ_MAXK];
-    const double th = warp_eig_exact(nk, a, b, rows, 0, [] {});
+__device__ void lz_decide_step(LzState* st, LzDecision& d, int j, cudaGraphConditionalHandle cond) {
+    const int nk = j + 1, lane = threadIdx.x & 31;
+    const double th = warp_eig_exact(nk, d.a, d.b, d.rows, 0, [] {});
     double tn = 0;
-    if (st->tol_rel > 0) {
-        for (int i = threadIdx.x; i < nk; i += 32)
-            tn = fmax(tn, fabs(a[i]) + fabs(b[i]) + (i > 0 ? fabs(b[i - 1]) : 0.0));
+    if (d.tol_rel > 0) {
+        for (int i = lane; i < nk; i += 32)
+            tn = fmax(tn, fabs(d.a[i]) + fabs(d.b[i]) + (i > 0 ? fabs(d.b[i - 1]) : 0.0));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) tn = fmax(tn, __shfl_xor_sync(0xffffffffu, tn, o));
     }
-    if (threadIdx.x == 0) {
-        const double yl = last_component_rows(nk, rows, a, b, th);
-        const double bj = b[j];
+    if (lane == 0) {
+        const double yl = last_component_rows(nk, d.rows, d.a, d.b, th);
+        const double bj = d.b[j];
         const double resid = bj * yl;
-        double tolEff = fmax(st->tol, 1e-13 * fmax(1.0, fabs(th)));
-        if (st->tol_rel > 0) tolEff = fmax(tolEff, st->tol_rel * tn);
+        double tolEff = fmax(d.tol, 1e-13 * fmax(1.0, fabs(th)));
+        if (d.tol_rel > 0) tolEff = fmax(tolEff, d.tol_rel * tn);
+        int done = 0;
+        const bool conv = (resid <= tolEff) || (bj <= 1e-14 * fmax(1.0, fabs(th)));
+        if (conv) { done = 1; st->converged = 1; }
+        if (d.tol_rel > 0 && j >= 2 && resid > 0.5 * d.resid2) done = 1;
+        if (nk >= d.mmax || nk >= LZ_MAXK - 1) done = 1;  // basis exhausted for this restart
+        if (done) st->done = 1;
+        if (cond) cudaGraphSetConditional(cond, done ? 0u : 1u);
         st->theta = th;
         st->resid = resid;
         st->nb = nk;
         st->rhist[j] = resid;
-        int done = 0;
-        const bool conv = (resid <= tolEff) || (bj <= 1e-14 * fmax(1.0, fabs(th)));
-        if (conv) { done = 1; st->converged = 1; }
-        if (st->tol_rel > 0 && j >= 2 && resid > 0.5 * st->rhist[j - 2]) done = 1;
-        if (nk >= st->mmax || nk >= LZ_MAXK - 1) done = 1;  // basis exhausted for this restart
-        if (done) st->done = 1;
-        if (cond) cudaGraphSetConditional(cond, done ? 0u : 1u);
     }
 }
 
@@ -352,7 +352,7 @@ __global__ void lz_scale_kernel(const double* x, double* v0, long long N, const 
 // sums that end them.  All sums of a pass stay in registers (LZ_CHUNK at a time) and are reduced together, the
 // update reads the basis once from L2 (a second time from L1), and the step's tridiagonal
 // problem has a block of its own beside the vector's.  N = 262144, 40 vectors (20 on average): dots, update and
-// next 9.0, 14.6 and 14.7 us where they took 16.1, 23.1 and 30.3.
+// next 8.8, 14.6 and 13.2 us where they took 16.1, 23.1 and 30.3.
 
 // Partials of h_k = V_k . w, k = 0..j, into partA.
 __global__ void __launch_bounds__(LZ_THREADS) lz_dots_kernel(const double* __restrict__ V,
@@ -384,8 +384,10 @@ __global__ void __launch_bounds__(LZ_THREADS) lz_update_kernel(const double* __r
     __shared__ double hs[LZ_MAXK];
     const int nk = st->j + 1;
     sum_partials(partA, gridDim.x, nk, hs);
-    if (blockIdx.x == 0)
+    if (blockIdx.x == 0) {
         for (int k = threadIdx.x; k < nk; k += blockDim.x) st->h[k] = hs[k];
+        if (threadIdx.x == 0) st->jn = nk - 1;
+    }
     for (int k0 = 0; k0 < nk + 1; k0 += LZ_CHUNK) {
         const int nq = min(LZ_CHUNK, nk + 1 - k0);
         double v[LZ_CHUNK] = {0};
@@ -406,11 +408,11 @@ __global__ void __launch_bounds__(LZ_THREADS) lz_update_kernel(const double* __r
 // h2 and |w'|^2 from partB, beta_j; V_{j+1} = (w' - V h2) / beta_j, also into
 // the matvec input xcur.  Block 0 records alpha_j and beta_j, solves the
 // tridiagonal problem of step j and decides whether the restart ends (and,
-// inside a graph loop, whether the loop runs another step); the others have the
-// vector.  The last block to finish advances the step index.  Blocks
+// inside a graph loop, whether the loop runs another step), and advances the step
+// index (this kernel reads the copy that the update made, so no block needs to
+// wait for another); the others have the vector.  Blocks
 // that start after block 0 has ended the restart return at once; the step's
-// vector is then unused (and the half-counted ticket is cleared by the next
-// reset).
+// vector is then unused.
 __global__ void __launch_bounds__(LZ_THREADS) lz_next_kernel(double* __restrict__ V, const double* __restrict__ w,
                                                              long long N, const double* partB, LzState* st,
                                                              double* __restrict__ xcur, VecSplit sp,
@@ -421,10 +423,24 @@ __global__ void __launch_bounds__(LZ_THREADS) lz_next_kernel(double* __restrict_
         return;
     }
     __shared__ double h2s[LZ_MAXK];
-    __shared__ bool last;
-    const int j = st->j;
+    __shared__ LzDecision dec;
+    const int j = st->jn;
     const int nk = j + 1;
     const int nv = gridDim.x - 1;  // vector blocks
+    if (blockIdx.x == 0) {
+        for (int k = threadIdx.x; k < j; k += blockDim.x) {
+            dec.a[k] = st->alpha[k];
+            dec.b[k] = st->beta[k];
+        }
+        if (threadIdx.x == blockDim.x - 1) {
+            dec.tol = st->tol;
+            dec.tol_rel = st->tol_rel;
+            dec.h = st->h[j];
+            dec.resid2 = j >= 2 ? st->rhist[j - 2] : 0.0;
+            dec.mmax = st->mmax;
+            dec.matvecs = st->matvecs;
+        }
+    }
     sum_partials(partB, nv, nk + 1, h2s);
     double ss = 0;
     for (int k = 0; k < nk; ++k) ss = fma(h2s[k], h2s[k], ss);
@@ -441,27 +457,21 @@ __global__ void __launch_bounds__(LZ_THREADS) lz_next_kernel(double* __restrict_
             xcur[i] = wi;
             if (sp.out) split_bf16((float)wi, sp.ns, sp.out, sp.stride, i);
         }
-    } else {
-        for (int k = threadIdx.x; k < nk; k += blockDim.x) st->h2[k] = h2s[k];
+    } else if (threadIdx.x < 32) {
         if (threadIdx.x == 0) {
-            st->alpha[j] = st->h[j] + h2s[j];
-            st->beta[j] = beta;
-            st->matvecs += 1;
-            st->jn = j + 1;
+            dec.a[j] = dec.h + h2s[j];
+            dec.b[j] = beta;
         }
-        __syncthreads();
-        lz_decide_step(st, j, cond);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        unsigned int prev = atomicAdd(&st->counter, 1u);
-        last = (prev == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        st->j = j + 1;
-        st->counter = 0;
+        __syncwarp();
+        lz_decide_step(st, dec, j, cond);
+        if (threadIdx.x == 0) st->j = j + 1;
+    } else if (threadIdx.x < 64) {
+        for (int k = threadIdx.x - 32; k < nk; k += 32) st->h2[k] = h2s[k];
+        if (threadIdx.x == 32) {
+            st->alpha[j] = dec.h + h2s[j];
+            st->beta[j] = beta;
+            st->matvecs = dec.matvecs + 1;
+        }
     }
 }
 

@@ -15,8 +15,8 @@ struct LzState {
     int matvecs;           // Heff applications so far
     int converged;         // residual criterion met
     unsigned int counter;  // last-block reduction ticket
-    int j;                 // step of the current restart (read by dots / update)
-    int jn;                // index of the vector lz_next builds (set by update)
+    int j;                 // step of the current restart (read by dots and update, advanced by next)
+    int jn;                // the same for next (set by update)
     int mmax;              // basis limit of the current restart
     double tol, theta, theta2, resid, xnorm;
     double tol_rel;        // additional residual target relative to |T| (split-precision operators)
