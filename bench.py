@@ -564,8 +564,8 @@ def run_ours(args, rank, world, local_rank):
     ph = main_run["phases"] or {}
     roofline_qr = {"bound": "fp64 (latency)", "achieved": round(F_qr / t_qr / 1e12, 4), "peak": round(p64, 2),
                    "unit": "TFLOP/s", "frac": round(F_qr / t_qr / 1e12 / p64, 5), "traffic": None,
-                   "kernel": f"gauge QR of a {d_ * args.D} x {args.D} site matrix (tn_qr: persistent Householder "
-                             "kernel + Q read-out)" if d_ * args.D <= 512 else
+                   "kernel": f"gauge QR of a {d_ * args.D} x {args.D} site matrix (tn_qr: cluster Householder "
+                             "kernel; the sweep's own gauge moves keep the persistent kernel's order)" if d_ * args.D <= 512 else
                              f"gauge QR of a {d_ * args.D} x {args.D} site matrix (tn_qr)",
                    "per_launch_us": round(t_qr * 1e6, 1), "flop_per_launch": F_qr,
                    "share_of_step": ph.get("gauge_share"),
