@@ -22,12 +22,17 @@
 // partial Z summed and multiplied by T^T (or T) a slice of columns per CTA, then
 // C -= V Z2 by DMMA; V and T come in one bulk copy.
 //
-// What bounds it: the chain of k column steps, ~0.75 us each (u by shuffles 0.1,
+// What bounds it: the chain of k column steps, ~0.85 us each (u by shuffles 0.1,
 // dots and butterfly 0.15, exchange 0.2, sums of 4C warps 0.12, two reciprocal square
-// roots 0.13, update 0.06), and per panel ~9 us of publication (3) and application (6: DMMA
-// at the FP64 rate on C SMs).  512 x 256 276 us against 460 for the persistent
-// two-level kernel of qr.cu (one CTA per panel, one task queue), 64 x 64 66 (86),
-// 1024 x 512 741 (1819), 1536 x 512 1105 (2470), 512 x 1536 566 (1787).
+// roots 0.13, update 0.06, the divisions of tau and 1 / (alpha - beta) 0.1), and per panel ~9 us of publication (3) and application (6: DMMA
+// at the FP64 rate on C SMs).  512 x 256 305 us against 460 for the persistent
+// two-level kernel of qr.cu (one CTA per panel, one task queue), 64 x 64 71 (87),
+// 1024 x 512 802 (1822), 1536 x 512 1180 (2471), 512 x 1536 624 (1791).
+//
+// Rounding: 512 x 256, graded over five decades, |Q^T Q - I|_F 9.0e-15 and |QR - A| / |A| 5.0e-16 in extended
+// precision (persistent kernel 1.3e-14, 6.1e-16).  Without the divisions (tau and 1 / (alpha - beta)
+// from the chain's kap: 282 us) and with the products accumulated onto C the factors
+// were a quarter further from the exact ones.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -239,23 +244,26 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
         {
             constexpr int JN = 16 / W;
             const int rt = w & 3, j0 = (w >> 2) * JN;
-            double acc[JN][2];
+            double acc[JN][2], ac2[JN][2];  // two halves of the rows' chain: less rounding, more in flight
 #pragma unroll
-            for (int j = 0; j < JN; ++j) acc[j][0] = acc[j][1] = 0.0;
+            for (int j = 0; j < JN; ++j) acc[j][0] = acc[j][1] = ac2[j][0] = ac2[j][1] = 0.0;
             const double* vp = Vs + (8 * rt + gid) * ldr + tig;
             const double* cp = Cs + (8 * j0 + gid) * ldr + tig;
-#pragma unroll 4
-            for (int r = lr0; r < L::rows; r += 4) {
-                const double av = vp[r];
+#pragma unroll 2
+            for (int r = lr0; r < L::rows; r += 8) {
+                const double av = vp[r], aw = vp[r + 4];
 #pragma unroll
                 for (int j = 0; j < JN; ++j) dmma(acc[j], av, cp[8 * j * ldr + r]);
+#pragma unroll
+                for (int j = 0; j < JN; ++j) dmma(ac2[j], aw, cp[8 * j * ldr + r + 4]);
             }
             // to the CTA that owns the columns: [source][row][column in slice]
 #pragma unroll
             for (int j = 0; j < JN; ++j) {
                 const int col = 8 * (j0 + j) + 2 * tig, dst = col / SC;
                 const int at = rank * 32 * SC + (8 * rt + gid) * SC + col % SC;
-                qc_st_async(qc_remote(qc_smem(zp + at), dst), acc[j][0], acc[j][1], qc_remote(qc_smem(&zbar), dst));
+                qc_st_async(qc_remote(qc_smem(zp + at), dst), acc[j][0] + ac2[j][0], acc[j][1] + ac2[j][1],
+                            qc_remote(qc_smem(&zbar), dst));
             }
         }
         if (!qc_mbar_wait(&zbar, ph, a.err)) fail();
@@ -288,22 +296,20 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
             for (int ks = 0; ks < 8; ++ks) bz[j][ks] = z2[(4 * ks + tig) * QC_ZLD + 8 * j + gid];
 #pragma unroll 2
         for (int r = lr0 + 8 * w; r < L::rows; r += 8 * W) {
+            // the product by itself, then one addition to C: one rounding of C's size instead of eight
             double av[8], acc[4][2];
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) av[ks] = Vs[(4 * ks + tig) * ldr + r + gid];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc[j][0] = Cs[(8 * j + 2 * tig) * ldr + r + gid];
-                acc[j][1] = Cs[(8 * j + 2 * tig + 1) * ldr + r + gid];
-            }
+            for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = 0.0;
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) dmma(acc[j], av[ks], bz[j][ks]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                Cs[(8 * j + 2 * tig) * ldr + r + gid] = acc[j][0];
-                Cs[(8 * j + 2 * tig + 1) * ldr + r + gid] = acc[j][1];
+                Cs[(8 * j + 2 * tig) * ldr + r + gid] += acc[j][0];
+                Cs[(8 * j + 2 * tig + 1) * ldr + r + gid] += acc[j][1];
             }
         }
         return true;
@@ -438,8 +444,8 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
                     }
                     // w_j = u_j + (alpha - beta) e_j, beta = -sign(alpha) |(alpha, u)|, H = I - kap w w^T with
                     // kap = 1 / (|beta| |alpha - beta|): two reciprocal square roots, each with one Newton
-                    // correction.  dlarfg's tau and 1 / (alpha - beta) are kap (alpha - beta)^2 and kap |beta|.
-                    double kap = 0, beta = alpha, amb = 0, scal = 1;
+                    // correction, on the chain; dlarfg's tau and 1 / (alpha - beta) by division beside it.
+                    double kap = 0, beta = alpha, amb = 0;
                     if (xn2 > 0.0) {
                         const double n2 = fma(alpha, alpha, xn2), rn = rsqrt(n2);
                         double nrm = n2 * rn;
@@ -449,7 +455,6 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
                         kap = fma(kap, fma(-den, kap, 1.0), kap);
                         beta = alpha >= 0 ? -nrm : nrm;
                         amb = alpha - beta;
-                        scal = alpha >= 0 ? kap * nrm : -kap * nrm;
                     }
 #pragma unroll
                     for (int c = 0; c < 4; ++c) cu[c] = gid + 8 * c > j ? kap * fma(amb, ca[c], cu[c]) : 0.0;
@@ -459,8 +464,10 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
                     for (int r = 0; r < PR; ++r)
 #pragma unroll
                         for (int c = 0; c < 4; ++c) p[r][c] = fma(-cu[c], u[r], p[r][c]);
+                    const bool trivial = !(amb != 0.0);
+                    const double scal = trivial ? 1.0 : 1.0 / amb;
                     gl = myscal * fma(scal, S, ar);  // v_lc^T v_j (lc < j)
-                    tl = kap * amb * amb;
+                    tl = trivial ? 0.0 : -amb / beta;
                     if (lc == j) {
                         myscal = scal;
                         if (w == 0) {
@@ -614,7 +621,7 @@ int qr_cluster(Ctx& c, int m, int n, const double* A, long long ars, long long a
     a.R = R; a.rrs = rrs; a.rcs = rcs;
     bool served = false;
     int st = TN_OK;
-    // Rows per CTA: as few as keep the exchange small.  Measured with half the CTAs a cluster: 128 x 128 128 us
+    // Rows per CTA: as few as keep the exchange small.  Measured (without the divisions) with half the CTAs a cluster: 128 x 128 128 us
     // (122 here), 256 x 256 255 (243); with twice as many (RL = 2): 512 x 256 309 (276), 512 x 1536 679 (566);
     // with 8 warps a CTA instead of 8 CTAs: 1024 x 512 947 (741) -- above 512 rows that is left for when the
     // clusters of 8 do not all fit (1536 x 512: 15 of 16).
