@@ -69,7 +69,7 @@ void DevBuf::release() {
     part = false;
 }
 
-int slab_reserve(const std::vector<DevBuf*>& v, const std::vector<size_t>& need, DevBuf& slab) {
+int slab_reserve(Ctx& c, const std::vector<DevBuf*>& v, const std::vector<size_t>& need, DevBuf& slab) {
     bool enough = true;
     size_t total = 0;
     std::vector<size_t> size(v.size());
@@ -79,15 +79,19 @@ int slab_reserve(const std::vector<DevBuf*>& v, const std::vector<size_t>& need,
         total += (size[i] + 255) / 256 * 256;
     }
     if (enough) return TN_OK;
-    TN_CUDA_CHECK(cudaDeviceSynchronize());  // whatever still uses the buffers, on any stream
+    // Whatever uses the buffers: this context's streams, and the legacy stream's copies and clears.  Not the device:
+    // other contexts' streams have nothing to do with them and may be capturing, which a device-wide wait ends with
+    // an error on both sides.
+    for (cudaStream_t s : {c.stream, c.own_stream, c.aux, c.aux2, cudaStreamLegacy})
+        if (s) TN_CUDA_CHECK(cudaStreamSynchronize(s));
     DevBuf fresh;
     TN_CHECK(fresh.ensure(total));
     char* at = fresh.as<char>();
     for (size_t i = 0; i < v.size(); ++i) {
-        if (v[i]->p) TN_CUDA_CHECK(cudaMemcpy(at, v[i]->p, v[i]->bytes, cudaMemcpyDeviceToDevice));
+        if (v[i]->p) TN_CUDA_CHECK(cudaMemcpyAsync(at, v[i]->p, v[i]->bytes, cudaMemcpyDeviceToDevice, c.stream));
         at += (size[i] + 255) / 256 * 256;
     }
-    TN_CUDA_CHECK(cudaDeviceSynchronize());
+    TN_CUDA_CHECK(cudaStreamSynchronize(c.stream));
     at = fresh.as<char>();
     for (size_t i = 0; i < v.size(); ++i) {
         v[i]->release();

@@ -356,7 +356,7 @@ int MPSState::init(Hamiltonian* h, int D) {
 
 int MPSState::ensure_capacity(int D) {
     const size_t site = sizeof(double) * (size_t)d * D * D;
-    return slab_reserve(std::vector<DevBuf*>(A.begin() + 1, A.begin() + L + 1), std::vector<size_t>(L, site), siteSlab);
+    return slab_reserve(*ctx, std::vector<DevBuf*>(A.begin() + 1, A.begin() + L + 1), std::vector<size_t>(L, site), siteSlab);
 }
 
 // The environments that a sweep at the current bonds fills, in one allocation.
@@ -370,7 +370,7 @@ int MPSState::reserve_environments() {
         v.push_back(Renv[ia]);
         need.push_back(ia > 1 ? sizeof(double) * (size_t)op.Dw1 * D1[ia] * D1[ia] : 0);
     }
-    return slab_reserve(v, need, envSlab);
+    return slab_reserve(*ctx, v, need, envSlab);
 }
 
 // The triangular factors that a half-sweep in direction dir leaves, in one allocation.
@@ -381,7 +381,7 @@ int MPSState::reserve_factors(int dir) {
         v.push_back(bondR[dir][b]);
         need.push_back(sizeof(double) * (size_t)D2[b] * D2[b]);
     }
-    return v.empty() ? TN_OK : slab_reserve(v, need, factorSlab[dir]);
+    return v.empty() ? TN_OK : slab_reserve(*ctx, v, need, factorSlab[dir]);
 }
 
 // MPSSite::InitializeWith(Random) (MPSSite.C:119-127) with mt19937_64(seed),

@@ -102,9 +102,12 @@ struct DevBuf {
     DevBuf& operator=(const DevBuf&) = delete;
 };
 
+struct Ctx;
+
 // Every buffer of v gets its need[] bytes (where it has less) as a part of one
 // allocation, which replaces the slab they were parts of before; contents are kept.
-int slab_reserve(const std::vector<DevBuf*>& v, const std::vector<size_t>& need, DevBuf& slab);
+// Waits for the streams of c, which uses the buffers.
+int slab_reserve(Ctx& c, const std::vector<DevBuf*>& v, const std::vector<size_t>& need, DevBuf& slab);
 
 // Pinned host buffer for small device->host reads.
 struct HostBuf {
