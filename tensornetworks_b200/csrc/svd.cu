@@ -30,6 +30,15 @@ __device__ __forceinline__ double wsum(double v) {
     return v;
 }
 
+// The power of two that the rows to be orthogonalised are multiplied by, from their largest entry: 1 between
+// 2^-400 and 2^400 (and for zero, an infinity or NaN), else what brings it near 1.  Squared norms and dots then
+// neither underflow nor overflow for the columns that count.
+__device__ __forceinline__ double jc_matrix_scale(double amax) {
+    const int e = (__double2hiint(amax) >> 20) & 0x7ff;
+    if (amax == 0.0 || e == 0x7ff || (e >= 0x3ff - 400 && e <= 0x3ff + 400)) return 1.0;
+    return __hiloint2double(max(1, 0x7fe - e) << 20, 0);
+}
+
 __device__ __forceinline__ int rr_pos(int q, int r, int ne) {
     return q == 0 ? 0 : ((q - 1 + r) % (ne - 1)) + 1;
 }
@@ -150,8 +159,15 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_svd_kernel(const SvdJob* _
     bool in_smem = need * sizeof(double) <= smem_cap;
     double* A = in_smem ? tail : jb.W;
     double* V = vectors ? (in_smem ? tail + (size_t)m * n : jb.V) : nullptr;
-    if (in_smem)
-        for (size_t e = tid; e < (size_t)m * n; e += blockDim.x) A[e] = jb.W[e];
+    double amax = 0.0;
+    for (size_t e = tid; e < (size_t)m * n; e += blockDim.x) amax = fmax(amax, fabs(jb.W[e]));
+    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) red[wid] = amax;
+    __syncthreads();
+    for (int w = 0; w < nw; ++w) amax = fmax(amax, red[w]);
+    const double scale = jc_matrix_scale(amax);
+    if (in_smem || scale != 1.0)
+        for (size_t e = tid; e < (size_t)m * n; e += blockDim.x) A[e] = scale * jb.W[e];
     if (vectors)
         for (size_t e = tid; e < (size_t)n * n; e += blockDim.x) V[e] = ((e % n) == (e / n)) ? 1.0 : 0.0;
     __syncthreads();
@@ -217,26 +233,26 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_svd_kernel(const SvdJob* _
     __syncthreads();
     // descending rank, ties broken by column index
     for (int j = tid; j < n; j += blockDim.x) {
-        double sj = norms[j];
+        const double sj = norms[j];
         int rk = 0;
         for (int i = 0; i < n; ++i) {
             double si = norms[i];
             rk += (si > sj) || (si == sj && i < j);
         }
         rank[j] = rk;
-        jb.s[rk] = sj;
+        jb.s[rk] = sj / scale;
     }
     __syncthreads();
     double smax = 0;
     for (int j = 0; j < n; ++j) smax = fmax(smax, norms[j]);
-    const double cut = smax * 1e-13 * fmax(1.0, (double)m);
+    const double cut = smax * 1e-13 * fmax(1.0, (double)m) / scale;
     if (vectors) {
         for (int j = wid; j < n; j += nw) {
             const int rk = rank[j];
             const double sj = norms[j];
             const double* cj = A + (size_t)j * m;
             double* uo = jb.U + (size_t)rk * jb.ldu;
-            const bool good = sj > cut && sj > 0.0;
+            const bool good = sj / scale > cut && sj / scale > 0.0;
             for (int i = lane; i < m; i += 32) uo[i] = good ? cj[i] / sj : 0.0;
             const double* vj = V + (size_t)j * n;
             for (int i = lane; i < n; i += 32) jb.Vt[(size_t)i * jb.ldvt + rk] = vj[i];
@@ -423,6 +439,7 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
     const bool on = gw < NW;
     __shared__ int flags[3];                 // rank 0's are used: "something rotated", by sweep modulo 3
     __shared__ double red[32];
+    __shared__ double wmax[8];               // largest entry of each warp's columns
     __shared__ int at[32];
     constexpr int SLOT = jc_slot<E>();
     double* inbox = smem;                    // [parity][warp][top, bottom][SLOT]
@@ -497,7 +514,30 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
         na = v.x;
         nb = v.y;
     };
+    // the largest entry of this warp's columns; every warp gets the whole matrix's
+    double amax = 0.0;
+#pragma unroll
+    for (int q = 0; q < E; ++q)
+        if (q < ET) amax = fmax(amax, fmax(fmax(fabs(x0[q]), fabs(x1[q])), fmax(fabs(y0[q]), fabs(y1[q]))));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) wmax[wid] = amax;
     cl.sync();  // every CTA of the cluster runs before the first remote write; flags are zero
+    amax = 0.0;
+    for (int w = lane; w < ncta * nw; w += 32) amax = fmax(amax, cl.map_shared_rank(wmax, w / nw)[w % nw]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const double scale = jc_matrix_scale(amax);
+    if (scale != 1.0) {
+#pragma unroll
+        for (int q = 0; q < E; ++q)
+            if (q < ET) {
+                x0[q] *= scale;
+                x1[q] *= scale;
+                y0[q] *= scale;
+                y1[q] *= scale;
+            }
+    }
 
     const double tol = 1e-15 * fmax(1.0, sqrt((double)m) / 4.0), tol2 = tol * tol;
     int sweep = 0;
@@ -569,18 +609,18 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
             k += (si > sj) || (si == sj && i < j);
         }
         rk[j] = sj < 0 ? -1 : k;
-        if (rank == 0 && !(sj < 0)) jb.s[min(k, n - 1)] = sj;
+        if (rank == 0 && !(sj < 0)) jb.s[min(k, n - 1)] = sj / scale;
     }
     __syncthreads();
     if (vectors) {
         double smax = 0;
         for (int j = 0; j < np; ++j) smax = fmax(smax, sig[j]);
-        const double cut = smax * 1e-13 * fmax(1.0, (double)m);
+        const double cut = smax * 1e-13 * fmax(1.0, (double)m) / scale;
         auto emit = [&](const double(&v)[E], int j) {
             const int k = rk[j];
             if (k < 0) return;
-            const double sj = sig[j];
-            const bool good = sj > cut && sj > 0.0;
+            const double sj = sig[j], so = sj / scale;
+            const bool good = so > cut && so > 0.0;  // as complete_u asks
             const int kc = min(k, n - 1);
 #pragma unroll
             for (int q = 0; q < E; ++q) {

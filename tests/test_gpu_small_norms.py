@@ -1,0 +1,64 @@
+"""SVD at the ends of the floating-point range, where squares of the entries underflow or overflow: whole matrices of
+tiny and huge entries, and harmless tiny columns beside ordinary ones (with zero columns after them).  Tolerances:
+2 sqrt(m n) 1e-13 of the largest singular value, as for the Jacobi kernels elsewhere."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def tiny_columns(m, n):
+    """Ordinary columns, one of norm 1e-157, a smaller one, and zero ones after it."""
+    A = np.random.default_rng(m + 100 * n).standard_normal((m, n))
+    A[:, 5] *= 1e-157 / np.linalg.norm(A[:, 5])
+    A[:, 6] = 0.0
+    A[:, 8] = 0.0
+    A[:, 9] *= 1e-160
+    return A
+
+
+def check_svd(T, B):
+    U, s, Vt = T.CudaSVDSolver().SolveAll(B)
+    top = np.abs(B).max()  # LAPACK and the products below on a matrix of ordinary size
+    e = 2.0 ** np.round(np.log2(top)) if top > 0 else 1.0
+    s0 = np.linalg.svd(B / e, compute_uv=False)
+    k = len(s0)
+    tol = 2 * np.sqrt(B.shape[0] * B.shape[1]) * 1e-13
+    assert np.abs(s / e - s0).max() <= tol * s0[0]
+    assert np.abs(U.T @ U - np.eye(k)).max() < tol
+    assert np.abs(Vt @ Vt.T - np.eye(k)).max() < tol
+    assert np.abs((U * (s / e)) @ Vt - B / e).max() <= tol * s0[0]
+
+
+@pytest.mark.parametrize("scale", [1e-156, 1e-170, 1e-290, 1e-121, 1e121, 1e156, 1e290])
+@pytest.mark.parametrize("m,n", [(1, 1), (5, 4), (12, 8), (33, 24)])
+def test_svd_of_a_scaled_matrix(m, n, scale):
+    import tensornetworks_b200 as T
+    A = np.random.default_rng(m).standard_normal((m, n)) * 10.0 ** (-3.0 * np.arange(n) / n)
+    check_svd(T, A * scale)
+    check_svd(T, A.T * scale)
+
+
+@pytest.mark.parametrize("m,n", [(20, 16), (30, 24)])
+def test_svd_with_tiny_columns(m, n):
+    import tensornetworks_b200 as T
+    check_svd(T, tiny_columns(m, n))
+    check_svd(T, tiny_columns(m, n).T)
+
+
+@pytest.mark.parametrize("scale", [1e-156, 1e-290, 1e156])
+@pytest.mark.parametrize("m,n", [(7, 6), (64, 20), (600, 20)])
+def test_singular_values_alone(m, n, scale):
+    import torch
+    import tensornetworks_b200 as T
+    ctx = T.default_context()
+    A = np.random.default_rng(n).standard_normal((m, n))
+    dA = torch.from_numpy(np.ascontiguousarray((A * scale).T)).cuda()
+    s = torch.empty(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    T._capi.check(ctx._lib.tn_svd_values(ctx.handle, m, n, C.c_void_p(dA.data_ptr()), m, C.c_void_p(s.data_ptr())),
+                  "tn_svd_values")
+    s0 = np.linalg.svd(A, compute_uv=False)
+    assert np.abs(s.cpu().numpy() / scale - s0).max() <= 2 * np.sqrt(m * n) * 1e-13 * s0[0]
