@@ -315,7 +315,9 @@ __device__ __forceinline__ bool jc_rotate2(double (&x0)[E], double (&y0)[E], dou
     const bool real = al >= 0.0 && be >= 0.0;  // a padding column (norm -1) is never rotated
     const double sc = jc_scale(fmax(al, be));
     const double d = (be - al) * sc;
-    const double thr = tol2 * ((al * sc) * (be * sc));
+    // at least 2^-800: a smaller rotation changes nothing, and where the norms that followed the rotations have come
+    // out zero (columns that were equal), the squares below would be denormal and the rotation no longer orthogonal
+    const double thr = fmax(tol2 * ((al * sc) * (be * sc)), 0x1p-800);
     double a0 = 0, b0 = 0, a1 = 0, b1 = 0;
 #pragma unroll
     for (int q = 0; q < E; q += 2) {

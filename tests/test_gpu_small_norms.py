@@ -1,6 +1,7 @@
 """SVD at the ends of the floating-point range, where squares of the entries underflow or overflow: whole matrices of
-tiny and huge entries, and harmless tiny columns beside ordinary ones (with zero columns after them).  Tolerances:
-2 sqrt(m n) 1e-13 of the largest singular value, as for the Jacobi kernels elsewhere."""
+tiny and huge entries, harmless tiny columns beside ordinary ones (with zero columns after them), and equal columns,
+whose remainders shrink by a rounding error at a time.  Tolerances: 2 sqrt(m n) 1e-13 of the largest singular value,
+as for the Jacobi kernels elsewhere."""
 import ctypes as C
 
 import numpy as np
@@ -17,6 +18,12 @@ def tiny_columns(m, n):
     A[:, 8] = 0.0
     A[:, 9] *= 1e-160
     return A
+
+
+def equal_columns(m, n, seed):
+    rng = np.random.default_rng(seed)
+    V = rng.standard_normal((m, 2))
+    return V[:, rng.integers(0, 1 + seed % 2, n)]
 
 
 def check_svd(T, B):
@@ -46,6 +53,13 @@ def test_svd_with_tiny_columns(m, n):
     import tensornetworks_b200 as T
     check_svd(T, tiny_columns(m, n))
     check_svd(T, tiny_columns(m, n).T)
+
+
+@pytest.mark.parametrize("m,n", [(20, 16), (24, 24), (40, 32), (64, 60)])
+def test_svd_of_equal_columns(m, n):
+    import tensornetworks_b200 as T
+    for seed in range(40):
+        check_svd(T, equal_columns(m, n, seed))
 
 
 @pytest.mark.parametrize("scale", [1e-156, 1e-290, 1e156])
