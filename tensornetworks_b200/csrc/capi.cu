@@ -829,8 +829,9 @@ int tn_qr(tn_ctx c, int m, int n, const double* A, int lda, double* Q, int ldq, 
     const int k = std::min(m, n);
     if (ldq < m || ldr < k) return TN_BAD_ARG;
     Ctx& cx = c->c;
-    const int st = qr_cluster(cx, m, n, A, 1, lda, Q, 1, ldq, R, 1, ldr);
-    if (st != QR_UNAVAILABLE) return st ? st : check_device_error_on_stream(cx);
+    int st = qr_cluster(cx, m, n, A, 1, lda, Q, 1, ldq, R, 1, ldr);
+    if (st == TN_OK) st = qr_cluster_status(cx);
+    if (st != QR_UNAVAILABLE) return st;
     DevBuf& W = cx.apiw[0];
     TN_CHECK(W.ensure(sizeof(double) * (size_t)m * n));
     TN_CHECK(copy2d(m, n, A, idx(1), idx(lda), W.as<double>(), idx(1), idx(m), 1.0, cx.stream));
@@ -846,8 +847,9 @@ int tn_lq(tn_ctx c, int m, int n, const double* A, int lda, double* L, int ldl, 
     if (ldl < m || ldq < k) return TN_BAD_ARG;
     Ctx& cx = c->c;
     // A^T = Qt Rt: the cluster kernel reads A and writes Q and L through their strides
-    const int st = qr_cluster(cx, n, m, A, lda, 1, Q, ldq, 1, L, ldl, 1);
-    if (st != QR_UNAVAILABLE) return st ? st : check_device_error_on_stream(cx);
+    int st = qr_cluster(cx, n, m, A, lda, 1, Q, ldq, 1, L, ldl, 1);
+    if (st == TN_OK) st = qr_cluster_status(cx);
+    if (st != QR_UNAVAILABLE) return st;
     DevBuf &W = cx.apiw[0], &Qt = cx.apiw[1], &Rt = cx.apiw[2];
     TN_CHECK(W.ensure(sizeof(double) * (size_t)m * n));
     TN_CHECK(Qt.ensure(sizeof(double) * (size_t)n * k));
@@ -941,10 +943,11 @@ int tn_rq(tn_ctx c, int m, int n, const double* A, int lda, double* R, int ldr, 
     const int k = std::min(m, n);
     if (ldr < m || ldq < k) return TN_BAD_ARG;
     Ctx& cx = c->c;
-    const int st = qr_cluster(cx, n, m, A + (size_t)(n - 1) * lda + (m - 1), -(long long)lda, -1,
+    int st = qr_cluster(cx, n, m, A + (size_t)(n - 1) * lda + (m - 1), -(long long)lda, -1,
                               Q + (size_t)(n - 1) * ldq + (k - 1), -(long long)ldq, -1,
                               R + (size_t)(k - 1) * ldr + (m - 1), -(long long)ldr, -1);
-    if (st != QR_UNAVAILABLE) return st ? st : check_device_error_on_stream(cx);
+    if (st == TN_OK) st = qr_cluster_status(cx);
+    if (st != QR_UNAVAILABLE) return st;
     DevBuf &W = cx.apiw[0], &Qb = cx.apiw[1], &Rb = cx.cqr;
     TN_CHECK(W.ensure(sizeof(double) * (size_t)m * n));
     TN_CHECK(Qb.ensure(sizeof(double) * (size_t)n * k));
@@ -971,10 +974,11 @@ int tn_ql(tn_ctx c, int m, int n, const double* A, int lda, double* Q, int ldq, 
     const int k = std::min(m, n);
     if (ldq < m || ldl < k) return TN_BAD_ARG;
     Ctx& cx = c->c;
-    const int st = qr_cluster(cx, m, n, A + (size_t)(n - 1) * lda + (m - 1), -1, -(long long)lda,
+    int st = qr_cluster(cx, m, n, A + (size_t)(n - 1) * lda + (m - 1), -1, -(long long)lda,
                               Q + (size_t)(k - 1) * ldq + (m - 1), -1, -(long long)ldq,
                               L + (size_t)(n - 1) * ldl + (k - 1), -1, -(long long)ldl);
-    if (st != QR_UNAVAILABLE) return st ? st : check_device_error_on_stream(cx);
+    if (st == TN_OK) st = qr_cluster_status(cx);
+    if (st != QR_UNAVAILABLE) return st;
     DevBuf &W = cx.apiw[0], &Qb = cx.apiw[1], &Rb = cx.cqr;
     TN_CHECK(W.ensure(sizeof(double) * (size_t)m * n));
     TN_CHECK(Qb.ensure(sizeof(double) * (size_t)m * k));

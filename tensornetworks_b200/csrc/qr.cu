@@ -1441,13 +1441,24 @@ int qr_tall(Ctx& c, int m, int n, double* W, double* Qout, int ldq, double* Rout
 
 int ensure_device_error_word(Ctx& c) {
     if (c.derr.p) return TN_OK;
-    TN_CHECK(c.derr.ensure(sizeof(int)));
-    TN_CUDA_CHECK(cudaMemset(c.derr.p, 0, sizeof(int)));
+    TN_CHECK(c.derr.ensure(2 * sizeof(int)));
+    TN_CUDA_CHECK(cudaMemset(c.derr.p, 0, 2 * sizeof(int)));
     return TN_OK;
 }
 
+int qr_cluster_status(Ctx& c) {
+    TN_CHECK(c.derr_host.ensure(2 * sizeof(int)));
+    int* h = reinterpret_cast<int*>(c.derr_host.p);
+    TN_CUDA_CHECK(cudaMemcpyAsync(h, c.derr.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    TN_CUDA_CHECK(cudaStreamSynchronize(c.stream));
+    const bool range = h[1] != 0;
+    if (range) TN_CUDA_CHECK(cudaMemsetAsync(c.derr.as<int>() + 1, 0, sizeof(int), c.stream));
+    if (h[0]) return check_device_error(c);
+    return range ? QR_UNAVAILABLE : TN_OK;
+}
+
 int check_device_error_on_stream(Ctx& c) {
-    TN_CHECK(c.derr_host.ensure(sizeof(int)));
+    TN_CHECK(c.derr_host.ensure(2 * sizeof(int)));
     int* h = reinterpret_cast<int*>(c.derr_host.p);
     TN_CUDA_CHECK(cudaMemcpyAsync(h, c.derr.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     TN_CUDA_CHECK(cudaStreamSynchronize(c.stream));

@@ -17,13 +17,17 @@ int qr_dense(Ctx& c, int m, int n, double* W, double* Qout, int ldq, double* Rou
 constexpr int QR_UNAVAILABLE = -1;
 int qr_cluster(Ctx& c, int m, int n, const double* A, long long ars, long long acs, double* Q, long long qrs,
                long long qcs, double* R, long long rrs, long long rcs, const int* colmap = nullptr);
+// Waits for the stream after qr_cluster: TN_OK, the error of an expired wait, or QR_UNAVAILABLE when a column's
+// remainder had a norm outside 2^-500 .. 2^500 (zero is inside), whose reflector the kernel does not form; the
+// factors are then void, A is as it was.
+int qr_cluster_status(Ctx& c);
 
 // Reads (and clears) the context's sticky device error word, raised when a
 // bounded wait between CTAs expired; waits for the device.
 int check_device_error(Ctx& c);
 // The same by a copy on the context stream, which it then waits for.
 int check_device_error_on_stream(Ctx& c);
-// The error word allocated and zero (before the first kernel that may raise it).
+// The error word, and the QR's range word after it, allocated and zero (before the first kernel that may raise them).
 int ensure_device_error_word(Ctx& c);
 
 // One job of the batched one-sided Jacobi SVD (one cluster or CTA per job).  W is the

@@ -65,7 +65,7 @@ struct QcArgs {
     long long pub_stride;         // doubles per (panel, rank)
     int* ready;                   // [panel][rank]
     int* err;                     // this launch's error word
-    int* derr;                    // the context's
+    int* derr;                    // the context's, and its range word
     long long spin_limit;
 };
 
@@ -510,6 +510,12 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
                          : "memory");
             asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group 0;" ::: "memory");
             qc_st_release(a.ready + q * C + rank, 1);
+        }
+        // den and kap of a column below 2^-511 or above 2^511 are not finite (or have lost their digits): looked for
+        // here, behind the publication; tau = 0 marks the columns without a reflector
+        if (rank == 0 && tid < b && Ts[tid * QC_TLD + tid] != 0.0) {
+            const double nrm = fabs(be_s[tid]);
+            if (!(nrm >= 0x1p-500 && nrm <= 0x1p500)) atomicExch(a.derr + 1, 1);
         }
         ok = bad == 0;
     }

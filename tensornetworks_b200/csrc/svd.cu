@@ -657,18 +657,32 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
 }
 
 // perm: the columns of W (m x n) by descending norm, ties by index (a norm that is not a number counts as infinite).
-__global__ void __launch_bounds__(1024) svd_order_kernel(const double* __restrict__ W, int m, int n, int* __restrict__ perm) {
+// *range is raised for a matrix that the Jacobi kernel scales: its factorisation would not.
+__global__ void __launch_bounds__(1024) svd_order_kernel(const double* __restrict__ W, int m, int n, int* __restrict__ perm,
+                                                         int* range) {
     extern __shared__ double nrm2[];
+    __shared__ double wmax[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double amax = 0.0;
     for (int c = wid; c < n; c += 32) {
         const double* w = W + (size_t)c * m;
-        double s = 0;
+        double s = 0, x = 0;
 #pragma unroll 4
-        for (int i = lane; i < m; i += 32) s = fma(w[i], w[i], s);
+        for (int i = lane; i < m; i += 32) {
+            s = fma(w[i], w[i], s);
+            x = fmax(x, fabs(w[i]));
+        }
         s = wsum(s);
+        for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+        amax = fmax(amax, x);
         if (lane == 0) nrm2[c] = s >= 0 ? s : __longlong_as_double(0x7ff0000000000000LL);
     }
+    if (lane == 0) wmax[wid] = amax;
     __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 32; ++w) amax = fmax(amax, wmax[w]);
+        if (jc_matrix_scale(amax) != 1.0) *range = 1;
+    }
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
         const double sj = nrm2[j];
         int k = 0;
@@ -802,7 +816,8 @@ int svd_batched(Ctx& c, const std::vector<SvdJob>& jobs, bool vectors) {
         double* Q = c.svdpre.as<double>();
         double* X = Q + nq;
         int* perm = reinterpret_cast<int*>(X + nr);
-        svd_order_kernel<<<1, 1024, sizeof(double) * j0.n, c.stream>>>(j0.W, j0.m, j0.n, perm);
+        svd_order_kernel<<<1, 1024, sizeof(double) * j0.n, c.stream>>>(j0.W, j0.m, j0.n, perm,
+                                                                                 c.derr.as<int>() + 1);
         TN_LAUNCH_CHECK();
         const int st = qr_cluster(c, j0.m, j0.n, j0.W, 1, j0.m, vectors ? Q : nullptr, 1, j0.m, X, j0.n, 1, perm);
         if (st != QR_UNAVAILABLE) {
@@ -812,7 +827,13 @@ int svd_batched(Ctx& c, const std::vector<SvdJob>& jobs, bool vectors) {
             p.V = Q;
             p.perm = perm;
             TN_CHECK(run(p));
+            if (served) {
+                const int rc = qr_cluster_status(c);
+                if (rc != QR_UNAVAILABLE) return rc;
+                served = false;  // out of its range: the matrix itself, which only the QR has read
+            }
         }
+        TN_CUDA_CHECK(cudaMemsetAsync(c.derr.as<int>() + 1, 0, sizeof(int), c.stream));
     }
     if (!served) TN_CHECK(run(j0));
     if (!served) {

@@ -207,7 +207,7 @@ struct Ctx {
     DevBuf qrw;            // QR workspace
     DevBuf qaccum;         // QR: forward-accumulated Q (transposed)
     DevBuf qrsync;         // QR: progress words of the persistent kernel
-    DevBuf derr;           // sticky error word of kernels with bounded waits (zero until one expires)
+    DevBuf derr;           // sticky error word of kernels with bounded waits (zero until one expires); range word of the cluster QR
     DevBuf svdw;           // SVD workspace
     DevBuf svdpre;         // SVD of one matrix: Q, R^T and the column order
     DevBuf wterms;         // MPO term lists

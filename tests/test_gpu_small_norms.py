@@ -1,7 +1,8 @@
-"""SVD at the ends of the floating-point range, where squares of the entries underflow or overflow: whole matrices of
-tiny and huge entries, harmless tiny columns beside ordinary ones (with zero columns after them), and equal columns,
-whose remainders shrink by a rounding error at a time.  Tolerances: 2 sqrt(m n) 1e-13 of the largest singular value,
-as for the Jacobi kernels elsewhere."""
+"""SVD at the ends of the floating-point range, where squares of the entries underflow or overflow: whole
+matrices of tiny and huge entries, harmless tiny columns beside ordinary ones (with zero columns after them), and
+equal columns, whose remainders shrink by a rounding error a step.  Sizes next to those from which the SVD factors
+first, one and several warps and CTAs of its kernel, and batches (the values of a chain's bonds).  Tolerances:
+2 sqrt(m n) 1e-13 of the largest singular value, as for the Jacobi kernels elsewhere."""
 import ctypes as C
 
 import numpy as np
@@ -40,7 +41,7 @@ def check_svd(T, B):
 
 
 @pytest.mark.parametrize("scale", [1e-156, 1e-170, 1e-290, 1e-121, 1e121, 1e156, 1e290])
-@pytest.mark.parametrize("m,n", [(1, 1), (5, 4), (12, 8), (33, 24)])
+@pytest.mark.parametrize("m,n", [(1, 1), (5, 4), (12, 8), (33, 24), (25, 25), (40, 33), (150, 128), (300, 200)])
 def test_svd_of_a_scaled_matrix(m, n, scale):
     import tensornetworks_b200 as T
     A = np.random.default_rng(m).standard_normal((m, n)) * 10.0 ** (-3.0 * np.arange(n) / n)
@@ -48,7 +49,7 @@ def test_svd_of_a_scaled_matrix(m, n, scale):
     check_svd(T, A.T * scale)
 
 
-@pytest.mark.parametrize("m,n", [(20, 16), (30, 24)])
+@pytest.mark.parametrize("m,n", [(20, 16), (30, 24), (40, 25), (40, 32), (64, 64), (200, 100)])
 def test_svd_with_tiny_columns(m, n):
     import tensornetworks_b200 as T
     check_svd(T, tiny_columns(m, n))
@@ -63,7 +64,7 @@ def test_svd_of_equal_columns(m, n):
 
 
 @pytest.mark.parametrize("scale", [1e-156, 1e-290, 1e156])
-@pytest.mark.parametrize("m,n", [(7, 6), (64, 20), (600, 20)])
+@pytest.mark.parametrize("m,n", [(7, 6), (64, 40), (600, 20)])
 def test_singular_values_alone(m, n, scale):
     import torch
     import tensornetworks_b200 as T
