@@ -24,6 +24,10 @@ namespace {
 
 constexpr int QR_THREADS = 512;
 
+// A reflector's column whose squared norm is below QR_TINY2 (squares underflow from 2^-1022 on, and 1 / (beta
+// (alpha - beta)) overflows) is multiplied by QR_UP and its sums are formed again.
+constexpr double QR_TINY2 = 0x1p-960, QR_UP = 0x1p600, QR_DOWN = 0x1p-600;
+
 __device__ __forceinline__ double wsum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -71,10 +75,19 @@ __global__ void __launch_bounds__(QR_THREADS) qr_panel_kernel(double* __restrict
         double alpha = pc[jj];
         double t = 0, beta = alpha, scal = 0;
         if (xn2 > 0.0) {
-            double nrm = sqrt(alpha * alpha + xn2);
-            beta = alpha >= 0 ? -nrm : nrm;
-            t = (beta - alpha) / beta;
-            scal = 1.0 / (alpha - beta);
+            double al = alpha, n2 = alpha * alpha + xn2, up = 1.0;
+            if (n2 < QR_TINY2) {
+                up = QR_UP;
+                al *= up;
+                part = 0;
+                for (int i = jj + 1 + tid; i < mp; i += blockDim.x) part = fma(up * pc[i], up * pc[i], part);
+                n2 = al * al + block_sum(part, red);
+            }
+            double nrm = sqrt(n2);
+            beta = al >= 0 ? -nrm : nrm;
+            t = (beta - al) / beta;
+            scal = up / (al - beta);
+            beta /= up;
         }
         __syncthreads();
         if (tid == 0) { tau[jj] = t; pc[jj] = beta; }
@@ -281,36 +294,46 @@ __device__ __forceinline__ void panel_wc(double* __restrict__ W, int ldw, int m,
         for (int q = 0; q < RPL; ++q) u[q] = sm.ub[par][lane + 32 * q];
         const double alpha = sm.alph[par];
         double x[CPW + 1];
+        double al = alpha, n2;
+        bool tiny = false;
+#pragma unroll 1
+        for (;;) {  // u . p_c of the warp's columns and u . u; again with u scaled for a tiny column, in every warp alike
 #pragma unroll
-        for (int ci = 0; ci < CPW; ++ci) {
-            double a0 = 0, a1 = 0;
+            for (int ci = 0; ci < CPW; ++ci) {
+                double a0 = 0, a1 = 0;
 #pragma unroll
-            for (int q = 0; q < RPL; q += 2) {
-                a0 = fma(u[q], p[ci][q], a0);
-                if (q + 1 < RPL) a1 = fma(u[q + 1], p[ci][q + 1], a1);
+                for (int q = 0; q < RPL; q += 2) {
+                    a0 = fma(u[q], p[ci][q], a0);
+                    if (q + 1 < RPL) a1 = fma(u[q + 1], p[ci][q + 1], a1);
+                }
+                x[ci] = a0 + a1;
             }
-            x[ci] = a0 + a1;
-        }
-        {
-            double a0 = 0, a1 = 0;
+            {
+                double a0 = 0, a1 = 0;
 #pragma unroll
-            for (int q = 0; q < RPL; q += 2) {
-                a0 = fma(u[q], u[q], a0);
-                if (q + 1 < RPL) a1 = fma(u[q + 1], u[q + 1], a1);
+                for (int q = 0; q < RPL; q += 2) {
+                    a0 = fma(u[q], u[q], a0);
+                    if (q + 1 < RPL) a1 = fma(u[q + 1], u[q + 1], a1);
+                }
+                x[CPW] = a0 + a1;
             }
-            x[CPW] = a0 + a1;
-        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+            for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-            for (int v = 0; v <= CPW; ++v) x[v] += __shfl_xor_sync(0xffffffffu, x[v], o);
+                for (int v = 0; v <= CPW; ++v) x[v] += __shfl_xor_sync(0xffffffffu, x[v], o);
+            }
+            n2 = al * al + x[CPW];
+            if (n2 >= QR_TINY2 || tiny || !(x[CPW] > 0.0)) break;
+            tiny = true;
+            al *= QR_UP;
+#pragma unroll
+            for (int q = 0; q < RPL; ++q) u[q] *= QR_UP;
         }
-        const double xn2 = x[CPW];
         double tau = 0, beta = alpha, scal = 1;
-        if (xn2 > 0.0) {
-            const double nrm = sqrt(alpha * alpha + xn2);
-            beta = alpha >= 0 ? -nrm : nrm;
-            const double amb = alpha - beta;
+        if (x[CPW] > 0.0) {
+            const double nrm = sqrt(n2);
+            beta = al >= 0 ? -nrm : nrm;
+            const double amb = al - beta;
             const double rinv = 1.0 / (beta * amb);  // tau = -amb / beta, scal = 1 / amb
             tau = -amb * amb * rinv;
             scal = beta * rinv;
@@ -333,8 +356,8 @@ __device__ __forceinline__ void panel_wc(double* __restrict__ W, int ldw, int m,
         }
         if (w == j / CPW && lane == 0) {
             sm.taus[j] = tau;
-            sm.scals[j] = scal;
-            sm.betas[j] = beta;
+            sm.scals[j] = tiny ? scal * QR_UP : scal;
+            sm.betas[j] = tiny ? beta * QR_DOWN : beta;
         }
         if (j + 1 < b && w == (j + 1) / CPW) publish(j + 1, par ^ 1);
         __syncthreads();
@@ -1155,31 +1178,45 @@ __global__ void __launch_bounds__(PWC_THREADS, 1) qr_panel_tall_kernel(double* _
 #pragma unroll 1
     for (int j = 0; j < b; ++j) {
         const int par = j & 1;
-        const double* u = sm.ub[par];
+        double* u = sm.ub[par];
         const double alpha = sm.alph[par];
-        double x0 = 0, x1 = 0, n0 = 0, n1 = 0;
+        double x, xn2;
+        double al = alpha, n2;
+        bool tiny = false;
+#pragma unroll 1
+        for (;;) {  // u . p of the warp's column and u . u; again with u scaled for a tiny column, in every warp alike
+            double x0 = 0, x1 = 0, n0 = 0, n1 = 0;
 #pragma unroll
-        for (int q = 0; q < RPL; q += 2) {
-            const double ua = u[lane + 32 * q];
-            x0 = fma(ua, p[q], x0);
-            n0 = fma(ua, ua, n0);
-            if (q + 1 < RPL) {
-                const double ub = u[lane + 32 * (q + 1)];
-                x1 = fma(ub, p[q + 1], x1);
-                n1 = fma(ub, ub, n1);
+            for (int q = 0; q < RPL; q += 2) {
+                const double ua = u[lane + 32 * q];
+                x0 = fma(ua, p[q], x0);
+                n0 = fma(ua, ua, n0);
+                if (q + 1 < RPL) {
+                    const double ub = u[lane + 32 * (q + 1)];
+                    x1 = fma(ub, p[q + 1], x1);
+                    n1 = fma(ub, ub, n1);
+                }
             }
-        }
-        double x = x0 + x1, xn2 = n0 + n1;
+            x = x0 + x1;
+            xn2 = n0 + n1;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            x += __shfl_xor_sync(0xffffffffu, x, o);
-            xn2 += __shfl_xor_sync(0xffffffffu, xn2, o);
+            for (int o = 16; o > 0; o >>= 1) {
+                x += __shfl_xor_sync(0xffffffffu, x, o);
+                xn2 += __shfl_xor_sync(0xffffffffu, xn2, o);
+            }
+            n2 = al * al + xn2;
+            if (n2 >= QR_TINY2 || tiny || !(xn2 > 0.0)) break;
+            tiny = true;
+            al *= QR_UP;
+            __syncthreads();  // u has been read by all
+            for (int r = tid; r < 32 * RPL; r += PWC_THREADS) u[r] *= QR_UP;
+            __syncthreads();
         }
         double tau = 0, beta = alpha, scal = 1;
         if (xn2 > 0.0) {
-            const double nrm = sqrt(alpha * alpha + xn2);
-            beta = alpha >= 0 ? -nrm : nrm;
-            const double amb = alpha - beta;
+            const double nrm = sqrt(n2);
+            beta = al >= 0 ? -nrm : nrm;
+            const double amb = al - beta;
             const double rinv = 1.0 / (beta * amb);  // tau = -amb / beta, scal = 1 / amb
             tau = -amb * amb * rinv;
             scal = beta * rinv;
@@ -1198,8 +1235,8 @@ __global__ void __launch_bounds__(PWC_THREADS, 1) qr_panel_tall_kernel(double* _
         }
         if (w == j && lane == 0) {
             sm.taus[j] = tau;
-            sm.scals[j] = scal;
-            sm.betas[j] = beta;
+            sm.scals[j] = tiny ? scal * QR_UP : scal;
+            sm.betas[j] = tiny ? beta * QR_DOWN : beta;
         }
         if (j + 1 < b && w == j + 1) publish(j + 1, par ^ 1);
         __syncthreads();

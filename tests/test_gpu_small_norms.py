@@ -1,14 +1,17 @@
-"""SVD at the ends of the floating-point range, where squares of the entries underflow or overflow: whole
+"""SVD and QR at the ends of the floating-point range, where squares of the entries underflow or overflow: whole
 matrices of tiny and huge entries, harmless tiny columns beside ordinary ones (with zero columns after them), and
 equal columns, whose remainders shrink by a rounding error a step.  Sizes next to those from which the SVD factors
-first, one and several warps and CTAs of its kernel, and batches (the values of a chain's bonds).  Tolerances:
-2 sqrt(m n) 1e-13 of the largest singular value, as for the Jacobi kernels elsewhere."""
+first, one and several warps and CTAs of its kernel, and batches (the values of a chain's bonds).  SVD tolerances:
+2 sqrt(m n) 1e-13 of the largest singular value, as for the Jacobi kernels elsewhere; QR: the bounds of
+test_gpu_qr_cluster.py, 4 eps (k + 16) of orthogonality and of the matrix."""
 import ctypes as C
 
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
 
 
 def tiny_columns(m, n):
@@ -77,3 +80,50 @@ def test_singular_values_alone(m, n, scale):
                   "tn_svd_values")
     s0 = np.linalg.svd(A, compute_uv=False)
     assert np.abs(s.cpu().numpy() / scale - s0).max() <= 2 * np.sqrt(m * n) * 1e-13 * s0[0]
+
+
+def qr(A):
+    """tn_qr of A on a context of its own."""
+    import torch
+    import tensornetworks_b200 as T
+    ctx = T.Context(0)
+    m, n = A.shape
+    k = min(m, n)
+    a = torch.from_numpy(np.ascontiguousarray(A.T)).cuda()
+    q = torch.empty((k, m), dtype=torch.float64, device="cuda")
+    r = torch.empty((n, k), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    T._capi.check(ctx._lib.tn_qr(ctx.handle, m, n, C.c_void_p(a.data_ptr()), m, C.c_void_p(q.data_ptr()), m,
+                                 C.c_void_p(r.data_ptr()), k), "tn_qr")
+    return q.cpu().numpy().T, r.cpu().numpy().T
+
+
+def check_qr(A, e=1.0):
+    Q, R = qr(A)
+    k = min(A.shape)
+    unit = 4 * EPS * (k + 16)
+    assert np.abs(Q.T @ Q - np.eye(k)).max() <= unit
+    assert np.linalg.norm(Q @ (R / e) - A / e) <= unit * np.linalg.norm(A / e)
+    assert np.array_equal(np.tril(R[:, :k], -1), np.zeros((k, k)))
+
+
+@pytest.mark.parametrize("m,n", [(20, 16), (40, 32), (64, 64), (300, 96), (512, 100), (700, 80), (1300, 40), (1600, 40)])
+def test_qr_with_tiny_columns(m, n):
+    check_qr(tiny_columns(m, n))
+    for x in (1e-150, 1e-154, 1e-158):  # at and below the square root of the smallest normal number
+        A = tiny_columns(m, n)
+        A[:, 3] *= x / np.linalg.norm(A[:, 3])
+        check_qr(A)
+
+
+@pytest.mark.parametrize("m,n", [(20, 16), (40, 33), (300, 96), (512, 100), (700, 80), (1300, 40), (1600, 40)])
+def test_qr_of_a_tiny_matrix(m, n):
+    A = np.random.default_rng(m).standard_normal((m, n))
+    check_qr(A * 2.0 ** -512, 2.0 ** -512)
+    check_qr(A * 2.0 ** -505, 2.0 ** -505)
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_qr_of_equal_columns(seed):
+    check_qr(equal_columns(40, 32, seed))
+    check_qr(equal_columns(600, 96, seed))
