@@ -1067,7 +1067,10 @@ int MPSState::sweep(bool left, double epsEigen) {
                             1e6 * secs(t2, t3), launch_count() - n2);
         }
     }
-    TN_CHECK(rq_collect());
+    if (const int rc = rq_collect()) {  // a wait that ran out leaves summaries unwritten: say that instead
+        const int dev = check_device_error(*ctx);
+        return dev ? dev : rc;
+    }
     if (dev_phases) {
         TN_CUDA_CHECK(cudaEventSynchronize(phase_ev[(size_t)4 * (L - 1) + 3]));
         for (int step = 0; step < L; ++step)

@@ -777,6 +777,13 @@ int add_while(cudaGraph_t owner, cudaGraph_t g, const std::vector<cudaGraphNode_
     return TN_OK;
 }
 
+int ensure_summary(Ctx& c) {
+    if (c.lzsum.p) return TN_OK;
+    TN_CHECK(c.lzsum.ensure(sizeof(LzSummary)));
+    TN_CUDA_CHECK(cudaMemsetAsync(c.lzsum.p, 0, sizeof(LzSummary), c.stream));
+    return TN_OK;
+}
+
 int lanczos_solve_async(Ctx& c, long long N, double* x, int m, int maxRestarts, double tol, const MatvecFn& mv,
                         double tol_rel, unsigned long long graph_key, LzSummary* host_out, const VecSplit* split) {
     const VecSplit sp = split ? *split : VecSplit{};
@@ -791,7 +798,7 @@ int lanczos_solve_async(Ctx& c, long long N, double* x, int m, int maxRestarts, 
     size_t need = sizeof(double) * ((size_t)(mm + 4) * N + partial_doubles(N, c.sm_count) + 64);
     TN_CHECK(c.lz.ensure(need));
     TN_CHECK(c.lzstate.ensure(sizeof(LzState)));
-    TN_CHECK(c.lzsum.ensure(sizeof(LzSummary)));
+    TN_CHECK(ensure_summary(c));
     double* V = c.lz.as<double>();
     double* w = V + (size_t)(mm + 1) * N;
     double* xcur = w + N;

@@ -78,5 +78,7 @@ constexpr int LZ_ASYNC_UNAVAILABLE = -1;
 int lanczos_solve_async(Ctx& c, long long N, double* x, int m, int maxRestarts, double tol, const MatvecFn& mv,
                         double tol_rel, unsigned long long graph_key, LzSummary* host_out,
                         const VecSplit* split = nullptr);
+// The summary of the context's device-driven solves, zero before the first (a solve whose wait ran out leaves it).
+int ensure_summary(Ctx& c);
 
 }  // namespace tnb

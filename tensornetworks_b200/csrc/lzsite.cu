@@ -70,6 +70,7 @@ struct LsArgs {
     LzSummary* sum;
     int ldp, nblk, mm, maxR, clustered;  // nblk: CTAs that own vector elements
     double tol, tol_rel;
+    long long polls;                   // of a grid barrier
 };
 
 struct LsSm {
@@ -108,7 +109,7 @@ __device__ __forceinline__ void ls_cluster_wait() {
 // All CTAs have met.  gemm: only the eight product warps of each CTA take part
 // (the clustered form needs every thread: the decision warp arrives for itself).
 // False once a wait has run out of polls (sm.err, the context's error word).
-constexpr long long LS_POLLS = 1LL << 23;
+constexpr long long LS_POLLS = 1LL << 23;  // unless the context says otherwise
 __device__ bool ls_barrier(const LsArgs& a, LsSm& sm, unsigned& target, bool gemm) {
     if (a.clustered) {
         ls_cluster_arrive();
@@ -124,7 +125,7 @@ __device__ bool ls_barrier(const LsArgs& a, LsSm& sm, unsigned& target, bool gem
         long long it = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-        } while (v < target && ++it < LS_POLLS);
+        } while (v < target && ++it < a.polls);
         if (v < target) {
             atomicExch(a.derr, 1);
             sm.err = 1;
@@ -659,7 +660,7 @@ int ls_enqueue(Ctx& c, const LsPlan& p, const ContractShape& s, const WTermDev* 
     const int nblk = (int)((N + LS_BLK - 1) / LS_BLK);
     const size_t nPart = (size_t)(LZ_MAXK + 1) * nblk;
     TN_CHECK(c.lz.ensure(sizeof(double) * (nP + nY + nX + 3 * nPart + 64)));
-    TN_CHECK(c.lzsum.ensure(sizeof(LzSummary)));
+    TN_CHECK(ensure_summary(c));
     TN_CHECK(c.lzbar.ensure(sizeof(unsigned)));
     TN_CHECK(ensure_device_error_word(c));
     a.P = c.lz.as<double>();
@@ -673,6 +674,7 @@ int ls_enqueue(Ctx& c, const LsPlan& p, const ContractShape& s, const WTermDev* 
     a.sum = c.lzsum.as<LzSummary>();
     a.nblk = nblk; a.mm = mm; a.maxR = maxRestarts > 0 ? maxRestarts : 1; a.clustered = p.clustered;
     a.tol = tol; a.tol_rel = tol_rel;
+    a.polls = c.wait_polls < 0 ? LS_POLLS : c.wait_polls;
     const bool wide = s.D1 % 2 == 0 && s.D2 % 2 == 0 && ((reinterpret_cast<uintptr_t>(F) | reinterpret_cast<uintptr_t>(G)) & 15) == 0;
     auto kern = wide ? lz_site_kernel<2> : lz_site_kernel<1>;
     TN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LS_DYN_MAX));

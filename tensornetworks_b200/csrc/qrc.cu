@@ -49,7 +49,7 @@ namespace {
 
 constexpr int QC_TLD = 37;        // leading dimension of T: odd, so that rows are conflict-free
 constexpr int QC_ZLD = 36;        // of Z2: 4 mod 16, as the column blocks
-constexpr int QC_POLLS = 1 << 20;  // of an mbarrier (a poll waits some microseconds by itself)
+constexpr int QC_POLLS = 1 << 20;  // of an mbarrier (a poll waits some microseconds by itself), unless the context says otherwise
 
 struct QcArgs {
     int m, n, k, K;               // K panels
@@ -67,6 +67,7 @@ struct QcArgs {
     int* err;                     // this launch's error word
     int* derr;                    // the context's, and its range word
     long long spin_limit;
+    int polls;                    // of the exchanges' mbarriers
 };
 
 __device__ __forceinline__ unsigned qc_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -94,8 +95,8 @@ __device__ __forceinline__ int qc_ld_acquire(const int* p) {
 }
 // Bounded.  Returns false when the polls ran out, or, with an error word, when
 // another wait of the launch has already failed.
-__device__ __forceinline__ bool qc_mbar_wait(unsigned long long* b, unsigned phase, const int* err) {
-    for (int i = 1; i <= QC_POLLS; ++i) {
+__device__ __forceinline__ bool qc_mbar_wait(unsigned long long* b, unsigned phase, int polls, const int* err) {
+    for (int i = 1; i <= polls; ++i) {
         unsigned done;
         asm volatile(
             "{\n.reg .pred p;\n"
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
         if (!flag_ok) return false;
         const unsigned ph = aphase & 1;
         ++aphase;
-        if (!qc_mbar_wait(&vbar, ph, nullptr)) fail();  // this CTA's own copy
+        if (!qc_mbar_wait(&vbar, ph, QC_POLLS, nullptr)) fail();  // this CTA's own copy
         const int lr0 = 32 * kk / (SL * C) * SL;        // local rows above are zero in V
         // Z = V^T C over the CTA's rows: 16 tiles of 8 x 8 dealt to the warps
         {
@@ -266,7 +267,7 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
                             qc_remote(qc_smem(&zbar), dst));
             }
         }
-        if (!qc_mbar_wait(&zbar, ph, a.err)) fail();
+        if (!qc_mbar_wait(&zbar, ph, a.polls, a.err)) fail();
         // Z2 = T^T Z or T Z on the slice, -Z2 to every CTA
         for (int ct = w >> 2; 8 * ct < SC; ct += W / 4) {
             const int rt = w & 3;
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
                     qc_st_async(qc_remote(at, d), -acc[0], -acc[1], qc_remote(qc_smem(&wbar), d));
             }
         }
-        if (!qc_mbar_wait(&wbar, ph, a.err)) fail();
+        if (!qc_mbar_wait(&wbar, ph, a.polls, a.err)) fail();
         // C += V (-Z2), row tiles of 8 dealt to the warps
         double bz[4][8];
 #pragma unroll
@@ -415,9 +416,9 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
                     const double part = (b0 ? t2[1] : t2[0]) + __shfl_xor_sync(0xffffffffu, b0 ? t2[0] : t2[1], 1);
 #pragma unroll
                     for (int d = 0; d < C; ++d) qc_st_async(dsum[d] + par * NS * 256, part, dbar[d] + 8 * par);
-                    if (tid == 0) qc_mbar_expect(&pbar[par], step_bytes);
+                    if (tid == 0 && live) qc_mbar_expect(&pbar[par], step_bytes);  // one arrival per phase
                     if (j > 0) t_column(j - 1);
-                    if (live && !qc_mbar_wait(&pbar[par], (j >> 1) & 1, a.err)) {
+                    if (live && !qc_mbar_wait(&pbar[par], (j >> 1) & 1, a.polls, a.err)) {
                         live = false;
                         fail();
                     }
@@ -588,6 +589,7 @@ int qc_launch(Ctx& c, QcArgs a, bool* served) {
     a.ready = a.err + 1;
     a.derr = c.derr.as<int>();
     a.spin_limit = c.qr_spin_limit;
+    a.polls = c.wait_polls < 0 ? QC_POLLS : c.wait_polls;
     TN_CUDA_CHECK(cudaMemsetAsync(c.qrsync.p, 0, sizeof(int) * ((size_t)a.K * C + 1), c.stream));
     cfg.gridDim = dim3((unsigned)(C * clusters));
     cfg.numAttrs = 2;

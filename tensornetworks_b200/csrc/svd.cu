@@ -407,26 +407,39 @@ __device__ __forceinline__ void jc_st_async(unsigned dst, double a, double b, un
                  "d"(a), "d"(b), "r"(mbar)
                  : "memory");
 }
-// true once the phase has completed; false after `limit` polls
-__device__ __forceinline__ bool jc_mbar_wait(unsigned long long* b, unsigned phase, int limit) {
-    for (int i = 0; i < limit; ++i) {
-        unsigned done;
-        asm volatile(
-            "{\n.reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(jc_smem(b)), "r"(phase)
-            : "memory");
-        if (done) return true;
+__device__ __forceinline__ bool jc_mbar_try(unsigned long long* b, unsigned phase) {
+    unsigned done;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(jc_smem(b)), "r"(phase)
+        : "memory");
+    return done;
+}
+// The polls after a warp's first: true in every lane once the phase has completed; false after `limit` polls,
+// or when the error word says that another wait has run out.
+__device__ __noinline__ bool jc_mbar_poll(unsigned long long* b, unsigned phase, int limit, const int* err) {
+    for (int i = 1; i < limit; ++i) {
+        if (__all_sync(0xffffffffu, jc_mbar_try(b, phase))) return true;
+        if ((i & 15) == 0) {
+            int e;
+            asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(e) : "l"(err) : "memory");
+            if (__any_sync(0xffffffffu, e)) return false;
+        }
     }
     return false;
+}
+__device__ __forceinline__ bool jc_mbar_wait(unsigned long long* b, unsigned phase, int limit, const int* err) {
+    if (limit > 0 && __all_sync(0xffffffffu, jc_mbar_try(b, phase))) return true;
+    return jc_mbar_poll(b, phase, limit, err);
 }
 constexpr int JC_WAIT_POLLS = 1 << 20;  // a round takes about a microsecond; the waits end long before
 
 template <int E>
 __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __restrict__ jobs, SvdJob one,
-                                                                 int vectors, int parities, int nmax, int* __restrict__ derr) {
+                                                                 int vectors, int parities, int nmax, int polls, int* __restrict__ derr) {
     extern __shared__ __align__(16) double smem[];
     cg::cluster_group cl = cg::this_cluster();
     const int ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -440,6 +453,7 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
     const int ET = (mt + 31) / 32;
     const bool on = gw < NW;
     __shared__ int flags[3];                 // rank 0's are used: "something rotated", by sweep modulo 3
+    __shared__ int failed;                   // rank 0's is used: a wait has run out
     __shared__ double red[32];
     __shared__ double wmax[8];               // largest entry of each warp's columns
     __shared__ int at[32];
@@ -449,6 +463,7 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
     int* rk = reinterpret_cast<int*>(sig + nmax + 2);
     __shared__ unsigned long long mbar[2][8];  // [parity][warp]: the blocks of this round are in the inbox
     if (tid < 3) flags[tid] = 0;
+    if (tid == 0) failed = 0;
     // mbarrier of a warp's inbox: one arrival from each neighbour in this CTA, and the
     // warp's own, which also announces the bytes of those in other CTAs
     const bool from_left = on && gw > 0, from_right = on && gw < NW - 1;
@@ -544,6 +559,9 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
     const double tol = 1e-15 * fmax(1.0, sqrt((double)m) / 4.0), tol2 = tol * tol;
     int sweep = 0;
     unsigned round = 0;  // over all sweeps: inbox parity and mbarrier phase
+    // A warp whose wait ran out rotates, sends and waits no more; its neighbours' waits run out or see the error
+    // word, and the cluster leaves together at the end of the sweep.
+    bool live = on;
     for (sweep = 0; sweep < SVD_MAX_SWEEPS && n > 1; ++sweep) {
         bool rot = false;
         if (on) {
@@ -562,7 +580,7 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
             if (NW == 1) continue;
             const int par = round & 1;
             if (parities == 1 && round > 0) cl.sync();  // the inboxes have been read
-            if (!on) continue;
+            if (!live) continue;
             if (lane == 0) jc_mbar_expect(&mbar[par][wid], remote_bytes);
             if (gw == 0) put(1, 0, par, y0, y1, ny0, ny1);
             else put(-1, 1, par, y0, y1, ny0, ny1);
@@ -577,7 +595,14 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
             } else if (gw > 0) {
                 put(1, 0, par, x0, x1, nx0, nx1);
             }
-            if (!jc_mbar_wait(&mbar[par][wid], (round >> 1) & 1, JC_WAIT_POLLS) && lane == 0) atomicExch(derr, 1);
+            live = jc_mbar_wait(&mbar[par][wid], (round >> 1) & 1, polls, derr);
+            if (!live) {
+                if (lane == 0) {
+                    atomicExch(derr, 1);
+                    *cl.map_shared_rank(&failed, 0) = 1;
+                }
+                continue;
+            }
             if (from_left) get(slot(wid, 0, par), x0, x1, nx0, nx1);
             if (from_right) get(slot(wid, 1, par), y0, y1, ny0, ny1);
         }
@@ -585,7 +610,14 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
         if (rot && lane == 0) *cl.map_shared_rank(&flags[sweep % 3], 0) = 1;
         if (rank == 0 && tid == 0) flags[(sweep + 1) % 3] = 0;
         cl.sync();
-        if (!*cl.map_shared_rank(&flags[sweep % 3], 0)) break;  // the same value in every thread of the cluster
+        // the same values in every thread of the cluster
+        const int f = *cl.map_shared_rank(&failed, 0), rotated = *cl.map_shared_rank(&flags[sweep % 3], 0);
+        if (f) {
+            __nanosleep(200000);  // messages that were given up may still be on their way
+            cl.sync();
+            return;
+        }
+        if (!rotated) break;
     }
 
     // singular values: every CTA gets all of them (slots 4 gw .. 4 gw + 3; padding columns -1)
@@ -750,7 +782,7 @@ int jc_launch(Ctx& c, const SvdJob* dev_jobs, const SvdJob& one, int njobs, JcSh
         }
     }
     TN_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, dev_jobs, one, vectors ? 1 : 0, parities, std::max(np, nmax),
-                                     c.derr.as<int>()));
+                                     c.wait_polls < 0 ? JC_WAIT_POLLS : c.wait_polls, c.derr.as<int>()));
     TN_LAUNCH_CHECK();
     *served = true;
     return TN_OK;
