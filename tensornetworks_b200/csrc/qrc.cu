@@ -608,7 +608,7 @@ int qc_launch(Ctx& c, QcArgs a, bool* served) {
 
 int qr_cluster(Ctx& c, int m, int n, const double* A, long long ars, long long acs, double* Q, long long qrs,
                long long qcs, double* R, long long rrs, long long rcs, const int* colmap) {
-    if (!c.use_persistent_qr || !c.qr_forward_q || m < 1 || n < 1 || m > 1536) return QR_UNAVAILABLE;
+    if (!c.use_cluster_qr || !c.use_persistent_qr || !c.qr_forward_q || m < 1 || n < 1 || m > 1536) return QR_UNAVAILABLE;
     const int k = std::min(m, n);
     // a block of A is read when its cluster starts: outputs in A's memory take the path with a copy
     auto span = [](const double* p, int r, int cl, long long rs, long long cs) {
