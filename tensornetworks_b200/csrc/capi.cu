@@ -215,6 +215,7 @@ int tn_ctx_create(int device, tn_ctx* out) {
     c->c.sm_count = prop.multiProcessorCount;
     if (const char* ng = std::getenv("TN_NO_GRAPHS")) c->c.use_graphs = !(ng[0] == '1');
     if (const char* nc = std::getenv("TN_NO_CLUSTER_QR")) c->c.use_cluster_qr = !(nc[0] == '1');
+    if (const char* ns = std::getenv("TN_NO_SITE_SOLVE")) c->c.use_site_solve = !(ns[0] == '1');
     if (const char* np = std::getenv("TN_NO_PERSISTENT_QR")) c->c.use_persistent_qr = !(np[0] == '1');
     if (const char* fq = std::getenv("TN_QR_FORWARD_Q")) c->c.qr_forward_q = (fq[0] != '0');
     if (const char* sl = std::getenv("TN_QR_SPIN_LIMIT")) c->c.qr_spin_limit = std::max(1LL, std::atoll(sl));

@@ -712,7 +712,7 @@ int lanczos_site(Ctx& c, const ContractShape& s, const WTermDev* terms, int nter
     const long long N = (long long)s.d * s.D1 * s.D2;
     // one element per thread of the chain's reductions (at most one block of 512 per SM), which
     // the sums' order follows
-    if (N <= 0 || N > (long long)LS_BLK * c.sm_count || c.sm_count > 160 || s.d * s.Dw2 > LS_MAXOUT ||
+    if (!c.use_site_solve || N <= 0 || N > (long long)LS_BLK * c.sm_count || c.sm_count > 160 || s.d * s.Dw2 > LS_MAXOUT ||
         nterms > LS_MAXTERMS || s.Dw1 * s.d > 64)
         return LZ_SITE_UNAVAILABLE;
     int mm = std::min(m, LZ_MAXK - 1);

@@ -219,6 +219,7 @@ struct Ctx {
     int sm_count = 148;
     int wait_polls = -1;            // TN_WAIT_POLLS: polls of the waits inside the SVD, cluster QR and site-solve kernels (-1: theirs)
     bool use_cluster_qr = true;     // TN_NO_CLUSTER_QR=1: qr_cluster is unavailable
+    bool use_site_solve = true;     // TN_NO_SITE_SOLVE=1: lanczos_site is unavailable
     bool use_persistent_qr = true;  // TN_NO_PERSISTENT_QR=1: the two-stream look-ahead QR instead
     bool qr_forward_q = true;       // TN_QR_FORWARD_Q=0: the persistent QR forms the thin Q after the panels
     long long qr_spin_limit = 1LL << 21;  // polls per wait in the persistent QR (TN_QR_SPIN_LIMIT)
