@@ -69,14 +69,14 @@ void DevBuf::release() {
     part = false;
 }
 
-int slab_reserve(Ctx& c, const std::vector<DevBuf*>& v, const std::vector<size_t>& need, DevBuf& slab) {
+constexpr size_t SLAB_CHUNK = size_t(64) << 20;
+
+int slab_reserve(Ctx& c, const std::vector<DevBuf*>& v, const std::vector<size_t>& need, Slab& slab) {
     bool enough = true;
-    size_t total = 0;
     std::vector<size_t> size(v.size());
     for (size_t i = 0; i < v.size(); ++i) {
         enough = enough && v[i]->bytes >= need[i];
-        size[i] = std::max(need[i], v[i]->bytes);
-        total += (size[i] + 255) / 256 * 256;
+        size[i] = (std::max(need[i], v[i]->bytes) + 255) / 256 * 256;
     }
     if (enough) return TN_OK;
     // Whatever uses the buffers: this context's streams, and the legacy stream's copies and clears.  Not the device:
@@ -84,25 +84,36 @@ int slab_reserve(Ctx& c, const std::vector<DevBuf*>& v, const std::vector<size_t
     // an error on both sides.
     for (cudaStream_t s : {c.stream, c.own_stream, c.aux, c.aux2, cudaStreamLegacy})
         if (s) TN_CUDA_CHECK(cudaStreamSynchronize(s));
-    DevBuf fresh;
-    TN_CHECK(fresh.ensure(total));
-    char* at = fresh.as<char>();
-    for (size_t i = 0; i < v.size(); ++i) {
-        if (v[i]->p) TN_CUDA_CHECK(cudaMemcpyAsync(at, v[i]->p, v[i]->bytes, cudaMemcpyDeviceToDevice, c.stream));
-        at += (size[i] + 255) / 256 * 256;
+    std::vector<std::unique_ptr<Slab::Chunk>> old;
+    std::swap(old, slab.chunks);
+    size_t freed = 0;  // old chunks with no buffer left in them
+    auto grow = [&](size_t i0, size_t i1, size_t total) -> int {
+        auto ch = std::make_unique<Slab::Chunk>();
+        ch->end = i1;
+        TN_CHECK(ch->mem.ensure(total));
+        char* at = ch->mem.as<char>();
+        for (size_t i = i0; i < i1; at += size[i++])
+            if (v[i]->p) TN_CUDA_CHECK(cudaMemcpyAsync(at, v[i]->p, v[i]->bytes, cudaMemcpyDeviceToDevice, c.stream));
+        TN_CUDA_CHECK(cudaStreamSynchronize(c.stream));
+        at = ch->mem.as<char>();
+        for (size_t i = i0; i < i1; at += size[i++]) {
+            v[i]->release();
+            v[i]->p = at;
+            v[i]->bytes = size[i];
+            v[i]->part = true;
+        }
+        slab.chunks.push_back(std::move(ch));
+        for (; freed < old.size() && old[freed]->end <= i1; ++freed) old[freed].reset();
+        return TN_OK;
+    };
+    int rc = TN_OK;
+    for (size_t i0 = 0, i1 = 0; i0 < v.size() && rc == TN_OK; i0 = i1) {
+        size_t total = 0;
+        for (i1 = i0; i1 < v.size() && (i1 == i0 || total + size[i1] <= SLAB_CHUNK); ++i1) total += size[i1];
+        rc = grow(i0, i1, total);
     }
-    TN_CUDA_CHECK(cudaStreamSynchronize(c.stream));
-    at = fresh.as<char>();
-    for (size_t i = 0; i < v.size(); ++i) {
-        v[i]->release();
-        v[i]->p = at;
-        v[i]->bytes = size[i];
-        v[i]->part = true;
-        at += (size[i] + 255) / 256 * 256;
-    }
-    std::swap(slab.p, fresh.p);
-    std::swap(slab.bytes, fresh.bytes);
-    return TN_OK;
+    for (; freed < old.size(); ++freed) slab.chunks.push_back(std::move(old[freed]));  // after a failure: the rest as it was
+    return rc;
 }
 
 int HostBuf::ensure(size_t nbytes) {

@@ -359,7 +359,7 @@ int MPSState::ensure_capacity(int D) {
     return slab_reserve(*ctx, std::vector<DevBuf*>(A.begin() + 1, A.begin() + L + 1), std::vector<size_t>(L, site), siteSlab);
 }
 
-// The environments that a sweep at the current bonds fills, in one allocation.
+// The environments that a sweep at the current bonds fills.
 int MPSState::reserve_environments() {
     std::vector<DevBuf*> v;
     std::vector<size_t> need;
@@ -373,7 +373,7 @@ int MPSState::reserve_environments() {
     return slab_reserve(*ctx, v, need, envSlab);
 }
 
-// The triangular factors that a half-sweep in direction dir leaves, in one allocation.
+// The triangular factors that a half-sweep in direction dir leaves.
 int MPSState::reserve_factors(int dir) {
     std::vector<DevBuf*> v;
     std::vector<size_t> need;

@@ -73,7 +73,7 @@ struct MPSState {
     std::vector<char> bondDirty;              // bond_s lags behind the latest factor
     std::vector<double> Emin, iterDE, gapE;
     std::unique_ptr<MpsScratch, MpsScratchDelete> scratch{new MpsScratch};
-    DevBuf siteSlab, envSlab, factorSlab[2];  // what the tensors, environments and factors are parts of
+    Slab siteSlab, envSlab, factorSlab[2];  // what the tensors, environments and factors are parts of
     static constexpr int RQ_SLOT = 12;  // doubles per site
     std::vector<char> rq_pending, rq_lz, rq_exact;  // rq_exact: an FP64 solve, no separate check
     std::vector<double> rq_dtheta, rq_flop;

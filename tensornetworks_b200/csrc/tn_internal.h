@@ -104,10 +104,20 @@ struct DevBuf {
 
 struct Ctx;
 
-// Every buffer of v gets its need[] bytes (where it has less) as a part of one
-// allocation, which replaces the slab they were parts of before; contents are kept.
+// The allocations that the buffers of a list are parts of, in the list's order.
+struct Slab {
+    struct Chunk {
+        DevBuf mem;
+        size_t end = 0;  // the list's buffers before this one are in this chunk or earlier ones
+    };
+    std::vector<std::unique_ptr<Chunk>> chunks;
+};
+
+// Every buffer of v gets its need[] bytes (where it has less) as a part of a few
+// allocations of about 64 MB (or one buffer), which replace those they were parts of
+// one by one: growth holds one of them beside the buffers.  Contents are kept.
 // Waits for the streams of c, which uses the buffers.
-int slab_reserve(Ctx& c, const std::vector<DevBuf*>& v, const std::vector<size_t>& need, DevBuf& slab);
+int slab_reserve(Ctx& c, const std::vector<DevBuf*>& v, const std::vector<size_t>& need, Slab& slab);
 
 // Pinned host buffer for small device->host reads.
 struct HostBuf {

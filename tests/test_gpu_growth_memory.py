@@ -1,0 +1,36 @@
+"""Growing a chain's site tensors holds the new ones and little else: with less free memory than the new tensors take
+together, but enough beside the old ones given back on the way, the growth succeeds and keeps the contents."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def test_growth_within_the_memory_of_the_new_tensors():
+    import torch
+    import tensornetworks_b200 as T
+    ctx = T.Context(0)
+    L, D = 64, 512                      # 64 tensors of 4 MB, then of 16 MB: 1024 MB, 768 MB more than before
+    H = T.Factory(ctx).Make1D_NN_HeisenbergHamiltonian(L, 0.5, T.RegularLower, 1.0, 1.0, 0.0)
+    psi = H.CreateMPS(D, 1e-12, 1e-12)
+    rng = np.random.default_rng(2)
+    some = {i: rng.standard_normal((2, 1 if i == 1 else D, 1 if i == L else D)) for i in (1, 2, 17, 33, 63, 64)}
+    for i, A in some.items():
+        psi.SetSite(i, A)
+    ctx.synchronize()
+    torch.cuda.synchronize()
+    fill = torch.cuda.mem_get_info()[0] - 960 * MB
+    if fill < 0:
+        pytest.skip("another process holds the memory")
+    hold = torch.empty(fill, dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < 1000 * MB
+        psi.SetSite(5, np.ones((2, D, 2 * D)))
+        for i, A in some.items():
+            assert np.array_equal(psi.GetSite(i), A)
+        assert (psi.GetSite(5) == 1).all()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
