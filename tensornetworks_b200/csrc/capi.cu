@@ -737,6 +737,16 @@ int tn_eigensolve_heff(tn_ctx c, const tn_solver_options* opt, int d, int Dw1, i
     return r.converged ? TN_OK : TN_NOT_CONVERGED;
 }
 
+// A dense solver's workspace stays in the context for the next call up to this size; a larger one, whose
+// solve takes a hundred times what an allocation does, is given back.
+constexpr size_t KEEP_BYTES = size_t(64) << 20;
+struct GiveBack {
+    DevBuf& b;
+    ~GiveBack() {
+        if (b.bytes > KEEP_BYTES) b.release();
+    }
+};
+
 int tn_eigensolve_dense(tn_ctx c, int N, const double* A, int lda, int k, double tol, double* w_host, double* U,
                         int ldu) {
     if (!c || !A || !w_host || !U || N < 1 || k < 1 || k > N || lda < N || ldu < N || !(tol >= 0.0)) return TN_BAD_ARG;
@@ -751,6 +761,7 @@ int tn_eigensolve_dense(tn_ctx c, int N, const double* A, int lda, int k, double
     // eigenvalues s_i - sigma (descending) -- all on the device.
     const size_t n2 = (size_t)N * N;
     DevBuf& work = cx.apiw[0];
+    GiveBack large{work};
     TN_CHECK(work.ensure(sizeof(double) * (4 * n2 + (size_t)N + 8)));
     double* W = work.as<double>();
     double* V = W + n2;
@@ -781,6 +792,7 @@ static int svd_common(tn_ctx c, int m, int n, const double* A, int lda, double* 
     const int tm = tall ? m : n, tn = tall ? n : m;
     size_t need = (size_t)tm * tn + (size_t)tn * tn + (tall ? 0 : (size_t)tm * tn + (size_t)tn * tn);
     DevBuf& work = cx.apiw[0];
+    GiveBack large{work};
     TN_CHECK(work.ensure(sizeof(double) * need));
     double* Wm = work.as<double>();
     double* V = Wm + (size_t)tm * tn;
@@ -825,6 +837,7 @@ int tn_svd_solve(tn_ctx c, int m, int n, const double* A, int lda, double eps, i
     TN_ON_DEVICE(c->c.device);
     Ctx& cx = c->c;
     DevBuf& full = cx.apiw[1];
+    GiveBack large{full};
     TN_CHECK(full.ensure(sizeof(double) * ((size_t)m * mn + (size_t)mn * n + mn)));
     double* Uf = full.as<double>();
     double* Vf = Uf + (size_t)m * mn;

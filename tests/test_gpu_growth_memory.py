@@ -1,5 +1,8 @@
-"""Growing a chain's site tensors holds the new ones and little else: with less free memory than the new tensors take
-together, but enough beside the old ones given back on the way, the growth succeeds and keeps the contents."""
+"""Memory that is held and given back.  Growing a chain's site tensors holds the new ones and little else: with less
+free memory than the new tensors take together, but enough beside the old ones given back on the way, the growth
+succeeds and keeps the contents.  Large workspaces of the dense solvers and of a chain do not stay behind."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -34,3 +37,39 @@ def test_growth_within_the_memory_of_the_new_tensors():
     finally:
         del hold
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("solve", ["values", "solve", "eigen"])
+def test_large_workspaces_of_the_dense_solvers_are_given_back(solve):
+    import torch
+    import tensornetworks_b200 as T
+    ctx = T.Context(0)
+
+    def run(m, n):
+        rng = np.random.default_rng(m)
+        A = rng.standard_normal((m, n))
+        if solve == "eigen":
+            A = np.diag(np.arange(1.0, n + 1))
+        a = torch.from_numpy(np.ascontiguousarray(A.T)).cuda()
+        u, s = torch.empty((n, m), dtype=torch.float64, device="cuda"), torch.empty(n, dtype=torch.float64, device="cuda")
+        v = torch.empty((n, n), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        p = lambda t: C.c_void_p(t.data_ptr())
+        if solve == "values":
+            rc = ctx._lib.tn_svd_values(ctx.handle, m, n, p(a), m, p(s))
+        elif solve == "solve":
+            rc = ctx._lib.tn_svd_solve(ctx.handle, m, n, p(a), m, 1e-12, n, p(u), m, p(s), p(v), n)
+        else:
+            w = np.empty(1)
+            rc = ctx._lib.tn_eigensolve_dense(ctx.handle, n, p(a), n, 1, 1e-12, C.c_void_p(w.ctypes.data), p(u), m)
+            assert abs(w[0] - 1) < 1e-10 * n
+        assert rc == 0, T._capi.last_error()
+
+    big = (1600, 1600) if solve == "eigen" else (3000000, 3)  # 82 MB (four matrices) and 72 MB of workspace
+    run(3, 3)
+    torch.cuda.empty_cache()
+    ctx.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    run(*big)
+    torch.cuda.empty_cache()
+    assert before - torch.cuda.mem_get_info()[0] < 32 * MB
