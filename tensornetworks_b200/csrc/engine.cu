@@ -283,8 +283,16 @@ int Hamiltonian::build() {
 // ---------------------------------------------------------------------------
 void MpsScratchDelete::operator()(MpsScratch* s) const { delete s; }
 
+size_t MpsScratch::device_bytes() const {
+    size_t n = 0;
+    for (const DevBuf* b : {&tmp, &Wqr, &Qqr, &svdw, &envA, &envB, &yvec, &diagbuf, &rqP, &rqQ, &rqbuf, &msite.Fs,
+                            &msite.Gc, &msite.Xs, &msite.Ps, &msite.segs, &msite.tune})
+        n += b->bytes;
+    return n;
+}
+
 MPSState::~MPSState() {
-    if (ctx && scratch) {  // the work buffers go to the next MPS of this context
+    if (ctx && scratch && scratch->device_bytes() <= MpsScratch::KEEP_BYTES) {  // the work buffers go to the next MPS of this context
         std::lock_guard<std::mutex> lk(ctx->spare_mu);
         ctx->spare = std::move(scratch);
     }

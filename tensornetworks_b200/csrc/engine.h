@@ -36,8 +36,9 @@ struct SiteSet {
     std::vector<int> D1, D2;
 };
 
-// Work buffers of an MPS's sweeps, which the context hands from one MPS to the next.
+// Work buffers of an MPS's sweeps, which the context hands from one MPS to the next, up to KEEP_BYTES in all.
 struct MpsScratch {
+    static constexpr size_t KEEP_BYTES = size_t(256) << 20;  // L = 100, D = 256 at S = 1/2 takes about 80 MB
     DevBuf tmp, Wqr, Qqr, svdw, envA, envB, yvec, diagbuf;
     // FP64 check of the split-precision eigenvector on the context's second side
     // stream (refine_tol = 0): contraction scratch, reduction state, and per site
@@ -47,6 +48,7 @@ struct MpsScratch {
     DevBuf rqP, rqQ, rqbuf;
     HostBuf rqhost;
     MixedSite msite;
+    size_t device_bytes() const;
 };
 
 struct MPSState {

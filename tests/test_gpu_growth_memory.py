@@ -73,3 +73,23 @@ def test_large_workspaces_of_the_dense_solvers_are_given_back(solve):
     run(*big)
     torch.cuda.empty_cache()
     assert before - torch.cuda.mem_get_info()[0] < 32 * MB
+
+
+def test_large_workspaces_of_a_chain_are_given_back():
+    import gc
+    import torch
+    import tensornetworks_b200 as T
+    ctx = T.Context(0)
+    H = T.Factory(ctx).Make1D_NN_HeisenbergHamiltonian(4, 0.5, T.RegularLower, 1.0, 1.0, 0.0)
+    psi = H.CreateMPS(8, 1e-12, 1e-12)
+    psi.GetExpectation(H)
+    torch.cuda.empty_cache()
+    ctx.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    D = 3000  # two environments of 343 MB
+    psi = H.CreateMPS(D, 1e-12, 1e-12)
+    psi.GetExpectation(H)
+    del psi
+    gc.collect()
+    contraction = 2 * 8 * 2 * 5 * D * D  # the context's own pair of scratch buffers
+    assert before - torch.cuda.mem_get_info()[0] < contraction + 64 * MB
