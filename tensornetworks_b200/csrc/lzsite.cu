@@ -70,7 +70,7 @@ struct LsArgs {
     LzSummary* sum;
     int ldp, nblk, mm, maxR, clustered;  // nblk: CTAs that own vector elements
     double tol, tol_rel;
-    long long polls;                   // of a grid barrier
+    int polls;                         // of a grid barrier
 };
 
 struct LsSm {
@@ -109,7 +109,7 @@ __device__ __forceinline__ void ls_cluster_wait() {
 // All CTAs have met.  gemm: only the eight product warps of each CTA take part
 // (the clustered form needs every thread: the decision warp arrives for itself).
 // False once a wait has run out of polls (sm.err, the context's error word).
-constexpr long long LS_POLLS = 1LL << 23;  // unless the context says otherwise
+constexpr int LS_POLLS = 1 << 23;  // unless the context says otherwise
 __device__ bool ls_barrier(const LsArgs& a, LsSm& sm, unsigned& target, bool gemm) {
     if (a.clustered) {
         ls_cluster_arrive();
@@ -122,10 +122,10 @@ __device__ bool ls_barrier(const LsArgs& a, LsSm& sm, unsigned& target, bool gem
         target += gridDim.x;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
         unsigned v = 0;
-        long long it = 0;
+        int left = a.polls;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-        } while (v < target && ++it < a.polls);
+        } while (v < target && --left > 0);
         if (v < target) {
             atomicExch(a.derr, 1);
             sm.err = 1;
