@@ -25,8 +25,10 @@ namespace {
 constexpr int QR_THREADS = 512;
 
 // A reflector's column whose squared norm is below QR_TINY2 (squares underflow from 2^-1022 on, and 1 / (beta
-// (alpha - beta)) overflows) is multiplied by QR_UP and its sums are formed again.
-constexpr double QR_TINY2 = 0x1p-960, QR_UP = 0x1p600, QR_DOWN = 0x1p-600;
+// (alpha - beta)) overflows) is multiplied by QR_UP and its sums are formed again.  The register panels look for
+// such columns once, at their end, and only then factor again with that test in every step (CAREFUL), which
+// costs 17 us of a 512 x 256 QR's 430.
+constexpr double QR_TINY2 = 0x1p-960, QR_TINY = 0x1p-480, QR_UP = 0x1p600, QR_DOWN = 0x1p-600;
 
 __device__ __forceinline__ double wsum(double v) {
 #pragma unroll
@@ -251,10 +253,16 @@ __device__ void build_t(const double (&Gs)[32][33], const double* taus, double (
     }
 }
 
-template <int RPL>
-__device__ __forceinline__ void panel_wc(double* __restrict__ W, int ldw, int m, int j0, int b,
-                                         double* __restrict__ V, int ldv, double* __restrict__ T, int ldt,
-                                         PanelWcSmem& sm) {
+// Every thread of the block gets whether one of the panel's reflectors is of a tiny column (or not a number).
+__device__ __forceinline__ bool panel_has_tiny(const double* taus, const double* betas, int b) {
+    const int lane = threadIdx.x & 31;
+    return __any_sync(0xffffffffu, lane < b && taus[lane] != 0.0 && !(fabs(betas[lane]) >= QR_TINY));
+}
+
+template <int RPL, bool CAREFUL>
+__device__ __forceinline__ bool panel_wc_run(double* __restrict__ W, int ldw, int m, int j0, int b,
+                                             double* __restrict__ V, int ldv, double* __restrict__ T, int ldt,
+                                             PanelWcSmem& sm) {
     constexpr int B = 32, CPW = 32 / PWC_WARPS;  // columns per warp
     static_assert(32 * RPL <= PWC_MAXR && CPW * PWC_WARPS == B, "panel shape");
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -323,7 +331,7 @@ __device__ __forceinline__ void panel_wc(double* __restrict__ W, int ldw, int m,
                 for (int v = 0; v <= CPW; ++v) x[v] += __shfl_xor_sync(0xffffffffu, x[v], o);
             }
             n2 = al * al + x[CPW];
-            if (n2 >= QR_TINY2 || tiny || !(x[CPW] > 0.0)) break;
+            if (!CAREFUL || n2 >= QR_TINY2 || tiny || !(x[CPW] > 0.0)) break;
             tiny = true;
             al *= QR_UP;
 #pragma unroll
@@ -362,6 +370,7 @@ __device__ __forceinline__ void panel_wc(double* __restrict__ W, int ldw, int m,
         if (j + 1 < b && w == (j + 1) / CPW) publish(j + 1, par ^ 1);
         __syncthreads();
     }
+    if (!CAREFUL && panel_has_tiny(sm.taus, sm.betas, b)) return false;
     // the factored panel: R above and on the diagonal, v below it
 #pragma unroll
     for (int ci = 0; ci < CPW; ++ci) {
@@ -380,6 +389,21 @@ __device__ __forceinline__ void panel_wc(double* __restrict__ W, int ldw, int m,
         }
     }
     build_t(sm.Gs, sm.taus, sm.Tsm, sm.Xs, b, T, ldt);
+    return true;
+}
+
+template <int RPL>
+__device__ __noinline__ void panel_wc_careful(double* W, int ldw, int m, int j0, int b, double* V, int ldv, double* T,
+                                              int ldt, PanelWcSmem& sm) {
+    __syncthreads();  // the first attempt's scalars have been read; W is as it was
+    panel_wc_run<RPL, true>(W, ldw, m, j0, b, V, ldv, T, ldt, sm);
+}
+
+template <int RPL>
+__device__ __forceinline__ void panel_wc(double* W, int ldw, int m, int j0, int b, double* V, int ldv, double* T,
+                                         int ldt, PanelWcSmem& sm) {
+    if (!panel_wc_run<RPL, false>(W, ldw, m, j0, b, V, ldv, T, ldt, sm))
+        panel_wc_careful<RPL>(W, ldw, m, j0, b, V, ldv, T, ldt, sm);
 }
 
 // the panel by rows per lane
@@ -1150,12 +1174,10 @@ struct PanelTallSmem {
     double Xs[32][33];
 };
 
-template <int RPL>
-__global__ void __launch_bounds__(PWC_THREADS, 1) qr_panel_tall_kernel(double* __restrict__ W, int ldw, int m, int j0,
-                                                                        int b, double* __restrict__ T, int ldt) {
+template <int RPL, bool CAREFUL>
+__device__ __forceinline__ bool panel_tall_run(double* __restrict__ W, int ldw, int m, int j0, int b,
+                                               double* __restrict__ T, int ldt, PanelTallSmem& sm) {
     static_assert(32 * RPL <= TALL_MAXR, "panel rows");
-    extern __shared__ double tall_dyn[];
-    PanelTallSmem& sm = *reinterpret_cast<PanelTallSmem*>(tall_dyn);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;  // warp w: column w of the panel (w < b)
     const int mp = m - j0;
     for (int e = tid; e < 32 * 33; e += PWC_THREADS) (&sm.Gs[0][0])[e] = 0.0;
@@ -1205,7 +1227,7 @@ __global__ void __launch_bounds__(PWC_THREADS, 1) qr_panel_tall_kernel(double* _
                 xn2 += __shfl_xor_sync(0xffffffffu, xn2, o);
             }
             n2 = al * al + xn2;
-            if (n2 >= QR_TINY2 || tiny || !(xn2 > 0.0)) break;
+            if (!CAREFUL || n2 >= QR_TINY2 || tiny || !(xn2 > 0.0)) break;
             tiny = true;
             al *= QR_UP;
             __syncthreads();  // u has been read by all
@@ -1241,6 +1263,7 @@ __global__ void __launch_bounds__(PWC_THREADS, 1) qr_panel_tall_kernel(double* _
         if (j + 1 < b && w == j + 1) publish(j + 1, par ^ 1);
         __syncthreads();
     }
+    if (!CAREFUL && panel_has_tiny(sm.taus, sm.betas, b)) return false;
     // the factored panel: R above and on the diagonal, v below it
     if (w < b) {
         const double sc = sm.scals[w], be = sm.betas[w];
@@ -1251,6 +1274,22 @@ __global__ void __launch_bounds__(PWC_THREADS, 1) qr_panel_tall_kernel(double* _
         }
     }
     build_t(sm.Gs, sm.taus, sm.Tsm, sm.Xs, b, T, ldt);
+    return true;
+}
+
+template <int RPL>
+__device__ __noinline__ void panel_tall_careful(double* W, int ldw, int m, int j0, int b, double* T, int ldt,
+                                                PanelTallSmem& sm) {
+    __syncthreads();  // the first attempt's scalars have been read; W is as it was
+    panel_tall_run<RPL, true>(W, ldw, m, j0, b, T, ldt, sm);
+}
+
+template <int RPL>
+__global__ void __launch_bounds__(PWC_THREADS, 1) qr_panel_tall_kernel(double* __restrict__ W, int ldw, int m, int j0,
+                                                                        int b, double* __restrict__ T, int ldt) {
+    extern __shared__ double tall_dyn[];
+    PanelTallSmem& sm = *reinterpret_cast<PanelTallSmem*>(tall_dyn);
+    if (!panel_tall_run<RPL, false>(W, ldw, m, j0, b, T, ldt, sm)) panel_tall_careful<RPL>(W, ldw, m, j0, b, T, ldt, sm);
 }
 
 // C (mp x nc, ld ldc) <- (I - V T' V^T) C, V mp x b (b <= 16) unit lower
