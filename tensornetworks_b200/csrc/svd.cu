@@ -39,6 +39,18 @@ __device__ __forceinline__ double jc_matrix_scale(double amax) {
     return __hiloint2double(max(1, 0x7fe - e) << 20, 0);
 }
 
+// Descending order of values with their indices, NaN first: a total order, so that every column gets its own place.
+__device__ __forceinline__ bool ranks_before(double si, int i, double sj, int j) {
+    const bool ni = si != si, nj = sj != sj;
+    return ni || nj ? (ni && (!nj || i < j)) : si > sj || (si == sj && i < j);
+}
+
+__device__ __forceinline__ double nan_value() { return __longlong_as_double(0x7ff8000000000000LL); }
+
+// A column of U is that of the matrix, not one of its completion.  (NaN: the values of a matrix with a NaN in it
+// are all NaN, and nothing is completed.)
+__device__ __forceinline__ bool keeps_column(double s, double cut) { return !(s <= cut) && s != 0.0; }
+
 __device__ __forceinline__ int rr_pos(int q, int r, int ne) {
     return q == 0 ? 0 : ((q - 1 + r) % (ne - 1)) + 1;
 }
@@ -60,11 +72,11 @@ __device__ void complete_u(const SvdJob& jb, double* U, long long rs, long long 
     int next_e = 0;
     for (int c = 0; c < n; ++c) {
         const double sc = __ldcg(jb.s + c);
-        if (sc > cut && sc > 0.0) continue;
+        if (keeps_column(sc, cut)) continue;
         double* uc = U + c * cs;
         auto accepted = [&](int p) {
             const double sp = __ldcg(jb.s + p);
-            return p != c && ((sp > cut && sp > 0.0) || p < c);
+            return p != c && (keeps_column(sp, cut) || p < c);
         };
         for (bool placed = false; !placed;) {
             int e = next_e++;
@@ -231,28 +243,28 @@ __global__ void __launch_bounds__(SVD_THREADS) jacobi_svd_kernel(const SvdJob* _
         if (lane == 0) norms[j] = sqrt(s);
     }
     __syncthreads();
-    // descending rank, ties broken by column index
+    // descending rank, ties broken by column index; a NaN anywhere makes every value NaN
+    bool nan = false;
+    for (int j = 0; j < n; ++j) nan = nan || norms[j] != norms[j];
+    const double unscale = nan ? nan_value() : 1.0 / scale;
     for (int j = tid; j < n; j += blockDim.x) {
         const double sj = norms[j];
         int rk = 0;
-        for (int i = 0; i < n; ++i) {
-            double si = norms[i];
-            rk += (si > sj) || (si == sj && i < j);
-        }
+        for (int i = 0; i < n; ++i) rk += ranks_before(norms[i], i, sj, j);
         rank[j] = rk;
-        jb.s[rk] = sj / scale;
+        jb.s[rk] = sj * unscale;
     }
     __syncthreads();
     double smax = 0;
     for (int j = 0; j < n; ++j) smax = fmax(smax, norms[j]);
-    const double cut = smax * 1e-13 * fmax(1.0, (double)m) / scale;
+    const double cut = smax * 1e-13 * fmax(1.0, (double)m) * unscale;
     if (vectors) {
         for (int j = wid; j < n; j += nw) {
             const int rk = rank[j];
             const double sj = norms[j];
             const double* cj = A + (size_t)j * m;
             double* uo = jb.U + (size_t)rk * jb.ldu;
-            const bool good = sj / scale > cut && sj / scale > 0.0;
+            const bool good = keeps_column(sj * unscale, cut);
             for (int i = lane; i < m; i += 32) uo[i] = good ? cj[i] / sj : 0.0;
             const double* vj = V + (size_t)j * n;
             for (int i = lane; i < n; i += 32) jb.Vt[(size_t)i * jb.ldvt + rk] = vj[i];
@@ -633,28 +645,28 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(const SvdJob* __
         }
     }
     cl.sync();
-    // descending rank, ties broken by position
+    // descending rank, ties broken by position; a NaN anywhere makes every value NaN
     const int np = 4 * NW;
+    bool nan = false;
+    for (int j = 0; j < np; ++j) nan = nan || sig[j] != sig[j];
+    const double unscale = nan ? nan_value() : 1.0 / scale;
     for (int j = tid; j < np; j += blockDim.x) {
         const double sj = sig[j];
         int k = 0;
-        for (int i = 0; i < np; ++i) {
-            const double si = sig[i];
-            k += (si > sj) || (si == sj && i < j);
-        }
+        for (int i = 0; i < np; ++i) k += ranks_before(sig[i], i, sj, j);
         rk[j] = sj < 0 ? -1 : k;
-        if (rank == 0 && !(sj < 0)) jb.s[min(k, n - 1)] = sj / scale;
+        if (rank == 0 && !(sj < 0)) jb.s[min(k, n - 1)] = sj * unscale;
     }
     __syncthreads();
     if (vectors) {
         double smax = 0;
         for (int j = 0; j < np; ++j) smax = fmax(smax, sig[j]);
-        const double cut = smax * 1e-13 * fmax(1.0, (double)m) / scale;
+        const double cut = smax * 1e-13 * fmax(1.0, (double)m) * unscale;
         auto emit = [&](const double(&v)[E], int j) {
             const int k = rk[j];
             if (k < 0) return;
-            const double sj = sig[j], so = sj / scale;
-            const bool good = so > cut && so > 0.0;  // as complete_u asks
+            const double sj = sig[j];
+            const bool good = keeps_column(sj * unscale, cut);
             const int kc = min(k, n - 1);
 #pragma unroll
             for (int q = 0; q < E; ++q) {
@@ -730,7 +742,7 @@ __global__ void __launch_bounds__(1024) svd_order_kernel(const double* __restric
 // none: not served.  Four warps per CTA (one per scheduler) up to n = 128, eight
 // above, so that eight CTAs hold n = 256; with 16 row slots eight warps'
 // inboxes fit one parity only, and 16 CTAs of four warps are tried first
-// (256 x 256 with vectors, graded over three decades: 6.0 against 10.2 ms).
+// (256 x 256 with vectors, graded over three decades: 3.8 against 5.8 ms, 5.5 against 8.9 without the factorisation).
 struct JcShape {
     int ncta = 0, warps = 0;
 };
@@ -816,7 +828,7 @@ int svd_batched(Ctx& c, const std::vector<SvdJob>& jobs, bool vectors) {
     }
     // Every job of the batch fits the cluster kernel (n <= 512 and at most 16
     // slots of 32 rows per column, rows of U and V together): there it is the
-    // faster one at every size (25 x 25 0.24 against 0.44 ms, 150 x 128 1.95 against
+    // faster one at every size (25 x 25 0.22 against 0.44 ms, 150 x 128 1.87 against
     // 26.7, both without the factorisation below); otherwise one CTA per matrix with its columns in shared
     // memory or L2.
     TN_CHECK(ensure_device_error_word(c));
@@ -838,9 +850,9 @@ int svd_batched(Ctx& c, const std::vector<SvdJob>& jobs, bool vectors) {
     // A single matrix of some size is factored first, its columns by descending norm: A P = Q R, and the rotations
     // that orthogonalise the columns of R^T (Drmac and Veselic, SIAM J. Matrix Anal. Appl. 29, 2008: R^T is closer to
     // diagonal than A) turn Q into U: R^T J = V' S gives A = (Q J) S (P V')^T.  The same kernel with R^T
-    // above and Q's rows below, 9-11 sweeps instead of 14-19.  Factored and not (graded over three decades, host to
-    // host): 16 x 16 140 and 150 us, 20 x 20 166 and 166, 25 x 25 205 and 240, 64 x 64 488 and 630,
-    // 150 x 128 1383 and 1947, 160 x 160 2255 and 3220; 150 x 128 26.7 ms with one CTA per matrix.
+    // above and Q's rows below, 9-11 sweeps instead of 14-19.  Factored and not (a call of tn_svd, graded over three
+    // decades): 16 x 16 136 and 119 us, 20 x 20 159 and 142, 25 x 25 204 and 223, 64 x 64 479 and 614,
+    // 150 x 128 1421 and 1869, 160 x 160 2141 and 3197; 150 x 128 26.7 ms with one CTA per matrix.
     const SvdJob& j0 = jobs[0];
     if (nj == 1 && j0.n >= SVD_PRE_MIN && !shapes.empty()) {
         const size_t nq = vectors ? (size_t)j0.m * j0.n : 0, nr = (size_t)j0.n * j0.n;
