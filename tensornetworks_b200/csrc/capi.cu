@@ -267,7 +267,9 @@ int tn_ctx_destroy(tn_ctx c) {
 
 int tn_ctx_set_stream(tn_ctx c, void* stream) {
     if (!c) return TN_BAD_ARG;
-    c->c.stream = stream ? (cudaStream_t)stream : c->c.own_stream;
+    const cudaStream_t s = stream ? (cudaStream_t)stream : c->c.own_stream;
+    if (s != c->c.stream) ++c->c.stream_changes;
+    c->c.stream = s;
     return TN_OK;
 }
 

@@ -292,7 +292,9 @@ size_t MpsScratch::device_bytes() const {
 }
 
 MPSState::~MPSState() {
-    if (ctx && scratch && scratch->device_bytes() <= MpsScratch::KEEP_BYTES) {  // the work buffers go to the next MPS of this context
+    // The work buffers go to the next MPS of this context -- unless its stream has changed meanwhile: work of this MPS
+    // may then still run on the former stream, which only freeing the buffers waits for.
+    if (ctx && scratch && scratch->device_bytes() <= MpsScratch::KEEP_BYTES && ctx->stream_changes == stream_changes) {
         std::lock_guard<std::mutex> lk(ctx->spare_mu);
         ctx->spare = std::move(scratch);
     }
@@ -312,6 +314,7 @@ int MPSState::init(Hamiltonian* h, int D) {
         std::lock_guard<std::mutex> lk(ctx->spare_mu);
         if (ctx->spare) scratch = std::move(ctx->spare);
     }
+    stream_changes = ctx->stream_changes;
     L = h->L;
     d = h->d;
     D1.assign(L + 2, 1);

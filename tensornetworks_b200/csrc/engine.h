@@ -75,6 +75,7 @@ struct MPSState {
     std::vector<char> bondDirty;              // bond_s lags behind the latest factor
     std::vector<double> Emin, iterDE, gapE;
     std::unique_ptr<MpsScratch, MpsScratchDelete> scratch{new MpsScratch};
+    unsigned stream_changes = 0;  // the context's when the chain was made
     Slab siteSlab, envSlab, factorSlab[2];  // what the tensors, environments and factors are parts of
     static constexpr int RQ_SLOT = 12;  // doubles per site
     std::vector<char> rq_pending, rq_lz, rq_exact;  // rq_exact: an FP64 solve, no separate check

@@ -245,6 +245,7 @@ struct Ctx {
     // then stay the same, and nothing is allocated again); at most one set, freed with the
     // context.  The lock: an MPS may be destroyed by another thread than the one that uses
     // the context.
+    unsigned stream_changes = 0;  // by tn_ctx_set_stream
     std::mutex spare_mu;
     std::unique_ptr<MpsScratch, MpsScratchDelete> spare;
 };

@@ -93,3 +93,28 @@ def test_large_workspaces_of_a_chain_are_given_back():
     gc.collect()
     contraction = 2 * 8 * 2 * 5 * D * D  # the context's own pair of scratch buffers
     assert before - torch.cuda.mem_get_info()[0] < contraction + 64 * MB
+
+
+def test_work_buffers_do_not_outlive_a_change_of_stream():
+    """A chain that has worked on a stream that the context no longer uses frees its buffers (which waits for the
+    device) instead of handing them to the next chain, which would use them on another stream."""
+    import gc
+    import torch
+    import tensornetworks_b200 as T
+    ctx = T.Context(0)
+    H = T.Factory(ctx).Make1D_NN_HeisenbergHamiltonian(4, 0.5, T.RegularLower, 1.0, 1.0, 0.0)
+    D = 1000  # two environments of 38 MB
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    left = []
+    for change in (True, False):
+        T._capi.check(ctx._lib.tn_ctx_set_stream(ctx.handle, C.c_void_p(streams[0].cuda_stream)), "set_stream")
+        psi = H.CreateMPS(D, 1e-12, 1e-12)
+        psi.GetExpectation(H)
+        if change:
+            T._capi.check(ctx._lib.tn_ctx_set_stream(ctx.handle, C.c_void_p(streams[1].cuda_stream)), "set_stream")
+        del psi
+        gc.collect()
+        torch.cuda.synchronize()
+        left.append(torch.cuda.mem_get_info()[0])
+    T._capi.check(ctx._lib.tn_ctx_set_stream(ctx.handle, None), "set_stream")
+    assert left[0] - left[1] > 64 * MB  # kept without a change, not kept with one
