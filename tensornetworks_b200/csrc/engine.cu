@@ -446,8 +446,8 @@ int MPSState::rescale_site(int ia) {
 }
 
 // Thin QR of the gauge matrix W (m x n, ld m; overwritten) into Q (m x k, ld m)
-// and R (k x n, ld ldr): blocked Householder.  Not the cluster kernel (qr_cluster), though it takes 0.30 ms at
-// 512 x 256 where this takes 0.43: a sweep's stopping decisions see its rounding, and with its
+// and R (k x n, ld ldr): blocked Householder.  Not the cluster kernel (qr_cluster), though it takes a third
+// less time at 512 x 256 (tn_qr 0.33 ms, 0.49 with this): a sweep's stopping decisions see its rounding, and with its
 // sums in another order 1 of 50 split-precision searches (L = 32, D = 256) ended 3e-4 off in the bond
 // values and FP64 sweeps moved by 1e-8, where this order leaves both as they were bit for bit.
 int MPSState::gauge_qr(int m, int n, double* W, double* Q, double* R, int ldr) {

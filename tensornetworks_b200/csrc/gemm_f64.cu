@@ -1,4 +1,5 @@
-// gemm_f64.cu -- FP64 batched GEMM with split-index addressing (SIMT DFMA).
+// gemm_f64.cu -- FP64 batched GEMM with split-index addressing (tensor-core DMMA, SIMT for
+// split indices).
 //
 // Used by the plain FP64 sweep for the three contraction stages of the
 // effective-Hamiltonian matvec and of the environment updates

@@ -25,13 +25,13 @@
 // What bounds it: the chain of k column steps, ~0.85 us each (u by shuffles 0.1,
 // dots and butterfly 0.15, exchange 0.2, sums of 4C warps 0.12, two reciprocal square
 // roots 0.13, update 0.06, the divisions of tau and 1 / (alpha - beta) 0.1), and per panel ~9 us of publication (3) and application (6: DMMA
-// at the FP64 rate on C SMs).  512 x 256 305 us against 460 for the persistent
-// two-level kernel of qr.cu (one CTA per panel, one task queue), 64 x 64 71 (87),
-// 1024 x 512 802 (1822), 1536 x 512 1180 (2471), 512 x 1536 624 (1791).
+// at the FP64 rate on C SMs).  A call of tn_qr takes 325 us at 512 x 256 against 492 with
+// the kernels of qr.cu (one CTA per panel, one task queue), 90 (113) at 64 x 64,
+// 819 (1827) at 1024 x 512, 1127 (2428) at 1536 x 512, 645 (1843) at 512 x 1536.
 //
 // Rounding: 512 x 256, graded over five decades, |Q^T Q - I|_F 9.0e-15 and |QR - A| / |A| 5.0e-16 in extended
 // precision (persistent kernel 1.3e-14, 6.1e-16).  Without the divisions (tau and 1 / (alpha - beta)
-// from the chain's kap: 282 us) and with the products accumulated onto C the factors
+// from the chain's kap: 8 % less time) and with the products accumulated onto C the factors
 // were a quarter further from the exact ones.
 #include <cooperative_groups.h>
 
@@ -629,9 +629,9 @@ int qr_cluster(Ctx& c, int m, int n, const double* A, long long ars, long long a
     a.R = R; a.rrs = rrs; a.rcs = rcs;
     bool served = false;
     int st = TN_OK;
-    // Rows per CTA: as few as keep the exchange small.  Measured (without the divisions) with half the CTAs a cluster: 128 x 128 128 us
-    // (122 here), 256 x 256 255 (243); with twice as many (RL = 2): 512 x 256 309 (276), 512 x 1536 679 (566);
-    // with 8 warps a CTA instead of 8 CTAs: 1024 x 512 947 (741) -- above 512 rows that is left for when the
+    // Rows per CTA: as few as keep the exchange small.  A call of tn_qr with half the CTAs a cluster: 128 x 128 165 us
+    // (151 here), 256 x 256 300 (278); with twice as many (RL = 2): 512 x 256 351 (324), 512 x 1536 735 (645);
+    // with 8 warps a CTA instead of 8 CTAs: 1024 x 512 1020 (819) -- above 512 rows that is left for when the
     // clusters of 8 do not all fit (1536 x 512: 15 of 16).
     if (m <= 32) st = qc_launch<1, 1, 4>(c, a, &served);
     else if (m <= 64) st = qc_launch<2, 1, 4>(c, a, &served);
