@@ -139,6 +139,14 @@ struct QcLayout {
     static_assert(ldr % 16 == 4 && msg % 2 == 0 && x % 2 == 0, "alignment");
 };
 
+// den and kap of a column below 2^-511 or above 2^511 are not finite (or have lost their digits).  Its scale 1 /
+// (alpha - beta) tells (1 for a column without a reflector), looked at once, at the kernel's end, by one warp, in a
+// function of its own: in the panel the test cost 2 % of a 512 x 1536 QR.
+__device__ __noinline__ void qc_check_range(const double* scal, int* word) {
+    const double x = fabs(scal[threadIdx.x & 31]);
+    if (!(x <= 0x1p500 && x >= 0x1p-500)) atomicExch(word, 1);
+}
+
 template <int RL, int C, int W>
 __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
     using L = QcLayout<RL, C, W>;
@@ -512,12 +520,6 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
             asm volatile("cp.async.bulk.commit_group;\ncp.async.bulk.wait_group 0;" ::: "memory");
             qc_st_release(a.ready + q * C + rank, 1);
         }
-        // den and kap of a column below 2^-511 or above 2^511 are not finite (or have lost their digits): looked for
-        // here, behind the publication; tau = 0 marks the columns without a reflector
-        if (rank == 0 && tid < b && Ts[tid * QC_TLD + tid] != 0.0) {
-            const double nrm = fabs(be_s[tid]);
-            if (!(nrm >= 0x1p-500 && nrm <= 0x1p500)) atomicExch(a.derr + 1, 1);
-        }
         ok = bad == 0;
     }
     cl.sync();  // nor may a mate's partial Z land where the last step's sums are read
@@ -544,6 +546,7 @@ __global__ void __launch_bounds__(32 * W) qr_cluster_kernel(const QcArgs a) {
                 if (i < a.m && c < b) a.Q[(long long)i * a.qrs + (long long)(c0 + c) * a.qcs] = Cs[c * ldr + lr];
             });
     }
+    if (q < a.K && !qrows && w == 1) qc_check_range(sc_s, a.derr + 1);
     cl.sync();  // no CTA leaves while its shared memory may still be addressed
     // after a failure messages that nobody waits for may still be on their way
     if (qc_ld_acquire(a.err)) __nanosleep(200000);

@@ -329,7 +329,7 @@ __device__ __forceinline__ bool jc_rotate2(double (&x0)[E], double (&y0)[E], dou
     const double d = (be - al) * sc;
     // at least 2^-800: a smaller rotation changes nothing, and where the norms that followed the rotations have come
     // out zero (columns that were equal), the squares below would be denormal and the rotation no longer orthogonal
-    const double thr = fmax(tol2 * ((al * sc) * (be * sc)), 0x1p-800);
+    const double thr = fma(tol2, (al * sc) * (be * sc), 0x1p-800);
     double a0 = 0, b0 = 0, a1 = 0, b1 = 0;
 #pragma unroll
     for (int q = 0; q < E; q += 2) {
