@@ -749,7 +749,7 @@ __global__ void __launch_bounds__(1024) svd_order_kernel(const double* __restric
 // none: not served.  Four warps per CTA (one per scheduler) up to n = 128, eight
 // above, so that eight CTAs hold n = 256; with 16 row slots eight warps'
 // inboxes fit one parity only, and 16 CTAs of four warps are tried first
-// (256 x 256 with vectors, graded over three decades: 3.8 against 5.8 ms, 5.5 against 8.9 without the factorisation).
+// (256 x 256 with vectors, graded over three decades: 3.5 against 5.8 ms, 5.2 against 8.9 without the factorisation).
 struct JcShape {
     int ncta = 0, warps = 0;
 };
@@ -858,8 +858,8 @@ int svd_batched(Ctx& c, const std::vector<SvdJob>& jobs, bool vectors) {
     // that orthogonalise the columns of R^T (Drmac and Veselic, SIAM J. Matrix Anal. Appl. 29, 2008: R^T is closer to
     // diagonal than A) turn Q into U: R^T J = V' S gives A = (Q J) S (P V')^T.  The same kernel with R^T
     // above and Q's rows below, 9-11 sweeps instead of 14-19.  Factored and not (a call of tn_svd, graded over three
-    // decades): 16 x 16 136 and 119 us, 20 x 20 159 and 142, 25 x 25 204 and 223, 64 x 64 479 and 614,
-    // 150 x 128 1421 and 1869, 160 x 160 2141 and 3197; 150 x 128 26.7 ms with one CTA per matrix.
+    // decades): 16 x 16 135 and 122 us, 20 x 20 159 and 146, 25 x 25 204 and 226, 64 x 64 479 and 605,
+    // 150 x 128 1431 and 1881, 160 x 160 2154 and 3211; 150 x 128 26.7 ms with one CTA per matrix.
     const SvdJob& j0 = jobs[0];
     if (nj == 1 && j0.n >= SVD_PRE_MIN && !shapes.empty()) {
         const size_t nq = vectors ? (size_t)j0.m * j0.n : 0, nr = (size_t)j0.n * j0.n;
