@@ -27,7 +27,7 @@
 // roots 0.13, update 0.06, the divisions of tau and 1 / (alpha - beta) 0.1), and per panel ~9 us of publication (3) and application (6: DMMA
 // at the FP64 rate on C SMs).  A call of tn_qr takes 325 us at 512 x 256 against 492 with
 // the kernels of qr.cu (one CTA per panel, one task queue), 90 (113) at 64 x 64,
-// 819 (1827) at 1024 x 512, 1127 (2428) at 1536 x 512, 645 (1843) at 512 x 1536.
+// 819 (1827) at 1024 x 512, 1127 (2428) at 1536 x 512, 634 (1843) at 512 x 1536.
 //
 // Rounding: 512 x 256, graded over five decades, |Q^T Q - I|_F 9.0e-15 and |QR - A| / |A| 5.0e-16 in extended
 // precision (persistent kernel 1.3e-14, 6.1e-16).  Without the divisions (tau and 1 / (alpha - beta)
@@ -633,7 +633,7 @@ int qr_cluster(Ctx& c, int m, int n, const double* A, long long ars, long long a
     bool served = false;
     int st = TN_OK;
     // Rows per CTA: as few as keep the exchange small.  A call of tn_qr with half the CTAs a cluster: 128 x 128 165 us
-    // (151 here), 256 x 256 300 (278); with twice as many (RL = 2): 512 x 256 351 (324), 512 x 1536 735 (645);
+    // (151 here), 256 x 256 300 (278); with twice as many (RL = 2): 512 x 256 351 (324), 512 x 1536 735 (634);
     // with 8 warps a CTA instead of 8 CTAs: 1024 x 512 1020 (819) -- above 512 rows that is left for when the
     // clusters of 8 do not all fit (1536 x 512: 15 of 16).
     if (m <= 32) st = qc_launch<1, 1, 4>(c, a, &served);
